@@ -89,7 +89,10 @@ __device__ __forceinline__ V pdir(V beta, V p, V z) { return fmav<V>(beta, p, z)
 // Dot-product accumulator.  FP64 vectors accumulate in FP64.  FP32 vectors
 // accumulate exact products (a*b = p + e with e = fma(a,b,-p)) in a
 // compensated two-float sum, which keeps FP64-level accuracy of the sum while
-// issuing only FP32 instructions; the pair is widened to FP64 per thread.
+// issuing only FP32 instructions.  The pair is widened to FP64 once per warp:
+// an FP64 add occupies the SM's FP64 unit for 16 cycles a warp, so a shuffle
+// tree of FP64 adds over 32 resident warps and 8 sums costs some 10 us, and
+// the two-float tree adds no error of a higher order than the lo sums carry.
 template <typename V>
 struct DotAcc;
 template <>
@@ -109,6 +112,18 @@ struct DotAcc<float> {
     float err = (hi - (t - bp)) + (p - bp);
     hi = t;
     lo += err + e;
+  }
+  // the sum over lanes that differ in lane bits >= o0, exact in the high parts
+  __device__ __forceinline__ void warp_sum(int o0) {
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      if (o < o0) break;
+      const float h = __shfl_xor_sync(0xffffffffu, hi, o), l = __shfl_xor_sync(0xffffffffu, lo, o);
+      const float t = hi + h, bp = t - hi;
+      const float err = (hi - (t - bp)) + (h - bp);
+      hi = t;
+      lo = (lo + l) + err;
+    }
   }
   __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
@@ -896,131 +911,209 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_gather(
     // all threads: thread t sums blocks t/KR, t/KR + RED_THREADS/KR, ... of column t%KR in order
     __shared__ double sfin[RED_THREADS];
     double v = 0.0;
-    for (int idx = threadIdx.x; idx < (int)gridDim.x * KR; idx += RED_THREADS) v += __ldcg(part + idx);
+    const int np = (int)gridDim.x * KR;
+    for (int i0 = threadIdx.x; i0 < np; i0 += 4 * RED_THREADS) {
+      double x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = i0 + k * RED_THREADS < np ? __ldcg(part + i0 + k * RED_THREADS) : 0.0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v += x[k];
+    }
     sfin[threadIdx.x] = v;
     __syncthreads();
     if (threadIdx.x < KR) {
       int j = threadIdx.x;
       double s = 0.0;
-      for (int t = j; t < RED_THREADS; t += KR) s += sfin[t];
+      // a serial chain of FP64 adds: only entries that a block wrote (a PCG
+      // iteration of 300 elements in FP64, mostly these tails: 56 us with all
+      // 256 entries and one load in flight above, 37 now)
+      const int tn = min(RED_THREADS, np);
+      for (int t = j; t < tn; t += KR) s += sfin[t];
       if (cs[j].active && !cs[j].done) cs[j].alpha = cs[j].rz / s;
     }
     if (threadIdx.x == 0) G->cntB = 0;
   }
 }
 
-// Row-cooperative gather for FP32 with KR = 4, 8 or 16: a node's slot rows
-// (3*KR floats) are read by LPN = 3*KR/4 lanes, one 16-byte piece each, so a
-// warp's loads are coalesced runs of Y and no shared memory is needed.  Lane
-// (node, q) sums piece q over the node's slots in element order -- the same
-// additions in the same order as the staged gather, so kp and p are bitwise
-// equal to it; the p.kp partials are compensated sums over the lane's four
-// columns, reduced in a fixed order.
+// Flat gather for FP32: thread = one piece (VW columns, up to 16 bytes) of one
+// dof row of one node.  Consecutive threads take the LPN pieces of a node's
+// slot row, so a warp's loads are coalesced runs of Y and no lane idles; 960
+// threads per block keep the stride a multiple of LPN (3, 6 or 12), so a
+// thread's columns are fixed.  A node's pieces sum its slots in element order,
+// as the staged gather does: kp and p are bitwise equal to it.
+// What bounds it: HBM at large meshes, and below that the chain ptr -> slots
+// -> reduction tail.  So the next piece's slot range and dof number are
+// fetched one step ahead, and one block per SM (not four) leaves a quarter of
+// the partials for the last block, which reads them in one batch.  Gather and
+// update together at 16k elements and 16 columns: 145 us before, 94 now; at
+// 62k and 8 columns 189, 158 (event-timed).
 int g_gather_variant = 1;   // 0 = staged gather for every case
-constexpr int GATHER_ROWS_BLOCKS = 152 * 4;   // one wave: four resident CTAs per SM at 64 registers
-static_assert(GATHER_ROWS_BLOCKS * 16 <= NPART * 16 * 4, "p.kp partials fit the partial buffer");
 void set_gather_variant(int v) { g_gather_variant = v; }
+constexpr int FG_THREADS = 960;   // 30 warps at 64 registers: one block per SM
+constexpr int FU_THREADS = 512;   // update: 16 warps, four pieces a thread in flight
+constexpr int F_BLOCKS = 152;
+
+// Last-block sum of part[nblk][NQ] for the FP32 kernels: thread t adds entry
+// t % NQ of blocks t / NQ, t / NQ + NT / NQ, ... (eight loads in flight), then
+// the threads of one entry are added by a fixed tree.  maxq < NQ marks the
+// entries q with q % QS == maxq as maxima.  The result is in out[0..NQ).
+template <int NQ, int QS, int NT>
+__device__ __forceinline__ void last_block_sum(const double* __restrict__ part, int nblk, int maxq, double* sfin,
+                                               double* out) {
+  constexpr int R = NT / NQ;
+  const int t = threadIdx.x, q = t % NQ, r = t / NQ;
+  const bool mx = q % QS == maxq;
+  double v = 0.0;
+  if (r < R)
+    for (int b0 = r; b0 < nblk; b0 += 8 * R) {
+      double x[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[k] = b0 + k * R < nblk ? __ldcg(part + (size_t)(b0 + k * R) * NQ + q) : 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v = mx ? fmax(v, x[k]) : v + x[k];
+    }
+  sfin[t] = v;
+  __syncthreads();
+  if (t < NQ) {
+    // entries beyond the last block's row are zero
+    const int rn = min(R, nblk);
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int k = 0; k < rn; k += 4)
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        if (k + m < rn) a[m] = mx ? fmax(a[m], sfin[(k + m) * NQ + t]) : a[m] + sfin[(k + m) * NQ + t];
+    out[t] = mx ? fmax(fmax(a[0], a[1]), fmax(a[2], a[3])) : (a[0] + a[1]) + (a[2] + a[3]);
+  }
+  __syncthreads();
+}
+
+// VW consecutive floats
+template <int VW>
+struct Piece {
+  float v[VW];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int k = 0; k < VW; ++k) v[k] = 0.f;
+  }
+  __device__ __forceinline__ void load(const float* __restrict__ p) {
+    if constexpr (VW == 4) {
+      const float4 t = *reinterpret_cast<const float4*>(p);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else if constexpr (VW == 2) {
+      const float2 t = *reinterpret_cast<const float2*>(p);
+      v[0] = t.x; v[1] = t.y;
+    } else {
+      v[0] = *p;
+    }
+  }
+  __device__ __forceinline__ void load_once(const float* __restrict__ p) {
+    if constexpr (VW == 4) {
+      const float4 t = __ldcs(reinterpret_cast<const float4*>(p));
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else if constexpr (VW == 2) {
+      const float2 t = __ldcs(reinterpret_cast<const float2*>(p));
+      v[0] = t.x; v[1] = t.y;
+    } else {
+      v[0] = __ldcs(p);
+    }
+  }
+  __device__ __forceinline__ void store(float* __restrict__ p) const {
+    if constexpr (VW == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else if constexpr (VW == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+    else *p = v[0];
+  }
+};
 
 template <int KR>
-__global__ void __launch_bounds__(RED_THREADS, 4) k_pcg_gather_rows(
+__global__ void __launch_bounds__(FG_THREADS, 1) k_pcg_gather_flat(
     const int* __restrict__ ptr, const int* __restrict__ dof, int ng, const float* __restrict__ Y,
     float* __restrict__ kp, float* __restrict__ p, const float* __restrict__ z, int mode, ColState* __restrict__ cs,
     PcgGlobal* __restrict__ G, double* __restrict__ part) {
   if (G->all_done) return;
-  constexpr int QPD = KR / 4;      // 16-byte pieces per dof row
-  constexpr int LPN = 3 * QPD;     // lanes per node
-  constexpr int NPW = 32 / LPN;    // nodes per warp
+  constexpr int VW = KR < 4 ? KR : 4;   // columns per piece
+  constexpr int QPD = KR / VW;          // pieces per dof row
+  constexpr int LPN = 3 * QPD;          // pieces per node
+  static_assert(FG_THREADS % LPN == 0 && FG_THREADS % 32 == 0, "a thread keeps its columns");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nl = lane / LPN, q = lane - nl * LPN;
-  const int d = q / QPD, c0 = 4 * (q - d * QPD);
-  const bool act = nl < NPW;
-  DotAcc<float> dacc[4];
-  bool live[4];
-  float beta[4];
+  const int q = threadIdx.x % LPN, d = q / QPD, c0 = VW * (q % QPD);
+  DotAcc<float> dacc[VW];
+  bool live[VW];
+  float beta[VW];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int j = act ? c0 + k : 0;
-    live[k] = act && cs[j].active && !cs[j].done;
-    beta[k] = (float)cs[j].beta;
+  for (int k = 0; k < VW; ++k) {
+    live[k] = cs[c0 + k].active && !cs[c0 + k].done;
+    beta[k] = (float)cs[c0 + k].beta;
   }
-  const float4* yq = reinterpret_cast<const float4*>(Y) + q;
-  const int wstride = gridDim.x * GATHER_WARPS * NPW;
-  for (int g0 = (blockIdx.x * GATHER_WARPS + warp) * NPW; g0 < ng; g0 += wstride) {
-    const int g = g0 + nl;
-    if (!act || g >= ng) continue;
-    const int a = ptr[g], b = ptr[g + 1];
-    const int gd = dof[3 * g + d];
+  const float* yq = Y + VW * q;
+  const int gstride = gridDim.x * (FG_THREADS / LPN);
+  int g = blockIdx.x * (FG_THREADS / LPN) + threadIdx.x / LPN;
+  int a = 0, b = 0, gd = 0;
+  if (g < ng) { a = ptr[g]; b = ptr[g + 1]; gd = dof[3 * g + d]; }
+  for (; g < ng; g += gstride) {
     // the p and z rows do not depend on the sums: their loads go out with the
-    // first slot loads (two dependent trips per node instead of three)
-    float4* pp = reinterpret_cast<float4*>(p + (size_t)gd * KR + c0);
-    float4 pv = make_float4(0.f, 0.f, 0.f, 0.f), zv = pv;
+    // first slot loads
+    Piece<VW> pv, zv, acc, v[4];
+    pv.zero(); zv.zero(); acc.zero();
+    float* pp = p + (size_t)gd * KR + c0;
     if (mode != 0 && gd) {
-      pv = *pp;
-      zv = *reinterpret_cast<const float4*>(z + (size_t)gd * KR + c0);
+      pv.load(pp);
+      zv.load(z + (size_t)gd * KR + c0);
     }
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     // up to four slots in flight at once, summed in slot order
-    float4 v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      if (a + k < b) v[k] = __ldcs(yq + (size_t)(a + k) * LPN);
+      if (a + k < b) v[k].load_once(yq + (size_t)(a + k) * 3 * KR);
+    const int gn = g + gstride;
+    int an = 0, bn = 0, gdn = 0;
+    if (gn < ng) { an = ptr[gn]; bn = ptr[gn + 1]; gdn = dof[3 * gn + d]; }
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      if (a + k < b) {
-        acc.x = acc.x + v[k].x;
-        acc.y = acc.y + v[k].y;
-        acc.z = acc.z + v[k].z;
-        acc.w = acc.w + v[k].w;
+      if (a + k < b)
+#pragma unroll
+        for (int c = 0; c < VW; ++c) acc.v[c] = acc.v[c] + v[k].v[c];
+    for (int s0 = a + 4; s0 < b; s0 += 4) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (s0 + k < b) v[k].load_once(yq + (size_t)(s0 + k) * 3 * KR);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (s0 + k < b)
+#pragma unroll
+          for (int c = 0; c < VW; ++c) acc.v[c] = acc.v[c] + v[k].v[c];
+    }
+    if (gd) {
+      if (mode != 0) {
+#pragma unroll
+        for (int c = 0; c < VW; ++c)
+          if (live[c]) { pv.v[c] = pdir(beta[c], pv.v[c], zv.v[c]); dacc[c].add(pv.v[c], acc.v[c]); }
+        pv.store(pp);
       }
-    for (int sl = a + 4; sl < b; ++sl) {
-      const float4 w = __ldcs(yq + (size_t)sl * LPN);
-      acc.x = acc.x + w.x;
-      acc.y = acc.y + w.y;
-      acc.z = acc.z + w.z;
-      acc.w = acc.w + w.w;
+      acc.store(kp + (size_t)gd * KR + c0);
     }
-    if (!gd) continue;
-    float4* kpo = reinterpret_cast<float4*>(kp + (size_t)gd * KR + c0);
-    if (mode == 0) {
-      *kpo = acc;
-      continue;
-    }
-    if (live[0]) { pv.x = pdir(beta[0], pv.x, zv.x); dacc[0].add(pv.x, acc.x); }
-    if (live[1]) { pv.y = pdir(beta[1], pv.y, zv.y); dacc[1].add(pv.y, acc.y); }
-    if (live[2]) { pv.z = pdir(beta[2], pv.z, zv.z); dacc[2].add(pv.z, acc.z); }
-    if (live[3]) { pv.w = pdir(beta[3], pv.w, zv.w); dacc[3].add(pv.w, acc.w); }
-    *pp = pv;
-    *kpo = acc;
+    a = an; b = bn; gd = gdn;
   }
   if (mode == 0) return;
-  __shared__ double sred[RED_THREADS / 32][KR];
-  double mine[4];
+  __shared__ double sred[FG_THREADS / 32][KR];
+  __shared__ double sfin[FG_THREADS];
+  __shared__ double sout[KR];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) mine[k] = act ? dacc[k].value() : 0.0;
-#pragma unroll
-  for (int j = 0; j < KR; ++j) {
-    double v = (act && (j >> 2) == (c0 >> 2)) ? mine[j & 3] : 0.0;
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-    if (lane == 0) sred[warp][j] = v;
+  for (int k = 0; k < VW; ++k) {
+    dacc[k].warp_sum(QPD);
+    if (lane < QPD) sred[warp][VW * lane + k] = dacc[k].value();   // lane r holds pieces q % QPD of its lane class
   }
   __syncthreads();
+  // lane class r = lane % QPD of warp w holds columns VW * ((32 w + r) % QPD) ..: 32 is a multiple of QPD
   if (threadIdx.x < KR) {
     double v = 0.0;
-    for (int w = 0; w < RED_THREADS / 32; ++w) v += sred[w][threadIdx.x];
+#pragma unroll
+    for (int w = 0; w < FG_THREADS / 32; ++w) v += sred[w][threadIdx.x];
     part[(size_t)blockIdx.x * KR + threadIdx.x] = v;
   }
   if (last_block(&G->cntB)) {
-    __shared__ double sfin[RED_THREADS];
-    double v = 0.0;
-    for (int idx = threadIdx.x; idx < (int)gridDim.x * KR; idx += RED_THREADS) v += __ldcg(part + idx);
-    sfin[threadIdx.x] = v;
-    __syncthreads();
+    last_block_sum<KR, 1, FG_THREADS>(part, gridDim.x, 1, sfin, sout);
     if (threadIdx.x < KR) {
-      int j = threadIdx.x;
-      double t = 0.0;
-      for (int u = j; u < RED_THREADS; u += KR) t += sfin[u];
-      if (cs[j].active && !cs[j].done) cs[j].alpha = cs[j].rz / t;
+      const int j = threadIdx.x;
+      if (cs[j].active && !cs[j].done) cs[j].alpha = cs[j].rz / sout[j];
     }
     if (threadIdx.x == 0) G->cntB = 0;
   }
@@ -1276,12 +1369,12 @@ bool apply_uses_lanes(int dense, int KR) { return dense == 0 && (KR == 8 || KR =
 template <typename V, int KR>
 void pcg_gather(const GatherTopo& T, const V* Y, V* kp, V* p, const V* z, int mode, ColState* cs, PcgGlobal* G,
                 double* part, cudaStream_t s) {
-  if constexpr (std::is_same<V, float>::value && (KR == 4 || KR == 8 || KR == 16)) {
+  if constexpr (std::is_same<V, float>::value) {
     if (g_gather_variant == 1) {
-      // one wave of resident CTAs (the grid depends only on the problem size)
-      constexpr int NPB = GATHER_WARPS * (32 / (3 * KR / 4));   // nodes per block and pass
-      SG_LAUNCH k_pcg_gather_rows<KR><<<red_grid(T.ngroups, NPB * 4, GATHER_ROWS_BLOCKS), RED_THREADS, 0, s>>>(T.d_ptr, T.d_dof, T.ngroups, Y, kp, p, z, mode,
-                                                                   cs, G, part);
+      // at most one block per SM; the grid depends only on the problem size
+      constexpr int NPB = FG_THREADS / (3 * KR / (KR < 4 ? KR : 4));   // nodes per block and pass
+      SG_LAUNCH k_pcg_gather_flat<KR><<<red_grid(T.ngroups, NPB, F_BLOCKS), FG_THREADS, 0, s>>>(
+          T.d_ptr, T.d_dof, T.ngroups, Y, kp, p, z, mode, cs, G, part);
       return;
     }
   }
@@ -1337,13 +1430,42 @@ void launch_gather_plain(const GatherTopo& T, int KR, const V* Y, V* out, int ac
 // |alpha|*max|p|/max|u| <= tol (mode 0) or |r| <= tol*|r0| (mode 1), then
 // beta = r.z_new / r.z.
 // ---------------------------------------------------------------------------
-// Last block of an update: fixed-order reduction of the block partials and
-// the per-column stop test / beta (shared by both update kernels).
+// Stop test and beta of one column from its max|p|, max|u|, r.z and |r|^2.
+__device__ __forceinline__ void col_step(int init, int it, ColState& c, const PcgGlobal* __restrict__ G, double maxp,
+                                         double maxu, double rz, double rr) {
+  if (init) {
+    if (c.active) {
+      // keep_dir (G->mode & 2): continue the previous search direction after a
+      // residual replacement, beta = r.z_new / r.z of the last completed step
+      c.beta = (G->mode & 2) ? rz / c.rz : 0.0;
+      c.alpha = 0.0;   // the fused step's first vector update is empty
+      c.rz = rz; c.rr0 = rr; c.rr = rr; c.done = 0; c.failed = 0; c.iters = 0;
+    } else {
+      c.done = 1;
+    }
+  } else if (c.active && !c.done) {
+    c.maxp = maxp; c.maxu = maxu; c.rr = rr;
+    const bool stop =
+        ((G->mode & 1) == 0) ? (fabs(c.alpha) * maxp / maxu <= c.tol) : (rr <= c.tol * c.tol * c.rr0);
+    if (stop) {
+      c.done = 1; c.iters = it;
+    } else if (it >= G->maxiter) {
+      c.done = 1; c.failed = 1; c.iters = G->maxiter + 1;
+    } else {
+      c.beta = rz / c.rz;
+      c.rz = rz;
+    }
+  }
+}
+
+// Last block of an FP64 update: fixed-order reduction of the block partials
+// and the per-column step.
 template <int KR>
 __device__ __forceinline__ void update_finish(int init, ColState* __restrict__ cs, PcgGlobal* __restrict__ G,
                                               const double* __restrict__ part) {
   __shared__ int s_alldone;
   __shared__ double sfin[RED_THREADS];
+  const int it = init ? 0 : G->it + 1;
   if (threadIdx.x == 0) s_alldone = 1;
   // parallel fixed-order reduction of the block partials: thread t owns
   // quantity t % (4*KR) of blocks t/(4*KR), t/(4*KR) + RED_THREADS/(4*KR), ...
@@ -1351,44 +1473,27 @@ __device__ __forceinline__ void update_finish(int init, ColState* __restrict__ c
     constexpr int NQ = 4 * KR;
     const int q = threadIdx.x % 4;
     double v = 0.0;
-    for (int idx = threadIdx.x; idx < (int)gridDim.x * NQ; idx += RED_THREADS) {
-      double x = __ldcg(part + idx);
-      v = (q < 2) ? fmax(v, x) : v + x;
+    const int np = (int)gridDim.x * NQ;
+    for (int i0 = threadIdx.x; i0 < np; i0 += 8 * RED_THREADS) {
+      double x[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[k] = i0 + k * RED_THREADS < np ? __ldcg(part + i0 + k * RED_THREADS) : 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v = (q < 2) ? fmax(v, x[k]) : v + x[k];
     }
     sfin[threadIdx.x] = v;
   }
   __syncthreads();
-  const int it = init ? 0 : G->it + 1;
   if (threadIdx.x < KR) {
     const int jj = threadIdx.x;
     constexpr int NQ = 4 * KR;
     ColState& c = cs[jj];
     double a = 0.0, b = 0.0, s = 0.0, q = 0.0;
-    for (int t = jj * 4; t < RED_THREADS; t += NQ) {
+    const int tn = min(RED_THREADS, (int)gridDim.x * NQ);   // entries that a block wrote
+    for (int t = jj * 4; t < tn; t += NQ) {
       a = fmax(a, sfin[t]); b = fmax(b, sfin[t + 1]); s += sfin[t + 2]; q += sfin[t + 3];
     }
-    if (init) {
-      if (c.active) {
-        // keep_dir (G->mode & 2): continue the previous search direction after a
-        // residual replacement, beta = r.z_new / r.z of the last completed step
-        c.beta = (G->mode & 2) ? s / c.rz : 0.0;
-        c.alpha = 0.0;   // the fused step's first vector update is empty
-        c.rz = s; c.rr0 = q; c.rr = q; c.done = 0; c.failed = 0; c.iters = 0;
-      } else {
-        c.done = 1;
-      }
-    } else if (c.active && !c.done) {
-      c.maxp = a; c.maxu = b; c.rr = q;
-      bool stop = ((G->mode & 1) == 0) ? (fabs(c.alpha) * a / b <= c.tol) : (q <= c.tol * c.tol * c.rr0);
-      if (stop) {
-        c.done = 1; c.iters = it;
-      } else if (it >= G->maxiter) {
-        c.done = 1; c.failed = 1; c.iters = G->maxiter + 1;
-      } else {
-        c.beta = s / c.rz;
-        c.rz = s;
-      }
-    }
+    col_step(init, it, c, G, a, b, s, q);
     if (jj < G->kcols && c.active && !c.done) atomicAnd(&s_alldone, 0);
   }
   __syncthreads();
@@ -1482,145 +1587,170 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_update(
   update_finish<KR>(init, cs, G, part);
 }
 
-// FP32 update with KR = 4, 8 or 16 in 16-byte pieces: thread t always owns
-// columns c0..c0+3 (c0 = 4 (t mod KR/4)) of the rows it visits, so every load
-// moves 16 bytes; per-column max-norms and compensated dots are then reduced
-// over the lanes of equal c0 and finished exactly as in k_pcg_update.
+// FP32 update in 16-byte pieces: thread t takes pieces t, t + stride, ... of
+// the flat [n1][KR] arrays, so its four components always belong to the same
+// columns; per-column max-norms and compensated dots are reduced over the
+// lanes of equal columns.  max|u| only serves the step test of the FP64 solve
+// and is not formed.  HBM bounds it at large meshes (7 vector passes); one
+// block of 512 threads per SM with four pieces of four vectors a thread in
+// flight (128 KB) leaves 152 partials for the last block.
 template <int KR>
-__global__ void __launch_bounds__(RED_THREADS, 4) k_pcg_update4(
+__global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
     int n1, float* __restrict__ u, float* __restrict__ r, float* __restrict__ z, const float* __restrict__ p,
     const float* __restrict__ kp, const float* __restrict__ f, const float* __restrict__ dprecon, int init,
     ColState* __restrict__ cs, PcgGlobal* __restrict__ G, double* __restrict__ part) {
   if (G->all_done) return;
-  constexpr int QP = KR / 4;
-  const int c0 = 4 * (threadIdx.x % QP);
+  constexpr int QP = KR < 4 ? 1 : KR / 4;          // pieces per row (KR >= 4)
+  constexpr int NC = KR < 4 ? KR : 4;              // columns a thread touches
+  const int c0 = KR < 4 ? 0 : 4 * (threadIdx.x % QP);
   bool live[4];
   float alpha[4];
-  bool any = false;
+  bool any = false, all4 = true;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    live[k] = cs[c0 + k].active && (init || !cs[c0 + k].done);
-    alpha[k] = (float)(init ? 0.0 : cs[c0 + k].alpha);
+    const int j = c0 + k % NC;
+    live[k] = cs[j].active && (init || !cs[j].done);
+    alpha[k] = (float)(init ? 0.0 : cs[j].alpha);
     any = any || live[k];
+    all4 = all4 && live[k];
   }
-  const bool all4 = live[0] && live[1] && live[2] && live[3];
-  float mpv[4] = {0.f, 0.f, 0.f, 0.f}, muv[4] = {0.f, 0.f, 0.f, 0.f};
+  float mp[4] = {0.f, 0.f, 0.f, 0.f};
   DotAcc<float> rza[4], rra[4];
-  if (any) {
-    const size_t n4 = (size_t)n1 * QP;                    // 16-byte pieces
-    const size_t stride = (size_t)gridDim.x * blockDim.x;  // a multiple of QP: c0 is fixed
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const float4* p4 = reinterpret_cast<const float4*>(p);
-    const float4* k4 = reinterpret_cast<const float4*>(kp);
-    float4* u4 = reinterpret_cast<float4*>(u);
-    float4* r4 = reinterpret_cast<float4*>(r);
-    float4* z4 = reinterpret_cast<float4*>(z);
-    if (init) {
-      const float4* f4 = reinterpret_cast<const float4*>(f);
-      for (; i < n4; i += stride) {
-        const float4 fv = f4[i], kv = k4[i];
-        const float d = dprecon[i / QP];
-        float4 rn, zn;
-        rn.x = fv.x - kv.x; rn.y = fv.y - kv.y; rn.z = fv.z - kv.z; rn.w = fv.w - kv.w;
-        zn.x = d * rn.x; zn.y = d * rn.y; zn.z = d * rn.z; zn.w = d * rn.w;
-        const float rv[4] = {rn.x, rn.y, rn.z, rn.w}, zv[4] = {zn.x, zn.y, zn.z, zn.w};
-        if (all4) {
-          r4[i] = rn;
-          z4[i] = zn;
-        } else {
+  const size_t n = (size_t)n1 * KR, n4 = (n + 3) / 4;
+  const size_t stride = (size_t)gridDim.x * FU_THREADS;   // a multiple of QP
+  size_t i = (size_t)blockIdx.x * FU_THREADS + threadIdx.x;
+  // diagonal entries of piece o (KR < 4 spans several rows; the last piece may be cut)
+  auto diag = [&](size_t o, float (&dv)[4]) {
+    if constexpr (KR >= 4) {
+      const float d = dprecon[o / QP];
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (live[k]) { r[4 * i + k] = rv[k]; z[4 * i + k] = zv[k]; }
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (live[k]) { rza[k].add(rv[k], zv[k]); rra[k].add(rv[k], rv[k]); }
-      }
+      for (int k = 0; k < 4; ++k) dv[k] = d;
     } else {
-      // four 16-byte loads per thread in flight, four CTAs per SM
-      constexpr int U = 1;
-      for (; i < n4; i += U * stride) {
-        float4 pv[U], uv[U], rv[U], kv[U];
-        float dv[U];
-        bool in[U];
 #pragma unroll
-        for (int q = 0; q < U; ++q) {
-          const size_t o = i + q * stride;
-          in[q] = o < n4;
-          if (in[q]) { pv[q] = p4[o]; uv[q] = u4[o]; rv[q] = r4[o]; kv[q] = k4[o]; dv[q] = dprecon[o / QP]; }
-        }
+      for (int k = 0; k < 4; ++k) dv[k] = 4 * o + k < n ? dprecon[(4 * o + k) / KR] : 0.f;
+    }
+  };
+  auto load = [&](const float* __restrict__ x, size_t o, float (&v)[4]) {
+    if (KR >= 4 || 4 * o + 3 < n) {
+      const float4 t = reinterpret_cast<const float4*>(x)[o];
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
 #pragma unroll
-        for (int q = 0; q < U; ++q) {
-          if (!in[q]) continue;
-          const size_t o = i + q * stride;
-          const float pa[4] = {pv[q].x, pv[q].y, pv[q].z, pv[q].w};
-          const float ua[4] = {uv[q].x, uv[q].y, uv[q].z, uv[q].w};
-          const float ra[4] = {rv[q].x, rv[q].y, rv[q].z, rv[q].w};
-          const float ka[4] = {kv[q].x, kv[q].y, kv[q].z, kv[q].w};
-          float un[4], rn[4], zn[4];
+      for (int k = 0; k < 4; ++k) v[k] = 4 * o + k < n ? x[4 * o + k] : 0.f;
+    }
+  };
+  // columns that are not live are left untouched
+  auto store = [&](float* __restrict__ x, size_t o, const float (&v)[4]) {
+    if (all4 && (KR >= 4 || 4 * o + 3 < n)) {
+      reinterpret_cast<float4*>(x)[o] = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            un[k] = fmaf(alpha[k], pa[k], ua[k]);
-            rn[k] = fmaf(-alpha[k], ka[k], ra[k]);
-            zn[k] = dv[q] * rn[k];
-            if (live[k]) {
-              mpv[k] = fmaxf(mpv[k], fabsf(pa[k]));
-              muv[k] = fmaxf(muv[k], fabsf(un[k]));
-              rza[k].add(rn[k], zn[k]);
-              rra[k].add(rn[k], rn[k]);
-            }
+      for (int k = 0; k < 4; ++k)
+        if (live[k] && 4 * o + k < n) x[4 * o + k] = v[k];
+    }
+  };
+  if (any && init) {
+    for (; i < n4; i += stride) {
+      float fv[4], kv[4], dv[4], rn[4], zn[4];
+      load(f, i, fv);
+      load(kp, i, kv);
+      diag(i, dv);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        rn[k] = fv[k] - kv[k];
+        zn[k] = dv[k] * rn[k];
+        if (live[k]) { rza[k].add(rn[k], zn[k]); rra[k].add(rn[k], rn[k]); }
+      }
+      store(r, i, rn);
+      store(z, i, zn);
+    }
+  } else if (any) {
+    constexpr int U = 4;
+    for (; i < n4; i += U * stride) {
+      float pv[U][4], uv[U][4], rv[U][4], kv[U][4], dv[U][4];
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        const size_t o = i + q * stride;
+        if (o < n4) { load(p, o, pv[q]); load(u, o, uv[q]); load(r, o, rv[q]); load(kp, o, kv[q]); diag(o, dv[q]); }
+      }
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        const size_t o = i + q * stride;
+        if (o >= n4) continue;
+        float un[4], rn[4], zn[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          un[k] = fmaf(alpha[k], pv[q][k], uv[q][k]);
+          rn[k] = fmaf(-alpha[k], kv[q][k], rv[q][k]);
+          zn[k] = dv[q][k] * rn[k];
+          if (live[k]) {
+            mp[k] = fmaxf(mp[k], fabsf(pv[q][k]));
+            rza[k].add(rn[k], zn[k]);
+            rra[k].add(rn[k], rn[k]);
           }
-          if (all4) {
-            u4[o] = make_float4(un[0], un[1], un[2], un[3]);
-            r4[o] = make_float4(rn[0], rn[1], rn[2], rn[3]);
-            z4[o] = make_float4(zn[0], zn[1], zn[2], zn[3]);
-          } else {
-            // columns that are not live are left untouched
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              if (live[k]) { u[4 * o + k] = un[k]; r[4 * o + k] = rn[k]; z[4 * o + k] = zn[k]; }
-          }
         }
+        store(u, o, un);
+        store(r, o, rn);
+        store(z, o, zn);
       }
     }
   }
-  __shared__ double sred[RED_THREADS / 32][KR][4];
+  // partials [block][column][4] = max|p|, -, r.z, |r|^2
+  constexpr int NQ = 4 * KR;
+  __shared__ double sred[FU_THREADS / 32][NQ];
+  __shared__ double sfin[FU_THREADS];
+  __shared__ double sout[NQ];
+  __shared__ int s_alldone;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    double mp = (double)mpv[k], mu = (double)muv[k], rz = live[k] ? rza[k].value() : 0.0,
-           rr = live[k] ? rra[k].value() : 0.0;
+    rza[k].warp_sum(QP);
+    rra[k].warp_sum(QP);
 #pragma unroll
-    for (int o = 16; o >= QP; o >>= 1) {
-      mp = fmax(mp, __shfl_xor_sync(FULL, mp, o));
-      mu = fmax(mu, __shfl_xor_sync(FULL, mu, o));
-      rz += __shfl_xor_sync(FULL, rz, o);
-      rr += __shfl_xor_sync(FULL, rr, o);
-    }
-    if (lane < QP) {
-      const int j = 4 * lane + k;
-      sred[warp][j][0] = mp; sred[warp][j][1] = mu; sred[warp][j][2] = rz; sred[warp][j][3] = rr;
+    for (int o = 16; o >= QP; o >>= 1) mp[k] = fmaxf(mp[k], __shfl_xor_sync(FULL, mp[k], o));
+  }
+  if (lane < QP) {
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      double* o = sred[warp] + 4 * (4 * lane * (KR >= 4) + k);
+      double m = 0.0, a = 0.0, b = 0.0;
+#pragma unroll
+      for (int c = k; c < 4; c += NC) { m = fmax(m, (double)mp[c]); a += rza[c].value(); b += rra[c].value(); }
+      o[0] = m; o[1] = 0.0; o[2] = a; o[3] = b;
     }
   }
   __syncthreads();
-  if (threadIdx.x < KR) {
-    double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
-    for (int w = 0; w < RED_THREADS / 32; ++w) {
-      a = fmax(a, sred[w][threadIdx.x][0]); b = fmax(b, sred[w][threadIdx.x][1]);
-      c += sred[w][threadIdx.x][2]; d += sred[w][threadIdx.x][3];
-    }
-    double* o = part + ((size_t)blockIdx.x * KR + threadIdx.x) * 4;
-    o[0] = a; o[1] = b; o[2] = c; o[3] = d;
+  if (threadIdx.x < NQ) {
+    const int q = threadIdx.x & 3;
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < FU_THREADS / 32; ++w) v = q == 0 ? fmax(v, sred[w][threadIdx.x]) : v + sred[w][threadIdx.x];
+    part[(size_t)blockIdx.x * NQ + threadIdx.x] = v;
   }
   if (!last_block(&G->cntC)) return;
-  update_finish<KR>(init, cs, G, part);
+  last_block_sum<NQ, 4, FU_THREADS>(part, gridDim.x, 0, sfin, sout);
+  if (threadIdx.x == 0) s_alldone = 1;
+  __syncthreads();
+  const int it = init ? 0 : G->it + 1;
+  if (threadIdx.x < KR) {
+    const double* o = sout + 4 * threadIdx.x;
+    ColState& c = cs[threadIdx.x];
+    col_step(init, it, c, G, o[0], 0.0, o[2], o[3]);
+    if ((int)threadIdx.x < G->kcols && c.active && !c.done) atomicAnd(&s_alldone, 0);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    G->it = it;
+    G->all_done = s_alldone;
+    G->cntC = 0;
+  }
 }
 
 template <typename V, int KR>
 void pcg_update(int n1, V* u, V* r, V* z, const V* p, const V* kp, const V* f, const V* dprecon, int init,
                 ColState* cs, PcgGlobal* G, double* part, cudaStream_t s) {
-  if constexpr (std::is_same<V, float>::value && (KR == 4 || KR == 8 || KR == 16)) {
-    SG_LAUNCH k_pcg_update4<KR><<<red_grid((size_t)n1 * (KR / 4), RED_THREADS * 4, NPART), RED_THREADS, 0, s>>>(
+  if constexpr (std::is_same<V, float>::value) {
+    SG_LAUNCH k_pcg_update_flat<KR><<<red_grid((size_t)n1 * KR, FU_THREADS * 4, F_BLOCKS), FU_THREADS, 0, s>>>(
         n1, u, r, z, p, kp, f, dprecon, init, cs, G, part);
     return;
   }

@@ -1,0 +1,44 @@
+"""The FP32 PCG kernels by width and mesh size: each pair of ways to run an
+iteration drives the mixed solve to the same trials.
+
+The FP64 residual decides when a solve is done, so two FP32 paths that differ
+in rounding only agree to the refinement target (1e-10 of the load) times the
+conditioning of these small meshes: 1e-8 is two orders above what that gives,
+and far below any wrong sum, column or index.
+"""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-8
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def trials(dims, k, tmp, **env):
+    out = str(tmp / ("_".join(env.values()) + ".npz"))
+    code = ("import sys; sys.path.insert(0, %r); import numpy as np; import specfem3d_geotech_gb300 as sg;"
+            "from specfem3d_geotech_gb300 import meshgen; m = sg.Model(meshgen.slope3d(*%r), precision=sg.PREC_MIXED);"
+            "r, x = m.trials([1.0 + 0.02 * t for t in range(%d)], sg.make_control(nl_maxiter=2, precision=sg.PREC_MIXED),"
+            " want_x=True); np.savez(%r, x=x, nl=[t['nl_iter'] for t in r], e=[t['errcode'] for t in r])") % (
+        ROOT, dims, k, out)
+    subprocess.run([sys.executable, "-c", code], check=True, env=dict(os.environ, **env), timeout=300)
+    return np.load(out)
+
+
+def same(a, b):
+    assert not a["e"].any() and not b["e"].any() and np.array_equal(a["nl"], b["nl"])
+    for x, y in zip(a["x"], b["x"]):
+        assert np.linalg.norm(x - y) <= TOL * np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 5, 16])
+@pytest.mark.parametrize("dims", [(2, 2, 2), (11, 5, 3)])
+def test_flat_gather_and_update_match_staged(tmp_path, dims, k):
+    a = trials(dims, k, tmp_path, SG_PERSIST="0", SG_GATHER_VARIANT="1")
+    b = trials(dims, k, tmp_path, SG_PERSIST="0", SG_GATHER_VARIANT="0")
+    same(a, b)
