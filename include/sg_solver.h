@@ -353,7 +353,7 @@ int sg_excavation(sg_model* model, const sg_control* ctl, int s0_type, double z0
 int sg_excavation_fields(const sg_model* model, double* vmeps, double* scf);
 
 /* ---- timing of the device work of the last call ----------------------- */
-/* ms[0] total, ms[1] element apply, ms[2] gather, ms[3] PCG vector update,
+/* ms[0] PCG chunks that run as one kernel (small meshes), ms[1] element apply, ms[2] gather, ms[3] PCG vector update,
  * ms[4] stress update, ms[5] stiffness build; counts[0..3] = launches of the
  * apply kernel, total kernel launches, PCG iterations, FP64 refinement residuals.
  * Collected with CUDA events on the context's stream when enabled. */

@@ -306,19 +306,24 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
       (uintptr_t)C->d_nbr, (uintptr_t)B.Y, (uintptr_t)B.kp, (uintptr_t)B.p, (uintptr_t)B.z, (uintptr_t)B.r,
       (uintptr_t)B.cs, (uintptr_t)B.G, (uintptr_t)B.part, (uintptr_t)u, (uintptr_t)f, (uintptr_t)dp,
       (uintptr_t)n1, (uintptr_t)KR, (uintptr_t)sizeof(V), (uintptr_t)chunk, (uintptr_t)fused};
-  // very small meshes with the matrix-free FP32 operator: the whole chunk as
-  // one persistent cooperative launch (sg_pcg_persist.cu), below the size at
-  // which the grid barrier costs more than the launches it saves
+  // small and medium meshes with the matrix-free FP32 operator: the whole chunk
+  // as one persistent cooperative launch (sg_pcg_persist.cu).  It stops by
+  // itself at the solve's end, so the chunk only bounds the time between two
+  // looks of the host.
   bool persist = false;
-  if constexpr (std::is_same<V, float>::value && KR <= 8)
-    persist = op.dense == 2 && op.nelmt < persist_max_elements() && !C->prof.on && persist_enabled();
+  if constexpr (std::is_same<V, float>::value)
+    persist = op.dense == 2 && (mode & 1) && op.nelmt < persist_max_elements(KR) && persist_enabled();
+  constexpr int persist_chunk = 512;
   int nchunks = 0;
   while (true) {
     bool done_chunk = false;
     if constexpr (std::is_same<V, float>::value)
-      if (persist)
-        done_chunk = launch_pcg_persistent<KR>((const float*)op.K, op.ge, op.nelmt, op.T->d_pos, *op.T, n1, u, B.r,
-                                               B.z, B.p, B.kp, B.Y, dp, B.cs, B.G, B.part, chunk, s);
+      if (persist) {
+        ev = C->prof_begin();
+        done_chunk = launch_pcg_persistent<KR>((const float*)op.K, op.ge, op.nelmt, op.T->d_pos, *op.T, u, B.r, B.z,
+                                               B.p, B.kp, B.Y, dp, B.cs, B.G, B.part, persist_chunk, s);
+        C->prof_end(ev, 0);
+      }
     cudaGraphExec_t ex = (!done_chunk && graphs && nchunks > 0) ? C->chunk_graph(key, eager_chunk) : nullptr;
     if (done_chunk) {
     } else if (ex) {
@@ -338,7 +343,7 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
       break;
     }
     if (hG->all_done) break;
-    if (it >= maxiter + chunk) { status = SG_ERR_TIMEOUT; break; }
+    if (it >= maxiter + std::max(chunk, persist_chunk)) { status = SG_ERR_TIMEOUT; break; }
     double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     if (el > 3600.0) { status = SG_ERR_TIMEOUT; C->err = "PCG wall-clock guard"; break; }
   }

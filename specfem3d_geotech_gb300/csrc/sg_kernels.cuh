@@ -89,16 +89,16 @@ constexpr int MF_REC = 12;        // floats per GLL point of the matrix-free rec
 void launch_nodal_average(const int* ptr, const int* slot, int nnode, const double* stress, double* out,
                           cudaStream_t s);  // sg_output.cu
 bool fp32_matrix_free(int nelmt);
-// Persistent cooperative FP32 PCG chunk for small meshes (sg_pcg_persist.cu);
-// false when it cannot run (the caller launches the separate kernels).
+// Persistent cooperative FP32 PCG chunk for small and medium meshes
+// (sg_pcg_persist.cu); false when it cannot run (the caller launches the
+// separate kernels).  A chunk whose bounded wait ran out sets G->err.
 template <int KR>
-bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int* pos, const GatherTopo& T, int n1,
-                           float* u, float* r, float* z, float* p, float* kp, float* Y, const float* dp,
-                           ColState* cs, PcgGlobal* G, double* part, int chunk, cudaStream_t s);
+bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int* pos, const GatherTopo& T, float* u,
+                           float* r, float* z, float* p, float* kp, float* Y, const float* dp, ColState* cs,
+                           PcgGlobal* G, double* part, int chunk, cudaStream_t s);
 bool persist_enabled();                 // SG_PERSIST=0 turns the persistent chunk off
-int persist_max_elements();             // meshes below this use it
-// a persistent chunk whose grid barrier timed out sets G->err
-void set_gather_variant(int v);  // 1 row-cooperative gather for FP32 with 4/8/16 RHS (default), 0 staged
+int persist_max_elements(int KR);       // meshes below this use it
+void set_gather_variant(int v);  // 1 flat gather for FP32 (default), 0 staged
 template <typename V, int KR>
 // Y receives element slot (e, a)'s three rows (x KR) at the slot's gather
 // position pos[e*27+a] (slots of fully fixed nodes, pos < 0, are skipped).

@@ -1,33 +1,46 @@
-// sg_pcg_persist.cu -- the FP32 PCG iterations of small meshes as one
-// persistent cooperative kernel.
+// sg_pcg_persist.cu -- the FP32 PCG iterations of small and medium meshes as
+// one persistent cooperative kernel.
 //
 // On a few thousand elements a PCG iteration (element apply, gather, vector
-// update) does about a microsecond of work but costs three dependent kernels,
-// each a chain of global-memory round trips plus a last-block reduction.
-// Here a chunk of iterations runs inside one cooperative launch: the three
-// phases of an iteration are separated by a grid barrier, and instead of a
-// last block every block recomputes alpha (after the gather) and the stop
-// test and beta (after the update) from the block partials, in the same fixed
-// order, so all blocks agree without another barrier and the results are
-// deterministic.  Data written by another block in the same launch is read
-// through L2 (ld.global.cg).
+// update) is a microsecond or two of work, but three dependent kernels cost
+// some 12 us each: the launch, a chain of L2 round trips (control word,
+// column state, data), and a last-block reduction behind an atomic.  Here a
+// chunk of iterations runs inside one launch of one block per SM:
 //
-// The phases do the arithmetic of the separate kernels: the matrix-free
-// element apply with p = z + beta p_old formed on the fly (sg_apply_mf.cu),
-// the gather of element products in element order fused with p = z + beta p
-// and the compensated p.kp partials, and u += alpha p, r -= alpha kp,
-// z = D r with the max-norms and compensated r.z, r.r partials; the
-// per-column stop tests are those of the update kernel (reference step test
-// of src/solver.f90:61-73 or the residual-reduction test).
+//   A  element products of p = z + beta p_old -> Y          | barrier
+//   B  kp = sum of Y per node, p = z + beta p_old, p.kp      | barrier, sums
+//   C  u += alpha p, r -= alpha kp, z = D r, r.z, r.r        | barrier, sums
 //
-// The barrier is bounded: a block that waits too long sets the error word of
-// the solve's control word and leaves; every other block's wait then runs out
-// as well, the launch ends and the solve reports SG_ERR_TIMEOUT without
-// launching another chunk.  The barrier's arrival count and generation live in
-// the solve's own control word (the count is zeroed before every launch), so
-// concurrent solves on other streams do not share them.
+// The barrier is one counter: a block's first thread adds to it with release
+// order and alone polls it (2,600 cycles on 152 blocks; flags or partials that
+// every block polls from every other took 8,700, clusters with one flag each
+// 3,700).  Partial sums are written before the barrier of their phase and
+// added by every block after it, in the same order, so all blocks take the
+// same decisions and results are deterministic.
+//
+// FP64 arithmetic is kept out of the loop: an FP64 add or conversion holds the
+// SM's FP64 unit for 16 cycles a warp, and the trees over 15 warps and up to 32
+// sums took longer than the barrier.  Sums stay two-float pairs (exact
+// products, compensated adds) up to the scalars, which are formed from pairs
+// and rounded to FP32 once, as the vector operations take them.
+//
+// A dof row's u, r, p stay in the registers of the thread that owns it while
+// the mesh is small enough (R pieces of up to four columns a thread, R = 1 or
+// 2); beyond that (R = 0) they stream through L2.  The element maps and point
+// records of a block's elements stay in shared memory where they fit.
+//
+// Phase A gives a warp one element and up to four columns, lane = node: the
+// warp is its own barrier, each lane's four columns are independent chains,
+// and all shared traffic is 16 bytes a lane.  The arithmetic per column and its
+// order are those of sg_apply_mf.cu, and phases B and C do that of the gather
+// and update kernels, so the two ways differ only in how the dots are grouped.
+//
+// Waits are bounded: a block that polls too long sets the solve's error word
+// and leaves, the others' waits then run out as well, the launch ends and the
+// solve reports SG_ERR_TIMEOUT without launching another chunk.
 #include <cstdint>
 #include <cstdlib>
+#include <type_traits>
 
 #include "sg_kernels.cuh"
 
@@ -35,8 +48,10 @@ namespace sg {
 
 namespace pp {
 
-constexpr int NT = 256;               // threads per block
-constexpr int BAR_TRIES = 1 << 20;    // bounded barrier wait (x ~64 ns)
+constexpr int NT = 480;               // 15 warps; a multiple of 3, 6 and 12 pieces per node
+constexpr int NWARP = NT / 32;
+constexpr int MAX_BLOCKS = 152;       // one block per SM
+constexpr int POLL_TRIES = 1 << 20;   // bounded wait, below a second
 
 // compensated FP32 dot accumulator (exact products, two-float sum)
 struct CompSum {
@@ -48,44 +63,102 @@ struct CompSum {
     hi = t;
     lo += err + e;
   }
-  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+  __device__ __forceinline__ void add(const float2 x) {   // another such sum
+    const float t = hi + x.x, bp = t - hi;
+    const float err = (hi - (t - bp)) + (x.x - bp);
+    hi = t;
+    lo = (lo + x.y) + err;
+  }
+  // sum over the lanes whose index differs in bits >= o0
+  __device__ __forceinline__ void warp_sum(int o0) {
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      if (o < o0) break;
+      add(make_float2(__shfl_xor_sync(0xffffffffu, hi, o), __shfl_xor_sync(0xffffffffu, lo, o)));
+    }
+  }
+  __device__ __forceinline__ float2 pair() const { return make_float2(hi, lo); }
 };
+__device__ __forceinline__ double value(const float2 x) { return (double)x.x + (double)x.y; }
+__device__ __forceinline__ float2 split(double x) {
+  const float h = (float)x;
+  return make_float2(h, (float)(x - (double)h));
+}
+__device__ __forceinline__ float2 norm2(const float2 x) {   // |lo| <= ulp(hi) / 2
+  const float h = x.x + x.y;
+  return make_float2(h, x.y - (h - x.x));
+}
+// a / b of two-float numbers: the FP32 quotient and its residual's
+__device__ __forceinline__ float2 div2(float2 a, float2 b) {
+  a = norm2(a);
+  b = norm2(b);
+  const float q = a.x / b.x;
+  const float r = fmaf(-q, b.x, a.x) + fmaf(-q, b.y, a.y);
+  return norm2(make_float2(q, r / b.x));
+}
 
-__device__ __forceinline__ float ldf(const float* p) { return __ldcg(p); }
-
-// Grid barrier on (count = G->cntB, generation = G->pad).  Returns false (for
-// every thread of the block) when the wait ran out.
-__device__ __forceinline__ bool grid_barrier(PcgGlobal* G) {
-  __syncthreads();
-  int ok = 1;
-  if (threadIdx.x == 0) {
-    volatile unsigned* gen = &G->pad;
-    const unsigned g0 = *gen;
-    __threadfence();
-    if (atomicAdd(&G->cntB, 1u) == gridDim.x - 1) {
-      atomicExch(&G->cntB, 0u);
-      __threadfence();
-      atomicAdd(&G->pad, 1u);
-    } else {
-      int tries = 0;
-      while (*gen == g0) {
-        if (++tries > BAR_TRIES) {
-          ok = 0;
-          atomicExch(&G->err, 1);
-          break;
+// Sums x[0..N) over the lanes that differ in bits O, O/2, ..., O0, halving the
+// values a lane carries at each step while it has several (N - 1 + steps adds
+// instead of N * steps): the lane ends with value index() in x[0].
+template <int N, int O, int O0>
+struct Reduce {
+  static __device__ __forceinline__ void run(CompSum (&x)[N], int lane) {
+    if constexpr (O >= O0) {
+      if constexpr (N > 1) {
+        const bool up = lane & O;
+        CompSum y[N / 2];
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+          const CompSum keep = up ? x[i + N / 2] : x[i], send = up ? x[i] : x[i + N / 2];
+          y[i] = keep;
+          y[i].add(make_float2(__shfl_xor_sync(0xffffffffu, send.hi, O), __shfl_xor_sync(0xffffffffu, send.lo, O)));
         }
-        __nanosleep(64);
+        Reduce<N / 2, O / 2, O0>::run(y, lane);
+        x[0] = y[0];
+      } else {
+        x[0].add(make_float2(__shfl_xor_sync(0xffffffffu, x[0].hi, O), __shfl_xor_sync(0xffffffffu, x[0].lo, O)));
+        Reduce<N, O / 2, O0>::run(x, lane);
       }
     }
-    __threadfence();
   }
-  return __syncthreads_and(threadIdx.x != 0 || ok) != 0;
-}
+};
 
-__device__ __forceinline__ constexpr float Dm(int i, int t) {
-  return i == 0 ? (t == 0 ? -1.5f : t == 1 ? 2.0f : -0.5f)
-                : i == 1 ? (t == 0 ? -0.5f : t == 1 ? 0.0f : 0.5f) : (t == 0 ? 0.5f : t == 1 ? -2.0f : 1.5f);
-}
+// VW consecutive floats; loads go through L2 (other blocks write the data)
+template <int VW>
+struct Vec {
+  float v[VW];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int k = 0; k < VW; ++k) v[k] = 0.f;
+  }
+  __device__ __forceinline__ void load_cg(const float* p) {
+    if constexpr (VW == 4) {
+      const float4 t = __ldcg(reinterpret_cast<const float4*>(p));
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else if constexpr (VW == 2) {
+      const float2 t = __ldcg(reinterpret_cast<const float2*>(p));
+      v[0] = t.x; v[1] = t.y;
+    } else {
+      v[0] = __ldcg(p);
+    }
+  }
+  __device__ __forceinline__ void load(const float* p) {   // shared memory
+    if constexpr (VW == 4) {
+      const float4 t = *reinterpret_cast<const float4*>(p);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else if constexpr (VW == 2) {
+      const float2 t = *reinterpret_cast<const float2*>(p);
+      v[0] = t.x; v[1] = t.y;
+    } else {
+      v[0] = *p;
+    }
+  }
+  __device__ __forceinline__ void store(float* p) const {
+    if constexpr (VW == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else if constexpr (VW == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+    else *p = v[0];
+  }
+};
 
 struct Args {
   const float* rec;   // matrix-free point records (MF_REC floats per GLL point)
@@ -95,375 +168,550 @@ struct Args {
   const int* gptr;    // gather groups: slot range and dof numbers
   const int* gdof;
   int ngroups;
-  int n1;
   float *u, *r, *z, *p, *kp, *Y;
   const float* dp;    // inverted diagonal
   ColState* cs;
   PcgGlobal* G;
-  double* part;       // gather partials [grid][KR], update partials [grid][KR][4]
+  float2* part;       // block partials: phase B [KR][grid], phase C [2 KR][grid]
+  unsigned* count;    // barrier arrivals
   int chunk;          // iterations to run
+  int cached;         // elements whose maps and records a block keeps in shared memory
 };
 
 template <int KR>
 struct Shape {
-  static constexpr int TPE = NGLL * KR;
-  static constexpr int EPC = NT / TPE;         // elements per block pass of the apply
-  static constexpr int UF = NEDOF * KR;
-  static constexpr int SF = NGLL * 9 * KR;
+  static constexpr int VW = KR < 4 ? KR : 4;     // columns per piece
+  static constexpr int QPD = KR / VW;            // pieces per dof row
+  static constexpr int LPN = 3 * QPD;            // pieces per node
+  static constexpr int UF = NEDOF * VW;          // shared floats per warp: p of the element
+  static constexpr int FF = NGLL * 9 * VW;       //   and the fluxes at its points
+  static constexpr size_t SMEM = (size_t)NWARP * (UF + FF) * sizeof(float);
+  static constexpr int EF = NGLL * (MF_REC + 4);  // words per cached element: records, maps {dof x 3, position}
+  static constexpr int CACHE = (int)((220 * 1024 - SMEM) / (EF * sizeof(float)));
+  static_assert(NT % LPN == 0, "a thread keeps its columns");
 };
 
+__device__ __forceinline__ float dcoef(int i, int t) {   // D[i][t] of the GLL points -1, 0, 1
+  return i == 0 ? (t == 0 ? -1.5f : t == 1 ? 2.0f : -0.5f)
+                : i == 1 ? (t == 0 ? -0.5f : t == 1 ? 0.0f : 0.5f) : (t == 0 ? 0.5f : t == 1 ? -2.0f : 1.5f);
+}
+
+// Element products of one warp: element e, columns c0 .. c0 + VW - 1.
 template <int KR>
-__global__ void __launch_bounds__(NT, 4) k_pcg_persistent(Args A) {
+__device__ __forceinline__ void element_product(const Args& A, int e, const float* cache, int c0, int lane,
+                                                const float (&beta)[Shape<KR>::VW], float* U, float* F) {
   using S = Shape<KR>;
-  static_assert(S::EPC >= 1, "KR up to 8");
-  __shared__ __align__(16) float sU[S::EPC][S::UF];
-  __shared__ __align__(16) float sF[S::EPC][S::SF];
-  __shared__ double sred[NT / 32][KR][4];
-  __shared__ double sfin[NT];
+  constexpr int VW = S::VW;
+  const int a = lane;
+  Vec<VW> u[3];
+  int q = -1;
+  float Ji[9], c11 = 0.f, c12 = 0.f, c44 = 0.f;
+  if (a < NGLL) {
+    int gd[3];
+    float4 r0, r1, r2;
+    if (cache) {
+      const float4* Rp = reinterpret_cast<const float4*>(cache) + 4 * a;
+      const int4 m = *reinterpret_cast<const int4*>(Rp + 3);
+      r0 = Rp[0]; r1 = Rp[1]; r2 = Rp[2];
+      gd[0] = m.x; gd[1] = m.y; gd[2] = m.z; q = m.w;
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) gd[c] = __ldg(A.ge + (size_t)e * NEDOF + 3 * a + c);
+      q = __ldg(A.pos + (size_t)e * NGLL + a);
+      const float4* Rp = reinterpret_cast<const float4*>(A.rec + ((size_t)e * NGLL + a) * MF_REC);
+      r0 = __ldg(Rp); r1 = __ldg(Rp + 1); r2 = __ldg(Rp + 2);
+    }
+    Ji[0] = r0.x; Ji[1] = r0.y; Ji[2] = r0.z; Ji[3] = r0.w; Ji[4] = r1.x; Ji[5] = r1.y; Ji[6] = r1.z; Ji[7] = r1.w;
+    Ji[8] = r2.x; c11 = r2.y; c12 = r2.z; c44 = r2.w;
+    Vec<VW> pv[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      pv[c].load_cg(A.p + (size_t)gd[c] * KR + c0);
+      u[c].load_cg(A.z + (size_t)gd[c] * KR + c0);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+      for (int k = 0; k < VW; ++k) u[c].v[k] = fmaf(beta[k], pv[c].v[k], u[c].v[k]);
+      u[c].store(U + (3 * a + c) * VW);
+    }
+  }
+  __syncwarp();
+  const int ic[3] = {a % 3, (a / 3) % 3, a / 9};
+  if (a < NGLL) {
+    // reference gradient gr[c][r], the line's nodes in order
+    Vec<VW> gr[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      constexpr int st[3] = {1, 3, 9};
+      const float* ul = U + 3 * (a - ic[r] * st[r]) * VW;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int tt = 0; tt < 3; ++tt) {
+          const float d = dcoef(ic[r], tt);
+          Vec<VW> x;
+          x.load(ul + (3 * tt * st[r] + c) * VW);
+#pragma unroll
+          for (int k = 0; k < VW; ++k) gr[c][r].v[k] = tt == 0 ? d * x.v[k] : fmaf(d, x.v[k], gr[c][r].v[k]);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < VW; ++k) {
+      float gp[3][3], T[3][3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          gp[c][d] = fmaf(Ji[3 * d], gr[c][0].v[k], fmaf(Ji[3 * d + 1], gr[c][1].v[k], Ji[3 * d + 2] * gr[c][2].v[k]));
+      T[0][0] = fmaf(c11, gp[0][0], c12 * (gp[1][1] + gp[2][2]));
+      T[1][1] = fmaf(c11, gp[1][1], c12 * (gp[0][0] + gp[2][2]));
+      T[2][2] = fmaf(c11, gp[2][2], c12 * (gp[0][0] + gp[1][1]));
+      T[0][1] = T[1][0] = c44 * (gp[0][1] + gp[1][0]);
+      T[1][2] = T[2][1] = c44 * (gp[1][2] + gp[2][1]);
+      T[0][2] = T[2][0] = c44 * (gp[0][2] + gp[2][0]);
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+          gr[c][r].v[k] = fmaf(Ji[r], T[c][0], fmaf(Ji[3 + r], T[c][1], Ji[6 + r] * T[c][2]));
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int r = 0; r < 3; ++r) gr[c][r].store(F + (9 * a + 3 * r + c) * VW);
+  }
+  __syncwarp();
+  if (a < NGLL) {
+    // rows of node a: the xi, eta and zeta fluxes of its lines in order
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      constexpr int st[3] = {1, 3, 9};
+      const float* fl = F + (9 * (a - ic[r] * st[r]) + 3 * r) * VW;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int tt = 0; tt < 3; ++tt) {
+          const float d = dcoef(tt, ic[r]);
+          Vec<VW> x;
+          x.load(fl + (9 * tt * st[r] + c) * VW);
+#pragma unroll
+          for (int k = 0; k < VW; ++k) u[c].v[k] = r == 0 && tt == 0 ? d * x.v[k] : fmaf(d, x.v[k], u[c].v[k]);
+        }
+    }
+    if (q >= 0) {
+      float* dst = A.Y + (size_t)q * 3 * KR + c0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) u[c].store(dst + c * KR);
+    }
+  }
+}
+
+// R pieces per thread in registers; R = 0: streamed.
+template <int KR, int R>
+__global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
+  using S = Shape<KR>;
+  constexpr int VW = S::VW, QPD = S::QPD, LPN = S::LPN;
+  constexpr int RR = R > 0 ? R : 1;
+  extern __shared__ __align__(16) float smem[];
+  __shared__ float2 sred[2 * KR][NWARP + 1];
   // block-local copy of the column state (identical in every block)
-  __shared__ double c_rz[KR], c_alpha[KR], c_beta[KR], c_tol[KR], c_rr0[KR], c_maxp[KR], c_maxu[KR], c_rr[KR];
-  __shared__ int c_active[KR], c_done[KR], c_iters[KR], c_failed[KR];
-  __shared__ int s_it, s_alldone;
+  __shared__ float2 c_rz[KR], c_alpha[KR], c_beta[KR], c_rr[KR], c_goal[KR];
+  __shared__ int c_live[KR], c_iters[KR], c_failed[KR];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   PcgGlobal* G = A.G;
   if (G->all_done) return;
   if (t < KR) {
     const ColState c = A.cs[t];
-    c_rz[t] = c.rz; c_alpha[t] = c.alpha; c_beta[t] = c.beta; c_tol[t] = c.tol; c_rr0[t] = c.rr0;
-    c_maxp[t] = c.maxp; c_maxu[t] = c.maxu; c_rr[t] = c.rr;
-    c_active[t] = c.active; c_done[t] = c.done; c_iters[t] = c.iters; c_failed[t] = c.failed;
+    c_rz[t] = split(c.rz); c_alpha[t] = split(c.alpha); c_beta[t] = split(c.beta); c_rr[t] = split(c.rr);
+    c_goal[t] = split(c.tol * c.tol * c.rr0);   // |r|^2 at which the column stops
+    c_live[t] = c.active && !c.done; c_iters[t] = c.iters; c_failed[t] = c.failed;
   }
-  if (t == 0) { s_it = G->it; s_alldone = 0; }
-  const int maxiter = G->maxiter, mode = G->mode, kcols = G->kcols;
+  int itn = G->it, alldone = 0;
+  const int maxiter = G->maxiter, kcols = G->kcols;
+  const int grid = gridDim.x, bid = blockIdx.x;
+  unsigned arrivals = 0;
+
+  // Grid barrier: earlier writes of the block are visible to every block
+  // after it.  Returns false when the wait ran out.
+  auto barrier = [&]() -> bool {
+    __syncthreads();
+    bool good = true;
+    if (t == 0) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(A.count) : "memory");
+      arrivals += (unsigned)grid;
+      unsigned n;
+      int tries = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(A.count) : "memory");
+        if (++tries > POLL_TRIES) good = false;
+      } while (n < arrivals && good);
+      if (!good) atomicExch(&G->err, 1);
+    }
+    return !__syncthreads_or(!good);
+  };
+  // sred[v][warp] summed over warps into this block's column of the partials
+  // (the maximum of the high parts when MAXOP); 32 / NV lanes per value
+  auto publish = [&](auto nvc, auto maxc, float2* out) {
+    constexpr int NV = decltype(nvc)::value;
+    constexpr bool MAXOP = decltype(maxc)::value;
+    __syncthreads();
+    if (warp == 0) {
+      constexpr int SUB = NV >= 32 ? 1 : (32 / NV > 8 ? 8 : 32 / NV);
+      const int v = lane / SUB, s = lane % SUB;
+      CompSum x[1];
+      if (v < NV)
+        for (int w = s; w < NWARP; w += SUB) {
+          if (MAXOP) x[0].hi = fmaxf(x[0].hi, sred[v][w].x);
+          else x[0].add(sred[v][w]);
+        }
+      if (MAXOP) {
+#pragma unroll
+        for (int o = SUB / 2; o >= 1; o >>= 1) x[0].hi = fmaxf(x[0].hi, __shfl_xor_sync(0xffffffffu, x[0].hi, o));
+      } else {
+        Reduce<1, SUB / 2, 1>::run(x, lane);
+      }
+      if (v < NV && s == 0) __stcg(out + (size_t)v * grid + bid, x[0].pair());
+    }
+  };
+  // sum over the blocks of one value's partials, by one warp
+  auto block_sum = [&](const float2* in) -> CompSum {
+    constexpr int NB = (MAX_BLOCKS + 31) / 32;
+    float2 w[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) w[i] = lane + 32 * i < grid ? __ldcg(in + lane + 32 * i) : make_float2(0.f, 0.f);
+    CompSum x[1];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) x[0].add(w[i]);
+    Reduce<1, 16, 1>::run(x, lane);
+    return x[0];
+  };
+
+  // the thread's pieces: columns c0 .. c0 + VW - 1 of dof row d of nodes g0, g0 + gstride, ...
+  const int qp = t % LPN, d = qp / QPD, c0 = VW * (qp % QPD);
+  const int gstride = grid * (NT / LPN);
+  // consecutive nodes stay in one block
+  const int g0 = bid * (NT / LPN) + t / LPN;
+  Vec<VW> ru[RR], rr[RR], rp[RR], rk[RR];
+  int gd[RR], sa[RR], sb[RR];
+  float dv[RR];
+  if constexpr (R > 0) {
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+      const int g = g0 + m * gstride;
+      gd[m] = g < A.ngroups ? A.gdof[3 * g + d] : 0;
+      sa[m] = g < A.ngroups ? A.gptr[g] : 0;
+      sb[m] = g < A.ngroups ? A.gptr[g + 1] : 0;
+      dv[m] = A.dp[gd[m]];
+      const size_t o = (size_t)gd[m] * KR + c0;
+      ru[m].load_cg(A.u + o);
+      rr[m].load_cg(A.r + o);
+      rp[m].load_cg(A.p + o);
+    }
+  }
+  float* U = smem + (size_t)warp * (S::UF + S::FF);
+  float* F = U + S::UF;
+  float2* partB = A.part;
+  float2* partC = A.part + (size_t)grid * KR;
+  // the block's run of (element, column group) pairs
+  const int nw = A.nelmt * QPD, per = (nw + grid - 1) / grid, w0 = bid * per, w1 = min(nw, w0 + per);
+  float* cache = smem + (size_t)NWARP * (S::UF + S::FF);
+  const int e0 = w0 / QPD;
+  for (int i = t; i < A.cached * NGLL; i += NT) {
+    const int e = e0 + i / NGLL, a = i % NGLL;
+    if (e >= A.nelmt) break;
+    float4* o = reinterpret_cast<float4*>(cache) + 4 * i;
+    const float4* Rp = reinterpret_cast<const float4*>(A.rec + ((size_t)e * NGLL + a) * MF_REC);
+    const int* g = A.ge + (size_t)e * NEDOF + 3 * a;
+    o[0] = Rp[0]; o[1] = Rp[1]; o[2] = Rp[2];
+    *reinterpret_cast<int4*>(o + 3) = make_int4(g[0], g[1], g[2], A.pos[(size_t)e * NGLL + a]);
+  }
   __syncthreads();
-  const int grid = gridDim.x;
-  double* partg = A.part;                          // [grid][KR]
-  double* partu = A.part + (size_t)grid * KR;      // [grid][KR][4]
-  // apply-phase thread mapping: element slot el, node a, column j
-  const int el = t / S::TPE, rem = t - el * S::TPE;
-  const int a = rem / KR, ja = rem - a * KR;
-  const bool act = el < S::EPC;
-  float* U = sU[act ? el : 0];
-  float* F = sF[act ? el : 0];
-  // gather / update mapping: the column of a thread is fixed (NT % KR == 0)
-  const int jt = t % KR;
+
+  // warp sums of the thread's values (x[i] of column VW r + i % VW, r = lane
+  // class) into sred[(i / VW) KR + column][warp]
+  auto reduce_lanes = [&](auto& x) {
+    constexpr int N = sizeof(x) / sizeof(x[0]);
+    constexpr int LOGN = N == 8 ? 3 : N == 4 ? 2 : N == 2 ? 1 : 0;
+    Reduce<N, 16, QPD>::run(x, lane);
+    // bit 4 of the lane chose the upper half of the values, bit 3 of that half, ...
+    const int i = N == 1 ? 0 : lane >> (5 - LOGN), rest = lane & ((32 >> LOGN) - 1);
+    if (rest < QPD) sred[(i / VW) * KR + VW * rest + i % VW][warp] = x[0].pair();
+  };
+  // kp of one piece: the node's slots in element order, four loads in flight
+  auto slot_sum = [&](int a, int b, Vec<VW>& acc) {
+    const float* y = A.Y + VW * qp;
+    acc.zero();
+    for (int s0 = a; s0 < b; s0 += 4) {
+      Vec<VW> v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (s0 + k < b) v[k].load_cg(y + (size_t)(s0 + k) * 3 * KR);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (s0 + k < b)
+#pragma unroll
+          for (int c = 0; c < VW; ++c) acc.v[c] = acc.v[c] + v[k].v[c];
+    }
+  };
 
   for (int k = 0; k < A.chunk; ++k) {
-    // ---- phase A: element products of p = z + beta p_old (matrix-free) ----
-    {
-      const float beta = act ? (float)c_beta[ja] : 0.f;
-      const int estride = grid * S::EPC;
-      // software pipeline: the next element's p and z values load while this
-      // element computes (its dof numbers one element further ahead)
-      int e = blockIdx.x * S::EPC + el;
-      int gd[3], gdn[3];
-      float pv[3], zv[3];
+    // ---- A: element products ----
+    for (int w = w0 + warp; w < w1; w += NWARP) {
+      const int e = w / QPD, cc = VW * (w - e * QPD);
+      float beta[VW];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) gd[c] = (act && e < A.nelmt) ? __ldg(A.ge + (size_t)e * NEDOF + 3 * a + c) : 0;
+      for (int q = 0; q < VW; ++q) beta[q] = c_beta[cc + q].x;
+      element_product<KR>(A, e, e - e0 < A.cached ? cache + (size_t)(e - e0) * S::EF : nullptr, cc, lane, beta, U, F);
+      __syncwarp();
+    }
+    if (!barrier()) return;
+    // ---- B: kp, p and p.kp ----
+    bool live[VW];
+    float beta[VW];
+    CompSum dot[VW];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        pv[c] = ldf(A.p + (size_t)gd[c] * KR + ja);
-        zv[c] = ldf(A.z + (size_t)gd[c] * KR + ja);
+    for (int q = 0; q < VW; ++q) { live[q] = c_live[c0 + q] != 0; beta[q] = c_beta[c0 + q].x; }
+    if constexpr (R > 0) {
+#pragma unroll
+      for (int m = 0; m < R; ++m) {
+        slot_sum(sa[m], sb[m], rk[m]);
+        if (!gd[m]) continue;
+#pragma unroll
+        for (int q = 0; q < VW; ++q)
+          if (live[q]) {
+            // z = D r as phase C formed it
+            rp[m].v[q] = fmaf(beta[q], rp[m].v[q], dv[m] * rr[m].v[q]);
+            dot[q].add(rp[m].v[q], rk[m].v[q]);
+          }
+        rp[m].store(A.p + (size_t)gd[m] * KR + c0);
       }
-      for (int e0 = blockIdx.x * S::EPC; e0 < A.nelmt; e0 += estride, e += estride) {
-        const bool valid = act && e < A.nelmt;
-        if (act) {
+    } else {
+      for (int g = g0; g < A.ngroups; g += gstride) {
+        const int gq = __ldg(A.gdof + 3 * g + d);
+        const size_t o = (size_t)gq * KR + c0;
+        Vec<VW> pv, zv, acc;
+        pv.load_cg(A.p + o);
+        zv.load_cg(A.z + o);
+        slot_sum(__ldg(A.gptr + g), __ldg(A.gptr + g + 1), acc);
+        if (!gq) continue;
 #pragma unroll
-          for (int c = 0; c < 3; ++c) U[(3 * a + c) * KR + ja] = valid ? fmaf(beta, pv[c], zv[c]) : 0.f;
-        }
-        const int en = e + estride;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) gdn[c] = (act && en < A.nelmt) ? __ldg(A.ge + (size_t)en * NEDOF + 3 * a + c) : 0;
-        __syncthreads();
-        if (valid) {
-          const int ic[3] = {a % 3, (a / 3) % 3, a / 9};
-          const int st[3] = {1, 3, 9};
-          float gr[3][3];
-#pragma unroll
-          for (int rr = 0; rr < 3; ++rr) {
-            const int base = a - ic[rr] * st[rr];
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-#pragma unroll
-            for (int tt = 0; tt < 3; ++tt) {
-              const float d = Dm(ic[rr], tt);
-              const float* uu = U + (size_t)(3 * (base + tt * st[rr])) * KR + ja;
-              s0 = fmaf(d, uu[0], s0);
-              s1 = fmaf(d, uu[KR], s1);
-              s2 = fmaf(d, uu[2 * KR], s2);
-            }
-            gr[0][rr] = s0; gr[1][rr] = s1; gr[2][rr] = s2;
+        for (int q = 0; q < VW; ++q)
+          if (live[q]) {
+            pv.v[q] = fmaf(beta[q], pv.v[q], zv.v[q]);
+            dot[q].add(pv.v[q], acc.v[q]);
           }
-          const float4* R = reinterpret_cast<const float4*>(A.rec + ((size_t)e * NGLL + a) * MF_REC);
-          const float4 r0 = __ldg(R), r1 = __ldg(R + 1), r2 = __ldg(R + 2);
-          const float Ji[9] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x};
-          const float c11 = r2.y, c12 = r2.z, c44 = r2.w;
-          float gp[3][3];
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-              gp[c][d] = fmaf(Ji[3 * d], gr[c][0], fmaf(Ji[3 * d + 1], gr[c][1], Ji[3 * d + 2] * gr[c][2]));
-          const float exx = gp[0][0], eyy = gp[1][1], ezz = gp[2][2];
-          float T[3][3];
-          T[0][0] = fmaf(c11, exx, c12 * (eyy + ezz));
-          T[1][1] = fmaf(c11, eyy, c12 * (exx + ezz));
-          T[2][2] = fmaf(c11, ezz, c12 * (exx + eyy));
-          T[0][1] = T[1][0] = c44 * (gp[0][1] + gp[1][0]);
-          T[1][2] = T[2][1] = c44 * (gp[1][2] + gp[2][1]);
-          T[0][2] = T[2][0] = c44 * (gp[0][2] + gp[2][0]);
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int rr = 0; rr < 3; ++rr)
-              F[((3 * a + c) * 3 + rr) * KR + ja] =
-                  fmaf(Ji[rr], T[c][0], fmaf(Ji[3 + rr], T[c][1], Ji[6 + rr] * T[c][2]));
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          pv[c] = ldf(A.p + (size_t)gdn[c] * KR + ja);
-          zv[c] = ldf(A.z + (size_t)gdn[c] * KR + ja);
-        }
-        __syncthreads();
-        if (valid) {
-          const int ic[3] = {a % 3, (a / 3) % 3, a / 9};
-          const int st[3] = {1, 3, 9};
-          float y0 = 0.f, y1 = 0.f, y2 = 0.f;
-#pragma unroll
-          for (int rr = 0; rr < 3; ++rr) {
-            const int base = a - ic[rr] * st[rr];
-#pragma unroll
-            for (int tt = 0; tt < 3; ++tt) {
-              const float d = Dm(tt, ic[rr]);
-              const float* f = F + (size_t)((3 * (base + tt * st[rr])) * 3 + rr) * KR + ja;
-              y0 = fmaf(d, f[0], y0);
-              y1 = fmaf(d, f[3 * KR], y1);
-              y2 = fmaf(d, f[6 * KR], y2);
-            }
-          }
-          const int q = __ldg(A.pos + (size_t)e * NGLL + a);
-          if (q >= 0) {
-            float* dst = A.Y + (size_t)q * 3 * KR + ja;
-            dst[0] = y0;
-            dst[KR] = y1;
-            dst[2 * KR] = y2;
-          }
-        }
-        __syncthreads();
+        pv.store(A.p + o);
+        acc.store(A.kp + o);
       }
     }
-    if (!grid_barrier(G)) return;
+    reduce_lanes(dot);
+    publish(std::integral_constant<int, KR>{}, std::false_type{}, partB);
+    if (!barrier()) return;
+    for (int j = warp; j < KR; j += NWARP) {
+      const CompSum x = block_sum(partB + (size_t)j * grid);
+      if (lane == 0 && c_live[j]) c_alpha[j] = div2(c_rz[j], x.pair());
+    }
+    __syncthreads();
+    // ---- C: u, r, z and r.z, r.r ----
+    float alpha[VW];
+    CompSum zz[2 * VW];   // r.z of the thread's columns, then r.r
+#pragma unroll
+    for (int q = 0; q < VW; ++q) alpha[q] = live[q] ? c_alpha[c0 + q].x : 0.f;
+    if constexpr (R > 0) {
+#pragma unroll
+      for (int m = 0; m < R; ++m) {
+        if (!gd[m]) continue;
+        Vec<VW> zv;
+#pragma unroll
+        for (int q = 0; q < VW; ++q) {
+          if (live[q]) {
+            ru[m].v[q] = fmaf(alpha[q], rp[m].v[q], ru[m].v[q]);
+            rr[m].v[q] = fmaf(-alpha[q], rk[m].v[q], rr[m].v[q]);
+          }
+          zv.v[q] = dv[m] * rr[m].v[q];
+          zz[q].add(rr[m].v[q], zv.v[q]);
+          zz[VW + q].add(rr[m].v[q], rr[m].v[q]);
+        }
+        zv.store(A.z + (size_t)gd[m] * KR + c0);
+      }
+    } else {
+      for (int g = g0; g < A.ngroups; g += gstride) {
+        const int gq = __ldg(A.gdof + 3 * g + d);
+        if (!gq) continue;
+        const size_t o = (size_t)gq * KR + c0;
+        const float D = __ldg(A.dp + gq);
+        Vec<VW> pv, uv, rv, kv, zv;
+        pv.load_cg(A.p + o);
+        uv.load_cg(A.u + o);
+        rv.load_cg(A.r + o);
+        kv.load_cg(A.kp + o);
+#pragma unroll
+        for (int q = 0; q < VW; ++q) {
+          if (live[q]) {
+            uv.v[q] = fmaf(alpha[q], pv.v[q], uv.v[q]);
+            rv.v[q] = fmaf(-alpha[q], kv.v[q], rv.v[q]);
+          }
+          zv.v[q] = D * rv.v[q];
+          zz[q].add(rv.v[q], zv.v[q]);
+          zz[VW + q].add(rv.v[q], rv.v[q]);
+        }
+        uv.store(A.u + o);
+        rv.store(A.r + o);
+        zv.store(A.z + o);
+      }
+    }
+    reduce_lanes(zz);
+    publish(std::integral_constant<int, 2 * KR>{}, std::false_type{}, partC);
+    if (!barrier()) return;
+    // stop test and beta, identical in every block
+    ++itn;
+    for (int j = warp; j < KR; j += NWARP) {
+      const CompSum x = block_sum(partC + (size_t)j * grid), y = block_sum(partC + (size_t)(KR + j) * grid);
+      if (lane == 0 && c_live[j]) {
+        c_rr[j] = norm2(y.pair());
+        if ((c_rr[j].x - c_goal[j].x) + (c_rr[j].y - c_goal[j].y) <= 0.f) {
+          c_live[j] = 0; c_iters[j] = itn;
+        } else if (itn >= maxiter) {
+          c_live[j] = 0; c_failed[j] = 1; c_iters[j] = maxiter + 1;
+        } else {
+          c_beta[j] = div2(x.pair(), c_rz[j]);
+          c_rz[j] = x.pair();
+        }
+      }
+    }
+    __syncthreads();
+    alldone = !__syncthreads_or(t < kcols && c_live[t < KR ? t : 0]);
+    if (alldone) break;
+  }
 
-    // ---- phase B: kp = sum of the element products in element order; p = z + beta p ----
-    {
-      const bool live = c_active[jt] && !c_done[jt];
-      const float beta = (float)c_beta[jt];
-      CompSum dot;
-      const size_t items = (size_t)A.ngroups * 3 * KR;
-      for (size_t it = (size_t)blockIdx.x * NT + t; it < items; it += (size_t)grid * NT) {
-        const int g = (int)(it / (3 * KR)), c = (int)(it - (size_t)g * 3 * KR), d = c / KR;
-        const int s0 = __ldg(A.gptr + g), s1 = __ldg(A.gptr + g + 1);
-        float acc = 0.f;
-        for (int sl = s0; sl < s1; ++sl) acc = acc + ldf(A.Y + (size_t)sl * 3 * KR + c);
-        const int gd = __ldg(A.gdof + 3 * g + d);
-        if (!gd) continue;
-        float* pp = A.p + (size_t)gd * KR + jt;
-        if (live) {
-          const float pv = fmaf(beta, ldf(pp), ldf(A.z + (size_t)gd * KR + jt));
-          dot.add(pv, acc);
-          *pp = pv;
-        }
-        A.kp[(size_t)gd * KR + jt] = acc;
-      }
-      double v = dot.value();
+  // max|p| of each column's last step (a stopped column keeps its direction)
+  float mp[VW];
 #pragma unroll
-      for (int o = 16; o >= KR; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane < KR) sred[warp][lane][0] = v;
-      __syncthreads();
-      if (t < KR) {
-        double s = 0.0;
-        for (int w = 0; w < NT / 32; ++w) s += sred[w][t][0];
-        partg[(size_t)blockIdx.x * KR + t] = s;
-      }
-    }
-    if (!grid_barrier(G)) return;
-    // alpha = r.z / p.kp, the block partials summed in a fixed order
-    {
-      double v = 0.0;
-      for (int b = t / KR; b < grid; b += NT / KR) v += __ldcg(partg + (size_t)b * KR + jt);
-      sfin[t] = v;
-      __syncthreads();
-      if (t < KR) {
-        double s = 0.0;
-        for (int u = t; u < NT; u += KR) s += sfin[u];
-        if (c_active[t] && !c_done[t]) c_alpha[t] = c_rz[t] / s;
-      }
-      __syncthreads();
-    }
-
-    // ---- phase C: u += alpha p, r -= alpha kp, z = D r, norms and dots ----
-    {
-      const bool live = c_active[jt] && !c_done[jt];
-      const float alpha = (float)c_alpha[jt];
-      float mp = 0.f, mu = 0.f;
-      CompSum rz, rr;
-      if (live) {
-        const size_t items = (size_t)A.n1 * KR;
-        for (size_t i = (size_t)blockIdx.x * NT + t; i < items; i += (size_t)grid * NT) {
-          const float pv = ldf(A.p + i), uv = ldf(A.u + i), rv = ldf(A.r + i), kv = ldf(A.kp + i);
-          const float un = fmaf(alpha, pv, uv);
-          const float rn = fmaf(-alpha, kv, rv);
-          const float zn = __ldg(A.dp + i / KR) * rn;
-          A.u[i] = un;
-          A.r[i] = rn;
-          A.z[i] = zn;
-          mp = fmaxf(mp, fabsf(pv));
-          mu = fmaxf(mu, fabsf(un));
-          rz.add(rn, zn);
-          rr.add(rn, rn);
-        }
-      }
-      double q4[4] = {(double)mp, (double)mu, live ? rz.value() : 0.0, live ? rr.value() : 0.0};
+  for (int q = 0; q < VW; ++q) mp[q] = 0.f;
+  if constexpr (R > 0) {
 #pragma unroll
-      for (int o = 16; o >= KR; o >>= 1) {
-        q4[0] = fmax(q4[0], __shfl_xor_sync(0xffffffffu, q4[0], o));
-        q4[1] = fmax(q4[1], __shfl_xor_sync(0xffffffffu, q4[1], o));
-        q4[2] += __shfl_xor_sync(0xffffffffu, q4[2], o);
-        q4[3] += __shfl_xor_sync(0xffffffffu, q4[3], o);
-      }
-      if (lane < KR)
+    for (int m = 0; m < R; ++m) {
+      if (!gd[m]) continue;
+      const size_t o = (size_t)gd[m] * KR + c0;
+      ru[m].store(A.u + o);
+      rr[m].store(A.r + o);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) sred[warp][lane][q] = q4[q];
-      __syncthreads();
-      if (t < 4 * KR) {
-        const int j = t / 4, q = t % 4;
-        double s = 0.0;
-        for (int w = 0; w < NT / 32; ++w) s = (q < 2) ? fmax(s, sred[w][j][q]) : s + sred[w][j][q];
-        partu[((size_t)blockIdx.x * KR + j) * 4 + q] = s;
-      }
+      for (int q = 0; q < VW; ++q) mp[q] = fmaxf(mp[q], fabsf(rp[m].v[q]));
     }
-    if (!grid_barrier(G)) return;
-    // stop tests and beta, identical in every block
-    {
-      constexpr int NQ = 4 * KR;
-      const int q = t % 4;
-      double v = 0.0;
-      for (int idx = t; idx < grid * NQ; idx += NT) {
-        const double x = __ldcg(partu + idx);
-        v = (q < 2) ? fmax(v, x) : v + x;
-      }
-      sfin[t] = v;
-      __syncthreads();
-      const int itn = s_it + 1;
-      if (t == 0) s_alldone = 1;
-      __syncthreads();
-      if (t < KR) {
-        double amax = 0.0, bmax = 0.0, s = 0.0, qq = 0.0;
-        for (int u = t * 4; u < NT; u += NQ) {
-          amax = fmax(amax, sfin[u]); bmax = fmax(bmax, sfin[u + 1]); s += sfin[u + 2]; qq += sfin[u + 3];
-        }
-        if (c_active[t] && !c_done[t]) {
-          c_maxp[t] = amax; c_maxu[t] = bmax; c_rr[t] = qq;
-          const bool stop = ((mode & 1) == 0) ? (fabs(c_alpha[t]) * amax / bmax <= c_tol[t])
-                                              : (qq <= c_tol[t] * c_tol[t] * c_rr0[t]);
-          if (stop) {
-            c_done[t] = 1; c_iters[t] = itn;
-          } else if (itn >= maxiter) {
-            c_done[t] = 1; c_failed[t] = 1; c_iters[t] = maxiter + 1;
-          } else {
-            c_beta[t] = s / c_rz[t];
-            c_rz[t] = s;
-          }
-        }
-        if (t < kcols && c_active[t] && !c_done[t]) atomicAnd(&s_alldone, 0);
-      }
-      __syncthreads();
-      if (t == 0) s_it = itn;
-      __syncthreads();
-      if (s_alldone) break;
+  } else {
+    for (int g = g0; g < A.ngroups; g += gstride) {
+      const int gq = __ldg(A.gdof + 3 * g + d);
+      if (!gq) continue;
+      Vec<VW> pv;
+      pv.load_cg(A.p + (size_t)gq * KR + c0);
+#pragma unroll
+      for (int q = 0; q < VW; ++q) mp[q] = fmaxf(mp[q], fabsf(pv.v[q]));
     }
   }
+#pragma unroll
+  for (int q = 0; q < VW; ++q) {
+#pragma unroll
+    for (int o = 16; o >= QPD; o >>= 1) mp[q] = fmaxf(mp[q], __shfl_xor_sync(0xffffffffu, mp[q], o));
+    if (lane < QPD) sred[VW * lane + q][warp] = make_float2(mp[q], 0.f);
+  }
+  publish(std::integral_constant<int, KR>{}, std::true_type{}, partB);
+  if (!barrier()) return;
   // the column state leaves with block 0
-  if (blockIdx.x == 0) {
+  if (bid == 0) {
     if (t < KR) {
       ColState& c = A.cs[t];
-      c.rz = c_rz[t]; c.alpha = c_alpha[t]; c.beta = c_beta[t]; c.maxp = c_maxp[t]; c.maxu = c_maxu[t];
-      c.rr = c_rr[t]; c.done = c_done[t]; c.iters = c_iters[t]; c.failed = c_failed[t];
+      float m = 0.f;
+      for (int b = 0; b < grid; ++b) m = fmaxf(m, __ldcg(partB + (size_t)t * grid + b).x);
+      if (c.active) {
+        c.rz = value(c_rz[t]); c.alpha = value(c_alpha[t]); c.beta = value(c_beta[t]); c.rr = value(c_rr[t]);
+        c.maxp = m; c.done = !c_live[t]; c.iters = c_iters[t]; c.failed = c_failed[t];
+      }
     }
     if (t == 0) {
-      G->it = s_it;
-      G->all_done = s_alldone;
+      G->it = itn;
+      G->all_done = alldone;
     }
   }
-}
-
-template <int KR>
-int max_blocks() {
-  static int per_sm = -1;
-  if (per_sm < 0) {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_pcg_persistent<KR>, NT, 0) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    per_sm = n;
-  }
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  return per_sm * nsm;
 }
 
 }  // namespace pp
 
-// Per PCG iteration with 8 trials, persistent against separate kernels:
-// 22.7 against 34.2 us at 270 elements, 33.5 against 39.9 at 1,125; at 3,000
-// and above the separate kernels are as fast or faster.
-int persist_max_elements() { return 1500; }
+// Largest mesh that takes the persistent chunk: where a phase has more work
+// than 15 warps per SM hide, separate launches with their own register budgets
+// win.  us per iteration of a whole trial, persistent against separate kernels:
+//   elements x columns   576 x 1   576 x 8   3289 x 8   5880 x 16   16000 x 8   12000 x 16   16000 x 1
+//   persistent              11.0      18.8         39         108         133          212          32
+//   separate                36.0      48.8         69         118         134          187          61
+// (with flags polled by every block and FP64 sums it was 21, 31 and 50 us for
+// the first three).
+int persist_max_elements(int KR) { return 130000 / KR; }
 
 bool persist_enabled() {
   static const bool on = !(getenv("SG_PERSIST") && atoi(getenv("SG_PERSIST")) == 0);
   return on;
 }
 
-// Runs `chunk` PCG iterations of the FP32 solve as one cooperative launch.
-// Returns false when the launch is not possible (the caller then runs the
-// separate kernels).
-template <int KR>
-bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int* pos, const GatherTopo& T, int n1,
-                           float* u, float* r, float* z, float* p, float* kp, float* Y, const float* dp,
-                           ColState* cs, PcgGlobal* G, double* part, int chunk, cudaStream_t s) {
-  if constexpr (KR > 8) {
-    return false;
-  } else {
-    using S = pp::Shape<KR>;
-    int cap = pp::max_blocks<KR>();
-    // the barrier's cost grows with the number of blocks: at most one block
-    // per SM (33.5 against 36.2 us per iteration with two at 1,125 elements),
-    // about four element passes of the apply per block
-    if (cap > 152) cap = 152;
-    int grid = (nelmt + 4 * S::EPC - 1) / (4 * S::EPC);
-    if (grid > cap) grid = cap;
-    if (grid < 1) return false;
-    // the partial buffer holds NPART * 16 * 4 doubles
-    if ((size_t)grid * KR * 5 > (size_t)NPART * 16 * 4) return false;
-    // a barrier count left behind by an earlier launch would release the
-    // first barrier early: start every launch from zero arrivals
-    cudaMemsetAsync(&G->cntB, 0, sizeof(unsigned), s);
-    pp::Args A{rec, ge, nelmt, pos, T.d_ptr, T.d_dof, T.ngroups, n1, u, r, z, p, kp, Y, dp, cs, G, part, chunk};
-    void* args[] = {&A};
-    if (cudaLaunchCooperativeKernel((const void*)pp::k_pcg_persistent<KR>, grid, pp::NT, args, 0, s) !=
-        cudaSuccess) {
+template <int KR, int R>
+static bool launch_persistent(const pp::Args& A, int grid, size_t smem, cudaStream_t s) {
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(pp::k_pcg_persistent<KR, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             220 * 1024) != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
-    add_launches(1);
-    return true;
+    attr = true;
   }
+  pp::Args a = A;
+  void* args[] = {&a};
+  if (cudaLaunchCooperativeKernel((const void*)pp::k_pcg_persistent<KR, R>, grid, pp::NT, args, smem, s) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  add_launches(1);
+  return true;
 }
 
-#define SG_PP_INST(KR)                                                                                              \
-  template bool launch_pcg_persistent<KR>(const float*, const int*, int, const int*, const GatherTopo&, int, float*, \
-                                          float*, float*, float*, float*, float*, const float*, ColState*,          \
+// Runs up to `chunk` PCG iterations of the FP32 solve (residual test) as one
+// cooperative launch.  Returns false when the launch is not possible (the
+// caller then runs the separate kernels).
+template <int KR>
+bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int* pos, const GatherTopo& T, float* u,
+                           float* r, float* z, float* p, float* kp, float* Y, const float* dp, ColState* cs,
+                           PcgGlobal* G, double* part, int chunk, cudaStream_t s) {
+  using S = pp::Shape<KR>;
+  // one block per SM, fewer where that still gives every scheduler of the
+  // SMs in use no more than one warp of phase A
+  long warps = (long)nelmt * S::QPD, pieces = (long)T.ngroups * S::LPN;
+  long grid = (warps + 3) / 4;
+  if (grid < (pieces + pp::NT - 1) / pp::NT) grid = (pieces + pp::NT - 1) / pp::NT;
+  if (grid > pp::MAX_BLOCKS) grid = pp::MAX_BLOCKS;
+  if (grid < 1) return false;
+  const long per = (pieces + grid * pp::NT - 1) / (grid * pp::NT);   // pieces per thread
+  // the block partials (3 KR pairs per block) and, behind them, the barrier count
+  const size_t np = (size_t)grid * 3 * KR * sizeof(float2);
+  static_assert((size_t)pp::MAX_BLOCKS * 3 * KR * sizeof(float2) + 64 <= (size_t)NPART * 16 * 4 * sizeof(double),
+                "partials fit the buffer");
+  unsigned* count = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(part) + np);
+  cudaMemsetAsync(count, 0, sizeof(unsigned), s);
+  // elements a block works on: its run of pairs touches at most this many
+  const long runs = (warps + grid - 1) / grid;
+  long cached = (runs + S::QPD - 1) / S::QPD + (S::QPD > 1 ? 1 : 0);
+  if (cached > S::CACHE) cached = S::CACHE;
+  const size_t smem = S::SMEM + (size_t)cached * S::EF * sizeof(float);
+  const pp::Args A{rec, ge, nelmt, pos, T.d_ptr, T.d_dof, T.ngroups, u, r, z, p, kp, Y, dp, cs, G,
+                   reinterpret_cast<float2*>(part), count, chunk, (int)cached};
+  if (per <= 1) return launch_persistent<KR, 1>(A, (int)grid, smem, s);
+  if (per <= 2) return launch_persistent<KR, 2>(A, (int)grid, smem, s);
+  return launch_persistent<KR, 0>(A, (int)grid, smem, s);
+}
+
+#define SG_PP_INST(KR)                                                                                             \
+  template bool launch_pcg_persistent<KR>(const float*, const int*, int, const int*, const GatherTopo&, float*,    \
+                                          float*, float*, float*, float*, float*, const float*, ColState*,         \
                                           PcgGlobal*, double*, int, cudaStream_t);
 SG_PP_INST(1)
 SG_PP_INST(2)

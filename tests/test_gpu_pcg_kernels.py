@@ -42,3 +42,13 @@ def test_flat_gather_and_update_match_staged(tmp_path, dims, k):
     a = trials(dims, k, tmp_path, SG_PERSIST="0", SG_GATHER_VARIANT="1")
     b = trials(dims, k, tmp_path, SG_PERSIST="0", SG_GATHER_VARIANT="0")
     same(a, b)
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 8, 16])
+@pytest.mark.parametrize("dims", [(2, 2, 2), (13, 7, 9), (29, 11, 13)])
+def test_persistent_matches_separate_kernels(tmp_path, dims, k):
+    """8 elements (fewer warps than schedulers), 819 and 4,147 (one, two or
+    streamed pieces a thread by k; the element cache full and not)."""
+    a = trials(dims, k, tmp_path, SG_PERSIST="1")
+    b = trials(dims, k, tmp_path, SG_PERSIST="0")
+    same(a, b)
