@@ -75,6 +75,8 @@ struct sg_ctx {
     double *u = nullptr, *f = nullptr, *dp = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *kp = nullptr,
            *Y = nullptr, *part = nullptr;
     int n1cap = 0, necap = 0;
+    double* rows = nullptr;  // the matrices packed by rows
+    int rowcap = 0;
     ColState* cs = nullptr;
     PcgGlobal* G = nullptr;
   } dropin;
@@ -202,6 +204,7 @@ struct Op {
   const int* ge = nullptr;
   int nelmt = 0;
   const GatherTopo* T = nullptr;
+  const double* rows = nullptr;   // dense: the matrices packed by rows, where their pattern allows it
 };
 
 template <typename V>
@@ -313,10 +316,21 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
   bool persist = false;
   if constexpr (std::is_same<V, float>::value)
     persist = op.dense == 2 && (mode & 1) && op.nelmt < persist_max_elements(KR) && persist_enabled();
+  // FP64, one column: the matrices' products bound every size (sg_pcg_persist64.cu)
+  if constexpr (std::is_same<V, double>::value && KR == 1)
+    persist = !(mode & 1) && (op.dense == 0 ? persist_default_apply() : op.rows != nullptr) && persist_enabled();
   constexpr int persist_chunk = 512;
   int nchunks = 0;
   while (true) {
     bool done_chunk = false;
+    if constexpr (std::is_same<V, double>::value && KR == 1)
+      if (persist) {
+        ev = C->prof_begin();
+        done_chunk = launch_pcg_persistent64(op.dense != 0, op.dense ? op.rows : (const double*)op.K, op.ge, op.nelmt,
+                                             op.T->d_pos, C->d_nbr, *op.T, n1, u, B.r, B.z, B.p, B.kp, B.Y, dp, B.cs,
+                                             B.G, B.part, persist_chunk, s);
+        C->prof_end(ev, 0);
+      }
     if constexpr (std::is_same<V, float>::value)
       if (persist) {
         ev = C->prof_begin();
@@ -570,6 +584,33 @@ int sg_pcg_solve(sg_ctx* c, int neq, int nelmt, int nedof, const double* k, doub
   cudaMemcpyAsync(D.dp, dprecon, sizeof(double) * n1, cudaMemcpyHostToDevice, s);
   Op op;
   op.dense = 1; op.K = D.d_K; op.ge = D.d_ge; op.nelmt = nelmt; op.T = &D.T;
+  // rows packed by the coupling pattern of 27-node elements, where every entry
+  // that the packing leaves out is zero and the room is no more than a quarter
+  // of what the budget has left (the solve also runs without)
+  if (persist_enabled() && nelmt > 0) {
+    const size_t room = sizeof(double) * (size_t)nelmt * ROW_STRIDE;
+    if (D.rowcap < nelmt) {
+      c->release(D.rows);
+      D.rows = nullptr;
+      if (c->used <= c->budget && room <= (c->budget - c->used) / 4) {
+        const std::string before = c->err;
+        D.rows = c->alloc<double>((size_t)nelmt * ROW_STRIDE);
+        if (!D.rows) c->err = before;
+      }
+      D.rowcap = D.rows ? nelmt : 0;
+    }
+    if (D.rows) {
+      int other = 1;
+      launch_pack_rows(D.d_K, nelmt, c->d_nbr, D.rows, c->d_err, s);
+      cudaMemcpyAsync(&other, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, s);
+      cudaMemsetAsync(c->d_err, 0, sizeof(int), s);
+      if (!c->check(cudaStreamSynchronize(s), "sg_pcg_solve")) {
+        set_tag(errtag, "ERROR: CUDA failure: " + c->err);
+        return SG_ERR_CUDA;
+      }
+      if (!other) op.rows = D.rows;
+    }
+  }
   PcgBufs<double> B;
   B.r = D.r; B.z = D.z; B.p = D.p; B.kp = D.kp; B.Y = D.Y; B.part = D.part; B.cs = D.cs; B.G = D.G;
   int active = 1, it = 0, failed = 0;

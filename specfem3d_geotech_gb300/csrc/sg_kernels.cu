@@ -429,6 +429,7 @@ constexpr int MF_AUTO_MAX = 100000;
 int g_apply_variant = 5;
 void set_apply_variant(int v) { g_apply_variant = v; }
 bool fp32_matrix_free(int nelmt) { return g_apply_variant == 4 || (g_apply_variant == 5 && nelmt < MF_AUTO_MAX); }
+bool persist_default_apply() { return g_apply_variant >= 2; }
 // device copy of the stored-entry table, needed by the tensor-core apply
 const int* g_entry_dev = nullptr;
 void set_entry_table(const int* d_entry) { g_entry_dev = d_entry; }
@@ -1384,7 +1385,7 @@ void pcg_gather(const GatherTopo& T, const V* Y, V* kp, V* p, const V* z, int mo
     cudaFuncSetAttribute(k_pcg_gather<V, KR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     attr = true;
   }
-  SG_LAUNCH k_pcg_gather<V, KR><<<red_grid(T.ngroups, GATHER_WARPS * 32 * 2, NPART), RED_THREADS, sm, s>>>(T.d_ptr, T.d_ent, T.d_dof, T.ngroups, Y, kp, p, z, mode,
+  SG_LAUNCH k_pcg_gather<V, KR><<<red_grid(T.ngroups, VGATHER, NPART), RED_THREADS, sm, s>>>(T.d_ptr, T.d_ent, T.d_dof, T.ngroups, Y, kp, p, z, mode,
                                                               cs, G, part);
 }
 
@@ -1754,7 +1755,7 @@ void pcg_update(int n1, V* u, V* r, V* z, const V* p, const V* kp, const V* f, c
         n1, u, r, z, p, kp, f, dprecon, init, cs, G, part);
     return;
   }
-  SG_LAUNCH k_pcg_update<V, KR><<<red_grid((size_t)n1 * KR, RED_THREADS * 4, NPART), RED_THREADS, 0, s>>>(
+  SG_LAUNCH k_pcg_update<V, KR><<<red_grid((size_t)n1 * KR, VUPDATE, NPART), RED_THREADS, 0, s>>>(
       n1, u, r, z, p, kp, f, dprecon, init, cs, G, part);
 }
 

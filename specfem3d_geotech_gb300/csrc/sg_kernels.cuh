@@ -46,6 +46,7 @@ void add_launches(long long n);  // kernels launched through a replayed CUDA gra
 void set_apply_variant(int v);   // 0 register-staged, 1 TMA pipeline, 2 tensor cores for 8/16 FP32 RHS,
                                  // 3 lane per (element, RHS) for 8/16 FP32 RHS, 4 matrix-free FP32,
                                  // 5 (default) 3 with matrix-free FP32 on small meshes
+bool persist_default_apply();    // the chosen variant leaves the FP64 apply at its default
 void set_entry_table(const int* d_entry);
 // The element applies that wait on mbarriers set *err to 1 when a bounded
 // wait runs out (err is the calling solve's own word, never shared between
@@ -98,6 +99,17 @@ bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int
                            PcgGlobal* G, double* part, int chunk, cudaStream_t s);
 bool persist_enabled();                 // SG_PERSIST=0 turns the persistent chunk off
 int persist_max_elements(int KR);       // meshes below this use it
+// FP64 solve of one right-hand side as a persistent cooperative kernel
+// (sg_pcg_persist64.cu), bitwise the separate kernels' solve; false when it
+// cannot run.  rows: K packed by launch_pack_rows, whose *other says that a
+// matrix has entries the packing drops.
+constexpr int ROW_STRIDE = 4618;   // doubles per packed element: 57 x 81, padded to 16 bytes
+constexpr int VGATHER = RED_THREADS * 2, VUPDATE = RED_THREADS * 4;   // items per block of the FP64 gather and update
+void launch_pack_rows(const double* K, int nelmt, const int* d_nbr, double* out, int* other, cudaStream_t s);
+bool launch_pcg_persistent64(bool rows, const double* K, const int* ge, int nelmt, const int* pos, const int* d_nbr,
+                             const GatherTopo& T, int n1, double* u, double* r, double* z, double* p, double* kp,
+                             double* Y, const double* dp, ColState* cs, PcgGlobal* G, double* part, int chunk,
+                             cudaStream_t s);
 void set_gather_variant(int v);  // 1 flat gather for FP32 (default), 0 staged
 template <typename V, int KR>
 // Y receives element slot (e, a)'s three rows (x KR) at the slot's gather

@@ -1,0 +1,469 @@
+// sg_pcg_persist64.cu -- the FP64 PCG iterations (one right-hand side) as one
+// persistent cooperative kernel, for the model's stored sparse matrices and
+// for the drop-in's dense ones.
+//
+// What bounds it: the FP64 unit takes a warp instruction in some 19 cycles, so
+// the element products (171 fused multiply-adds a lane with lane = node and 27
+// of 32 lanes at work) are nearly all of an iteration from a few thousand
+// elements on, and below that the launches, tails and round trips of three
+// kernels are.  So
+//   * a lane is one row of an element's product and the rows of a block's
+//     elements are cut into warps without regard to element borders: no lane
+//     idles (144 FP64 instructions an element instead of 171, or of the 243 of
+//     a dense column sweep);
+//   * only the 57 columns a row can be coupled to are multiplied.  The
+//     drop-in's dense matrices are checked for that pattern on the device once
+//     per call (k_pack_rows) and packed; matrices that do not have it take the
+//     dense kernel;
+//   * a block's matrices stay in shared memory for the whole launch while they
+//     fit, else they stream through two buffers filled by bulk copies, the
+//     next iteration's first group on its way during the vector phases;
+//   * the phases of an iteration are separated by the counter barrier of
+//     sg_pcg_persist.cu.
+//
+// The arithmetic and its order are those of k_apply_dense64 / k_apply_sparse*,
+// k_pcg_gather and k_pcg_update: products in column order (an exact zero adds
+// nothing), slots in element order, and dots over the same virtual grid of
+// 256-thread blocks with the same trees, so a solve is bitwise the one of the
+// separate kernels.
+//
+// us per iteration, separate kernels (with short tails) -> this: 300 elements
+// dense 43 -> 22, sparse 37 -> 22; 12,000 elements sparse 256 -> 170.
+//
+// Every wait is bounded; a timeout sets the solve's error word, the block
+// waits (bounded) for its own copies and leaves, and the others follow.
+#include <cstdint>
+#include <cstdlib>
+#include <type_traits>
+
+#include "sg_kernels.cuh"
+
+namespace sg {
+
+namespace p64 {
+
+constexpr int NT = 512, NWARP = NT / 32;
+constexpr int MAX_BLOCKS = 152;
+constexpr int POLL_TRIES = 1 << 20;
+constexpr int VT = RED_THREADS;          // threads of a virtual block
+constexpr unsigned FULL = 0xffffffffu;
+
+template <bool ROWS>
+struct Lay {
+  static constexpr int STRIDE = ROWS ? ROW_STRIDE : KS_STRIDE;        // doubles per element
+  static constexpr int GE = ROWS ? 2 : 5;                             // elements per streamed group
+  static constexpr int RES = ROWS ? 5 : 10;                           // elements that stay in shared memory
+  static constexpr int NP = RES > 2 * GE ? RES : 2 * GE;              // direction slots
+  static constexpr size_t SMEM = (size_t)NP * (STRIDE + NEDOF) * sizeof(double);
+  static_assert(RES <= NP && 2 * GE <= NP && GE * NEDOF <= NT, "buffers");
+  static_assert((STRIDE * sizeof(double)) % 16 == 0, "bulk copies");
+};
+
+struct Args {
+  const double* K;
+  const int *ge, *pos, *nbr;
+  int nelmt;
+  const int *gptr, *gdof;
+  int ngroups, n1, ggrid, ugrid;         // virtual grids of the gather and the update
+  double *u, *r, *z, *p, *kp, *Y;
+  const double* dp;
+  ColState* cs;
+  PcgGlobal* G;
+  double* part;                          // p.kp [ggrid], r.z, max|p|, max|u| [ugrid] each
+  unsigned* count;
+  int chunk;
+};
+
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
+  for (int tries = 0; tries < (1 << 22); ++tries) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void half_sync(int h) { asm volatile("bar.sync %0, 256;" ::"r"(1 + h) : "memory"); }
+
+// Rows of `nel` elements whose matrices start at kb and directions at ps.
+template <bool ROWS>
+__device__ __forceinline__ void row_products(const Args& A, const double* kb, const double* ps, int efirst, int nel,
+                                             const int* nbr, int warp, int lane) {
+  using L = Lay<ROWS>;
+  for (int c = warp; c * 32 < nel * NEDOF; c += NWARP) {
+    const int row = c * 32 + lane;
+    if (row >= nel * NEDOF) continue;
+    const int el = row / NEDOF, rr = row - el * NEDOF, n = rr / 3, cc = rr - 3 * n;
+    const double* k = kb + (size_t)el * L::STRIDE;
+    const double* pe = ps + el * NEDOF;
+    const int* tb = nbr + n * KS_NBR;
+    double y = 0.0;
+#pragma unroll
+    for (int s = 0; s < KS_NBR; ++s) {
+      const int pk = tb[s], m = pk & 31;
+      if constexpr (ROWS) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) y = fma(k[(3 * s + d) * NEDOF + rr], pe[3 * m + d], y);
+      } else {
+        // stored (n, m) row-major, or (m, n) read transposed
+        const bool tr = ((pk >> 5) & 3) == 2;
+        const double* kk = k + (pk >> 8) + (tr ? cc : 3 * cc);
+        const int sd = tr ? 3 : 1;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) y = fma(kk[d * sd], pe[3 * m + d], y);
+      }
+    }
+    const int q = __ldg(A.pos + (size_t)(efirst + el) * NGLL + n);
+    if (q >= 0) A.Y[(size_t)q * 3 + cc] = y;
+  }
+}
+
+template <bool ROWS>
+__global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
+  using L = Lay<ROWS>;
+  extern __shared__ __align__(128) double dsm[];
+  double* kb = dsm;                                   // matrices: resident, or two groups
+  double* ps = dsm + (size_t)L::NP * L::STRIDE;       // directions of the same elements
+  __shared__ int nbr[NGLL * KS_NBR];
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ double sred[NWARP][3];
+  __shared__ double sfin[VT], sm1[NWARP], sm2[NWARP];
+  __shared__ double s_alpha, s_beta, s_rz, s_maxp, s_maxu;
+  __shared__ int s_done, s_failed;
+  PcgGlobal* G = A.G;
+  if (G->all_done) return;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, h = t / VT, tl = t % VT, vw = tl >> 5;
+  const int grid = gridDim.x, bid = blockIdx.x;
+  const double tol = A.cs[0].tol;
+  if (t == 0) {
+    s_rz = A.cs[0].rz; s_alpha = A.cs[0].alpha; s_beta = A.cs[0].beta;
+    s_maxp = A.cs[0].maxp; s_maxu = A.cs[0].maxu; s_done = 0; s_failed = 0;
+    for (int b = 0; b < 2; ++b)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar + b)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = t; i < NGLL * KS_NBR; i += NT) nbr[i] = A.nbr[i];
+  int it = G->it;
+  const int maxiter = G->maxiter;
+  unsigned arrivals = 0;
+  // the block's elements
+  const int per = (A.nelmt + grid - 1) / grid, e0 = min(A.nelmt, bid * per), nel = min(A.nelmt, e0 + per) - e0;
+  const bool resident = nel <= L::RES;
+  const int ngrp = (nel + L::GE - 1) / L::GE;
+  unsigned uses = 0;        // groups copied so far (buffer uses % 2), the same in all threads
+  unsigned waited = 0;
+  __syncthreads();
+  auto copy_group = [&](int g) {
+    if (t == 0) {
+      const int first = g * L::GE, n = min(L::GE, nel - first);
+      const unsigned b = uses & 1, bytes = (unsigned)n * L::STRIDE * 8;
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar + b)), "r"(bytes)
+                   : "memory");
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+              smem_u32(kb + (size_t)b * L::GE * L::STRIDE)),
+          "l"(A.K + (size_t)(e0 + first) * L::STRIDE), "r"(bytes), "r"(smem_u32(bar + b))
+          : "memory");
+    }
+    ++uses;
+  };
+  if (resident) {
+    const double2* src = reinterpret_cast<const double2*>(A.K + (size_t)e0 * L::STRIDE);
+    for (int i = t; i < nel * (L::STRIDE / 2); i += NT) reinterpret_cast<double2*>(kb)[i] = __ldcs(src + i);
+  } else {
+    copy_group(0);
+  }
+  auto barrier = [&]() -> bool {
+    __syncthreads();
+    bool good = true;
+    if (t == 0) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(A.count) : "memory");
+      arrivals += (unsigned)grid;
+      unsigned n;
+      int tries = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(A.count) : "memory");
+        if (++tries > POLL_TRIES) good = false;
+      } while (n < arrivals && good);
+      if (!good) atomicExch(&G->err, 1);
+    }
+    return !__syncthreads_or(!good);
+  };
+  // direction value i of the elements from first on
+  auto direction = [&](int first, int i) -> double {
+    const int gd = __ldg(A.ge + (size_t)(e0 + first) * NEDOF + i);
+    return fma(s_beta, __ldcg(A.p + gd), __ldcg(A.z + gd));
+  };
+  double* partB = A.part;
+  double *partZ = A.part + A.ggrid, *partP = partZ + A.ugrid, *partU = partP + A.ugrid;
+  bool ok = true;
+  for (int k = 0; k < A.chunk && ok; ++k) {
+    // ---- element products of p = z + beta p_old ----
+    if (resident) {
+      for (int i = t; i < nel * NEDOF; i += NT) ps[i] = direction(0, i);
+      __syncthreads();
+      row_products<ROWS>(A, kb, ps, e0, nel, nbr, warp, lane);
+    } else {
+      if (t < min(L::GE, nel) * NEDOF) ps[t] = direction(0, t);
+      for (int g = 0; g < ngrp; ++g) {
+        const int b = waited & 1, n = min(L::GE, nel - g * L::GE), nn = min(L::GE, nel - (g + 1) * L::GE);
+        // the next group, or the next iteration's first, while this one is computed
+        copy_group(g + 1 < ngrp ? g + 1 : 0);
+        double nd = 0.0;
+        if (t < nn * NEDOF) nd = direction((g + 1) * L::GE, t);
+        ok = mbar_wait(bar + b, (waited >> 1) & 1);
+        if (__syncthreads_or(!ok)) { ok = false; break; }
+        ++waited;
+        row_products<ROWS>(A, kb + (size_t)b * L::GE * L::STRIDE, ps + (g & 1) * L::GE * NEDOF, e0 + g * L::GE, n, nbr,
+                           warp, lane);
+        if (t < nn * NEDOF) ps[((g + 1) & 1) * L::GE * NEDOF + t] = nd;
+        __syncthreads();
+      }
+      if (!ok) {
+        if (t == 0) atomicExch(&G->err, 1);
+        break;
+      }
+    }
+    if (!barrier()) { ok = false; break; }
+    // ---- kp, p and p.kp, a half block per virtual block ----
+    const double beta = s_beta;
+    for (int vb = bid + h * grid; vb < A.ggrid; vb += 2 * grid) {
+      double dot = 0.0;
+      for (int g = (vb * (VT / 32) + vw) * 32 + lane; g < A.ngroups; g += A.ggrid * VT) {
+        const int a = __ldg(A.gptr + g), b = __ldg(A.gptr + g + 1);
+        int gd[3];
+        double pv[3], zv[3], acc[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          gd[d] = __ldg(A.gdof + 3 * g + d);
+          pv[d] = __ldcg(A.p + gd[d]);
+          zv[d] = __ldcg(A.z + gd[d]);
+        }
+        for (int s0 = a; s0 < b; s0 += 4) {
+          double y[4][3];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) y[i][d] = s0 + i < b ? __ldcg(A.Y + (size_t)(s0 + i) * 3 + d) : 0.0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (s0 + i < b)
+#pragma unroll
+              for (int d = 0; d < 3; ++d) acc[d] = acc[d] + y[i][d];
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          if (!gd[d]) continue;
+          const double pn = fma(beta, pv[d], zv[d]);
+          dot = fma(pn, acc[d], dot);
+          A.p[gd[d]] = pn;
+          A.kp[gd[d]] = acc[d];
+        }
+      }
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) dot += __shfl_xor_sync(FULL, dot, o);
+      if (lane == 0) sred[warp][0] = dot;
+      half_sync(h);
+      if (tl == 0) {
+        double v = 0.0;
+        for (int w = 0; w < VT / 32; ++w) v += sred[h * (VT / 32) + w][0];
+        __stcg(partB + vb, v);
+      }
+      half_sync(h);
+    }
+    if (!barrier()) { ok = false; break; }
+    // alpha: the block partials in the order of the last block's sum
+    if (t < VT) {
+      double v = 0.0;
+      for (int i = t; i < A.ggrid; i += VT) v += __ldcg(partB + i);
+      sfin[t] = v;
+    }
+    __syncthreads();
+    if (t == 0) {
+      double s = 0.0;
+      const int n = min(VT, A.ggrid);
+      for (int i = 0; i < n; ++i) s += sfin[i];
+      s_alpha = s_rz / s;
+    }
+    __syncthreads();
+    // ---- u, r, z, max-norms and r.z ----
+    const double alpha = s_alpha;
+    for (int vb = bid + h * grid; vb < A.ugrid; vb += 2 * grid) {
+      double mp = 0.0, mu = 0.0, rz = 0.0;
+      const size_t stride = (size_t)A.ugrid * VT;
+      for (size_t i0 = (size_t)vb * VT + tl; i0 < (size_t)A.n1; i0 += 4 * stride) {
+        double pv[4], uv[4], rv[4], kv[4], dv[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const size_t i = i0 + q * stride;
+          if (i < (size_t)A.n1) {
+            pv[q] = __ldcg(A.p + i); uv[q] = __ldcg(A.u + i); rv[q] = __ldcg(A.r + i); kv[q] = __ldcg(A.kp + i);
+            dv[q] = __ldg(A.dp + i);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const size_t i = i0 + q * stride;
+          if (i >= (size_t)A.n1) continue;
+          const double un = fma(alpha, pv[q], uv[q]), rn = fma(-alpha, kv[q], rv[q]), zn = dv[q] * rn;
+          A.u[i] = un; A.r[i] = rn; A.z[i] = zn;
+          mp = fmax(mp, fabs(pv[q]));
+          mu = fmax(mu, fabs(un));
+          rz = fma(rn, zn, rz);
+        }
+      }
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) {
+        mp = fmax(mp, __shfl_xor_sync(FULL, mp, o));
+        mu = fmax(mu, __shfl_xor_sync(FULL, mu, o));
+        rz = rz + __shfl_xor_sync(FULL, rz, o);
+      }
+      if (lane == 0) { sred[warp][0] = mp; sred[warp][1] = mu; sred[warp][2] = rz; }
+      half_sync(h);
+      if (tl < 3) {
+        double v = 0.0;
+        for (int w = 0; w < VT / 32; ++w) {
+          const double x = sred[h * (VT / 32) + w][tl];
+          v = tl < 2 ? fmax(v, x) : v + x;
+        }
+        __stcg((tl == 0 ? partP : tl == 1 ? partU : partZ) + vb, v);
+      }
+      half_sync(h);
+    }
+    if (!barrier()) { ok = false; break; }
+    // stop test and beta, identical in every block: r.z over interleaved
+    // 64-block strides as the last block of k_pcg_update sums it
+    ++it;
+    {
+      constexpr int NJ = VT / 4;
+      double mp = 0.0, mu = 0.0;
+      if (t < NJ) {
+        double v = 0.0;
+        for (int b = t; b < A.ugrid; b += NJ) v += __ldcg(partZ + b);
+        sfin[t] = v;
+      } else {
+        for (int b = t - NJ; b < A.ugrid; b += NT - NJ) {
+          mp = fmax(mp, __ldcg(partP + b));
+          mu = fmax(mu, __ldcg(partU + b));
+        }
+      }
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) {
+        mp = fmax(mp, __shfl_xor_sync(FULL, mp, o));
+        mu = fmax(mu, __shfl_xor_sync(FULL, mu, o));
+      }
+      if (lane == 0) { sm1[warp] = mp; sm2[warp] = mu; }
+      __syncthreads();
+      if (t == 0) {
+        double s = 0.0;
+        const int n = min(NJ, A.ugrid);
+        for (int i = 0; i < n; ++i) s += sfin[i];
+        for (int w = 0; w < NWARP; ++w) { mp = fmax(mp, sm1[w]); mu = fmax(mu, sm2[w]); }
+        s_maxp = mp; s_maxu = mu;
+        if (fabs(s_alpha) * mp / mu <= tol) {
+          s_done = 1;
+        } else if (it >= maxiter) {
+          s_done = 1; s_failed = 1;
+        } else {
+          s_beta = s / s_rz;
+          s_rz = s;
+        }
+      }
+      __syncthreads();
+    }
+    if (s_done) break;
+  }
+  // copies still on their way must land before the block leaves (bounded)
+  for (; waited < uses; ++waited) mbar_wait(bar + (waited & 1), (waited >> 1) & 1);
+  if (!ok) return;
+  if (bid == 0 && t == 0) {
+    ColState& c = A.cs[0];
+    c.rz = s_rz; c.alpha = s_alpha; c.beta = s_beta; c.maxp = s_maxp; c.maxu = s_maxu;
+    if (s_done) { c.done = 1; c.failed = s_failed; c.iters = s_failed ? maxiter + 1 : it; }
+    G->it = it;
+    G->all_done = s_done;
+  }
+}
+
+// Packs dense column-major 81x81 matrices into [57][81]: entry (3 s + d, row)
+// is K(row, 3 m + d) with m the s-th node coupled to the row's node.  *other
+// is set when an entry outside that pattern is not zero (or is not a number).
+__global__ void __launch_bounds__(256) k_pack_rows(const double* __restrict__ K, const int* __restrict__ nbr_g,
+                                                   double* __restrict__ out, int* __restrict__ other) {
+  __shared__ signed char slot[NGLL][NGLL];   // s of (n, m), or -1
+  for (int i = threadIdx.x; i < NGLL * NGLL; i += blockDim.x) slot[i / NGLL][i % NGLL] = -1;
+  __syncthreads();
+  for (int i = threadIdx.x; i < NGLL * KS_NBR; i += blockDim.x) slot[i / KS_NBR][nbr_g[i] & 31] = (signed char)(i % KS_NBR);
+  __syncthreads();
+  const double* k = K + (size_t)blockIdx.x * NEDOF * NEDOF;
+  double* o = out + (size_t)blockIdx.x * ROW_STRIDE;
+  bool bad = false;
+  for (int i = threadIdx.x; i < NEDOF * NEDOF; i += blockDim.x) {
+    const int col = i / NEDOF, row = i - col * NEDOF, s = slot[row / 3][col / 3];
+    const double v = __ldcs(k + i);
+    if (s >= 0) o[(3 * s + col % 3) * NEDOF + row] = v;
+    else bad = bad || !(v == 0.0);
+  }
+  if (threadIdx.x < ROW_STRIDE - 3 * KS_NBR * NEDOF) o[3 * KS_NBR * NEDOF + threadIdx.x] = 0.0;
+  if (__syncthreads_or(bad) && threadIdx.x == 0) *other = 1;
+}
+
+template <bool ROWS>
+static bool launch(Args A, int grid, cudaStream_t s) {
+  using L = Lay<ROWS>;
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(k_pcg_persistent64<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    attr = true;
+  }
+  void* args[] = {&A};
+  if (cudaLaunchCooperativeKernel((const void*)k_pcg_persistent64<ROWS>, grid, NT, args, L::SMEM, s) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  add_launches(1);
+  return true;
+}
+
+}  // namespace p64
+
+void launch_pack_rows(const double* K, int nelmt, const int* d_nbr, double* out, int* other, cudaStream_t s) {
+  cudaMemsetAsync(other, 0, sizeof(int), s);
+  if (nelmt <= 0) return;
+  p64::k_pack_rows<<<nelmt, 256, 0, s>>>(K, d_nbr, out, other);
+  add_launches(1);
+}
+
+// Up to `chunk` PCG iterations (reference step test).  rows: K is packed by
+// k_pack_rows, else the sparse symmetric layout.  False when it cannot run.
+bool launch_pcg_persistent64(bool rows, const double* K, const int* ge, int nelmt, const int* pos, const int* d_nbr,
+                             const GatherTopo& T, int n1, double* u, double* r, double* z, double* p, double* kp,
+                             double* Y, const double* dp, ColState* cs, PcgGlobal* G, double* part, int chunk,
+                             cudaStream_t s) {
+  // the virtual grids are those of k_pcg_gather and k_pcg_update
+  auto red = [](size_t items, size_t per) {
+    const size_t g = (items + per - 1) / per;
+    return (int)(g < 1 ? 1 : g > (size_t)NPART ? (size_t)NPART : g);
+  };
+  const int ggrid = red(T.ngroups, VGATHER), ugrid = red(n1, VUPDATE);
+  int grid = nelmt > ggrid ? nelmt : ggrid;
+  if (grid < ugrid) grid = ugrid;
+  if (grid > p64::MAX_BLOCKS) grid = p64::MAX_BLOCKS;
+  unsigned* count = reinterpret_cast<unsigned*>(part + ggrid + 3 * ugrid);
+  static_assert(4 * NPART + 1 <= NPART * 16 * 4, "partials and the count fit the buffer");
+  cudaMemsetAsync(count, 0, sizeof(unsigned), s);
+  const p64::Args A{K, ge, pos, d_nbr, nelmt, T.d_ptr, T.d_dof, T.ngroups, n1, ggrid, ugrid,
+                    u, r, z, p, kp, Y, dp, cs, G, part, count, chunk};
+  return rows ? p64::launch<true>(A, grid, s) : p64::launch<false>(A, grid, s);
+}
+
+}  // namespace sg
