@@ -18,6 +18,11 @@
 //   * a block's matrices stay in shared memory for the whole launch while they
 //     fit, else they stream through two buffers filled by bulk copies, the
 //     next iteration's first group on its way during the vector phases;
+//   * the vector phases hand out warps, not blocks: the reference order of the
+//     dots groups 32 threads first, so each such warp may run on any SM, and
+//     a small mesh's few blocks of them do not queue on few FP64 units;
+//   * maxima are taken on the bits of the absolute values (integer unit), and
+//     the stop test divides only when the products do not decide it;
 //   * the phases of an iteration are separated by the counter barrier of
 //     sg_pcg_persist.cu.
 //
@@ -28,7 +33,10 @@
 // separate kernels.
 //
 // us per iteration, separate kernels (with short tails) -> this: 300 elements
-// dense 43 -> 22, sparse 37 -> 22; 12,000 elements sparse 256 -> 170.
+// dense 43 -> 16, sparse 37 -> 16; 12,000 elements sparse 256 -> 158, of which the
+// products take 119 (19 cycles for each FP64 warp instruction).  Code that one
+// warp runs once per iteration is kept short: unrolled twofold over nodes, the
+// gather took 10 us instead of 4.
 //
 // Every wait is bounded; a timeout sets the solve's error word, the block
 // waits (bounded) for its own copies and leaves, and the others follow.
@@ -69,7 +77,7 @@ struct Args {
   const double* dp;
   ColState* cs;
   PcgGlobal* G;
-  double* part;                          // p.kp [ggrid], r.z, max|p|, max|u| [ugrid] each
+  double* part;                          // warp partials: p.kp [8 ggrid], r.z, max|p|, max|u| [8 ugrid] each
   unsigned* count;
   int chunk;
 };
@@ -87,16 +95,54 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
   }
   return false;
 }
-__device__ __forceinline__ void half_sync(int h) { asm volatile("bar.sync %0, 256;" ::"r"(1 + h) : "memory"); }
+// |x| as an integer that orders like it; a NaN counts as 0, as fmax has it
+__device__ __forceinline__ unsigned long long mag(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+  return b > 0x7ff0000000000000ull ? 0ull : b;
+}
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long x) {
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    const unsigned long long y = __shfl_xor_sync(FULL, x, o);
+    x = x > y ? x : y;
+  }
+  return x;
+}
+// 0 + x[0] + x[1] + ... + x[n - 1], one add after the other, loads ahead of them
+__device__ __forceinline__ double chain(const double* x, int n) {
+  double s = 0.0;
+  int i = 0;
+#pragma unroll 1
+  for (; i + 8 <= n; i += 8) {
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = x[i + k];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += v[k];
+  }
+#pragma unroll 1
+  for (; i < n; ++i) s += x[i];
+  return s;
+}
+// a block's sum from its eight warps' partials
+__device__ __forceinline__ double block_partial(const double* part, int vb) {
+  const double2* w = reinterpret_cast<const double2*>(part + (size_t)vb * (VT / 32));
+  double2 x[VT / 64];
+#pragma unroll
+  for (int i = 0; i < VT / 64; ++i) x[i] = __ldcg(w + i);
+  double v = 0.0;
+#pragma unroll
+  for (int i = 0; i < VT / 64; ++i) { v += x[i].x; v += x[i].y; }
+  return v;
+}
 
-// Rows of `nel` elements whose matrices start at kb and directions at ps.
+// Rows [r0, r1) of the elements from efirst on, whose matrices start at kb and
+// directions at ps.
 template <bool ROWS>
-__device__ __forceinline__ void row_products(const Args& A, const double* kb, const double* ps, int efirst, int nel,
-                                             const int* nbr, int warp, int lane) {
+__device__ __forceinline__ void row_products(const Args& A, const double* kb, const double* ps, int efirst, int r0,
+                                             int r1, const int* nbr, int warp, int lane) {
   using L = Lay<ROWS>;
-  for (int c = warp; c * 32 < nel * NEDOF; c += NWARP) {
-    const int row = c * 32 + lane;
-    if (row >= nel * NEDOF) continue;
+  for (int row = r0 + warp * 32 + lane; row < r1; row += NT) {
     const int el = row / NEDOF, rr = row - el * NEDOF, n = rr / 3, cc = rr - 3 * n;
     const double* k = kb + (size_t)el * L::STRIDE;
     const double* pe = ps + el * NEDOF;
@@ -130,13 +176,15 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
   double* ps = dsm + (size_t)L::NP * L::STRIDE;       // directions of the same elements
   __shared__ int nbr[NGLL * KS_NBR];
   __shared__ __align__(8) uint64_t bar[2];
-  __shared__ double sred[NWARP][3];
-  __shared__ double sfin[VT], sm1[NWARP], sm2[NWARP];
+  __shared__ double spart[NPART], sfin[VT];
+  __shared__ int4 smap[NWARP][2][32];
+  __shared__ int smap2[NWARP][2][32];
+  __shared__ unsigned long long smax[NWARP][2];
   __shared__ double s_alpha, s_beta, s_rz, s_maxp, s_maxu;
   __shared__ int s_done, s_failed;
   PcgGlobal* G = A.G;
   if (G->all_done) return;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, h = t / VT, tl = t % VT, vw = tl >> 5;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int grid = gridDim.x, bid = blockIdx.x;
   const double tol = A.cs[0].tol;
   if (t == 0) {
@@ -150,9 +198,14 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
   int it = G->it;
   const int maxiter = G->maxiter;
   unsigned arrivals = 0;
-  // the block's elements
-  const int per = (A.nelmt + grid - 1) / grid, e0 = min(A.nelmt, bid * per), nel = min(A.nelmt, e0 + per) - e0;
-  const bool resident = nel <= L::RES;
+  // the block's rows: whole warps of 32 while the matrices they touch stay in
+  // shared memory, else whole elements
+  const int rows = A.nelmt * NEDOF, nchunk = (rows + 31) / 32, rper = (nchunk + grid - 1) / grid * 32;
+  const bool resident = (rper + NEDOF - 2) / NEDOF + 1 <= L::RES;   // a run of rper rows meets no more elements
+  const int per = (A.nelmt + grid - 1) / grid;
+  const int r0 = resident ? min(rows, bid * rper) : min(A.nelmt, bid * per) * NEDOF;
+  const int r1 = resident ? min(rows, r0 + rper) : min(A.nelmt, bid * per + per) * NEDOF;
+  const int e0 = min(r0 / NEDOF, A.nelmt), nel = r1 > r0 ? (r1 - 1) / NEDOF + 1 - e0 : 0;
   const int ngrp = (nel + L::GE - 1) / L::GE;
   unsigned uses = 0;        // groups copied so far (buffer uses % 2), the same in all threads
   unsigned waited = 0;
@@ -175,7 +228,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
   if (resident) {
     const double2* src = reinterpret_cast<const double2*>(A.K + (size_t)e0 * L::STRIDE);
     for (int i = t; i < nel * (L::STRIDE / 2); i += NT) reinterpret_cast<double2*>(kb)[i] = __ldcs(src + i);
-  } else {
+  } else if (nel > 0) {
     copy_group(0);
   }
   auto barrier = [&]() -> bool {
@@ -199,15 +252,34 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
     const int gd = __ldg(A.ge + (size_t)(e0 + first) * NEDOF + i);
     return fma(s_beta, __ldcg(A.p + gd), __ldcg(A.z + gd));
   };
+  // slot range and dof numbers of node g, {a, b, dof 0, dof 1} and dof 2
+  auto load_map = [&](int g, int4& m, int& gd2) {
+    m = make_int4(0, 0, 0, 0);
+    gd2 = 0;
+    if (g < A.ngroups) {
+      m = make_int4(__ldg(A.gptr + g), __ldg(A.gptr + g + 1), __ldg(A.gdof + 3 * g), __ldg(A.gdof + 3 * g + 1));
+      gd2 = __ldg(A.gdof + 3 * g + 2);
+    }
+  };
+  for (int j = 0; j < 2; ++j) {
+    int4 m;
+    int gd2;
+    load_map((bid + warp * grid) * 32 + lane + j * A.ggrid * VT, m, gd2);
+    smap[warp][j][lane] = m;
+    smap2[warp][j][lane] = gd2;
+  }
   double* partB = A.part;
-  double *partZ = A.part + A.ggrid, *partP = partZ + A.ugrid, *partU = partP + A.ugrid;
+  constexpr int VW = VT / 32;
+  double* partZ = A.part + VW * A.ggrid;
+  unsigned long long* partP = reinterpret_cast<unsigned long long*>(partZ + VW * A.ugrid);
+  unsigned long long* partU = partP + VW * A.ugrid;
   bool ok = true;
   for (int k = 0; k < A.chunk && ok; ++k) {
     // ---- element products of p = z + beta p_old ----
     if (resident) {
       for (int i = t; i < nel * NEDOF; i += NT) ps[i] = direction(0, i);
       __syncthreads();
-      row_products<ROWS>(A, kb, ps, e0, nel, nbr, warp, lane);
+      row_products<ROWS>(A, kb, ps, e0, r0 - e0 * NEDOF, r1 - e0 * NEDOF, nbr, warp, lane);
     } else {
       if (t < min(L::GE, nel) * NEDOF) ps[t] = direction(0, t);
       for (int g = 0; g < ngrp; ++g) {
@@ -219,8 +291,8 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
         ok = mbar_wait(bar + b, (waited >> 1) & 1);
         if (__syncthreads_or(!ok)) { ok = false; break; }
         ++waited;
-        row_products<ROWS>(A, kb + (size_t)b * L::GE * L::STRIDE, ps + (g & 1) * L::GE * NEDOF, e0 + g * L::GE, n, nbr,
-                           warp, lane);
+        row_products<ROWS>(A, kb + (size_t)b * L::GE * L::STRIDE, ps + (g & 1) * L::GE * NEDOF, e0 + g * L::GE, 0,
+                           n * NEDOF, nbr, warp, lane);
         if (t < nn * NEDOF) ps[((g + 1) & 1) * L::GE * NEDOF + t] = nd;
         __syncthreads();
       }
@@ -230,32 +302,45 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
       }
     }
     if (!barrier()) { ok = false; break; }
-    // ---- kp, p and p.kp, a half block per virtual block ----
+    // ---- kp, p and p.kp: warp w of the gather's grid takes 32 nodes, then the
+    // 32 a grid further on, ... ----
     const double beta = s_beta;
-    for (int vb = bid + h * grid; vb < A.ggrid; vb += 2 * grid) {
+    for (int w = bid + warp * grid; w < VW * A.ggrid; w += NWARP * grid) {
       double dot = 0.0;
-      for (int g = (vb * (VT / 32) + vw) * 32 + lane; g < A.ngroups; g += A.ggrid * VT) {
-        const int a = __ldg(A.gptr + g), b = __ldg(A.gptr + g + 1);
-        int gd[3];
-        double pv[3], zv[3], acc[3] = {0.0, 0.0, 0.0};
+      const int gs = A.ggrid * VT;
+      const bool mapped = w == bid + warp * grid;   // the first such warp keeps two nodes' maps in shared memory
+#pragma unroll 1
+      for (int j = 0; w * 32 + j * gs < A.ngroups; ++j) {
+        int4 m;
+        int gd2;
+        if (mapped && j < 2) {
+          m = smap[warp][j][lane];
+          gd2 = smap2[warp][j][lane];
+        } else {
+          load_map(w * 32 + lane + j * gs, m, gd2);
+        }
+        const int gd[3] = {m.z, m.w, gd2};
+        double pv[3], zv[3], y[4][3], acc[3] = {0.0, 0.0, 0.0};
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-          gd[d] = __ldg(A.gdof + 3 * g + d);
           pv[d] = __ldcg(A.p + gd[d]);
           zv[d] = __ldcg(A.z + gd[d]);
         }
-        for (int s0 = a; s0 < b; s0 += 4) {
-          double y[4][3];
+        // absent slots add +0, which changes no sum that began at +0
+        int s0 = m.x;
+#pragma unroll 1
+        do {
+          const double* yp = A.Y + (size_t)s0 * 3;
 #pragma unroll
           for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int d = 0; d < 3; ++d) y[i][d] = s0 + i < b ? __ldcg(A.Y + (size_t)(s0 + i) * 3 + d) : 0.0;
+            for (int d = 0; d < 3; ++d) y[i][d] = s0 + i < m.y ? __ldcg(yp + 3 * i + d) : 0.0;
 #pragma unroll
           for (int i = 0; i < 4; ++i)
-            if (s0 + i < b)
 #pragma unroll
-              for (int d = 0; d < 3; ++d) acc[d] = acc[d] + y[i][d];
-        }
+            for (int d = 0; d < 3; ++d) acc[d] = acc[d] + y[i][d];
+          s0 += 4;
+        } while (s0 < m.y);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           if (!gd[d]) continue;
@@ -267,36 +352,27 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
       }
 #pragma unroll
       for (int o = 16; o >= 1; o >>= 1) dot += __shfl_xor_sync(FULL, dot, o);
-      if (lane == 0) sred[warp][0] = dot;
-      half_sync(h);
-      if (tl == 0) {
-        double v = 0.0;
-        for (int w = 0; w < VT / 32; ++w) v += sred[h * (VT / 32) + w][0];
-        __stcg(partB + vb, v);
-      }
-      half_sync(h);
+      if (lane == 0) __stcg(partB + w, dot);
     }
     if (!barrier()) { ok = false; break; }
-    // alpha: the block partials in the order of the last block's sum
+    // alpha: the partials in the order of the last block's sum
+    for (int b = t; b < A.ggrid; b += NT) spart[b] = block_partial(partB, b);
+    __syncthreads();
     if (t < VT) {
       double v = 0.0;
-      for (int i = t; i < A.ggrid; i += VT) v += __ldcg(partB + i);
+      for (int b = t; b < A.ggrid; b += VT) v += spart[b];
       sfin[t] = v;
     }
     __syncthreads();
-    if (t == 0) {
-      double s = 0.0;
-      const int n = min(VT, A.ggrid);
-      for (int i = 0; i < n; ++i) s += sfin[i];
-      s_alpha = s_rz / s;
-    }
+    if (t == 0) s_alpha = s_rz / chain(sfin, min(VT, A.ggrid));
     __syncthreads();
-    // ---- u, r, z, max-norms and r.z ----
+    // ---- u, r, z, max-norms and r.z, by warps of the update's grid ----
     const double alpha = s_alpha;
-    for (int vb = bid + h * grid; vb < A.ugrid; vb += 2 * grid) {
-      double mp = 0.0, mu = 0.0, rz = 0.0;
+    for (int w = bid + warp * grid; w < VW * A.ugrid; w += NWARP * grid) {
+      unsigned long long mp = 0, mu = 0;
+      double rz = 0.0;
       const size_t stride = (size_t)A.ugrid * VT;
-      for (size_t i0 = (size_t)vb * VT + tl; i0 < (size_t)A.n1; i0 += 4 * stride) {
+      for (size_t i0 = (size_t)w * 32 + lane; i0 < (size_t)A.n1; i0 += 4 * stride) {
         double pv[4], uv[4], rv[4], kv[4], dv[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -312,28 +388,16 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
           if (i >= (size_t)A.n1) continue;
           const double un = fma(alpha, pv[q], uv[q]), rn = fma(-alpha, kv[q], rv[q]), zn = dv[q] * rn;
           A.u[i] = un; A.r[i] = rn; A.z[i] = zn;
-          mp = fmax(mp, fabs(pv[q]));
-          mu = fmax(mu, fabs(un));
+          mp = max(mp, mag(pv[q]));
+          mu = max(mu, mag(un));
           rz = fma(rn, zn, rz);
         }
       }
+      mp = warp_max(mp);
+      mu = warp_max(mu);
 #pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) {
-        mp = fmax(mp, __shfl_xor_sync(FULL, mp, o));
-        mu = fmax(mu, __shfl_xor_sync(FULL, mu, o));
-        rz = rz + __shfl_xor_sync(FULL, rz, o);
-      }
-      if (lane == 0) { sred[warp][0] = mp; sred[warp][1] = mu; sred[warp][2] = rz; }
-      half_sync(h);
-      if (tl < 3) {
-        double v = 0.0;
-        for (int w = 0; w < VT / 32; ++w) {
-          const double x = sred[h * (VT / 32) + w][tl];
-          v = tl < 2 ? fmax(v, x) : v + x;
-        }
-        __stcg((tl == 0 ? partP : tl == 1 ? partU : partZ) + vb, v);
-      }
-      half_sync(h);
+      for (int o = 16; o >= 1; o >>= 1) rz = rz + __shfl_xor_sync(FULL, rz, o);
+      if (lane == 0) { __stcg(partZ + w, rz); __stcg(partP + w, mp); __stcg(partU + w, mu); }
     }
     if (!barrier()) { ok = false; break; }
     // stop test and beta, identical in every block: r.z over interleaved
@@ -341,37 +405,43 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
     ++it;
     {
       constexpr int NJ = VT / 4;
-      double mp = 0.0, mu = 0.0;
+      for (int b = t; b < A.ugrid; b += NT) spart[b] = block_partial(partZ, b);
+      unsigned long long mp = 0, mu = 0;
+      for (int w = t; w < VW * A.ugrid; w += NT) {
+        mp = max(mp, __ldcg(partP + w));
+        mu = max(mu, __ldcg(partU + w));
+      }
+      mp = warp_max(mp);
+      mu = warp_max(mu);
+      if (lane == 0) { smax[warp][0] = mp; smax[warp][1] = mu; }
+      __syncthreads();
       if (t < NJ) {
         double v = 0.0;
-        for (int b = t; b < A.ugrid; b += NJ) v += __ldcg(partZ + b);
+        for (int b = t; b < A.ugrid; b += NJ) v += spart[b];
         sfin[t] = v;
-      } else {
-        for (int b = t - NJ; b < A.ugrid; b += NT - NJ) {
-          mp = fmax(mp, __ldcg(partP + b));
-          mu = fmax(mu, __ldcg(partU + b));
+      } else if (warp == NWARP - 1) {
+        // |alpha| max|p| / max|u| <= tol, divided only where the products are close
+        mp = lane < NWARP ? smax[lane][0] : 0;
+        mu = lane < NWARP ? smax[lane][1] : 0;
+        mp = warp_max(mp);
+        mu = warp_max(mu);
+        if (lane == 0) {
+          const double dp = __longlong_as_double((long long)mp), du = __longlong_as_double((long long)mu);
+          const double a = fabs(s_alpha) * dp, b = tol * du, eps = 1e-14 * b;
+          s_maxp = dp; s_maxu = du;
+          s_done = a < b - eps ? 1 : a > b + eps ? 0 : a / du <= tol;
         }
       }
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) {
-        mp = fmax(mp, __shfl_xor_sync(FULL, mp, o));
-        mu = fmax(mu, __shfl_xor_sync(FULL, mu, o));
-      }
-      if (lane == 0) { sm1[warp] = mp; sm2[warp] = mu; }
       __syncthreads();
       if (t == 0) {
-        double s = 0.0;
-        const int n = min(NJ, A.ugrid);
-        for (int i = 0; i < n; ++i) s += sfin[i];
-        for (int w = 0; w < NWARP; ++w) { mp = fmax(mp, sm1[w]); mu = fmax(mu, sm2[w]); }
-        s_maxp = mp; s_maxu = mu;
-        if (fabs(s_alpha) * mp / mu <= tol) {
-          s_done = 1;
-        } else if (it >= maxiter) {
-          s_done = 1; s_failed = 1;
-        } else {
-          s_beta = s / s_rz;
-          s_rz = s;
+        if (!s_done) {
+          if (it >= maxiter) {
+            s_done = 1; s_failed = 1;
+          } else {
+            const double s = chain(sfin, min(NJ, A.ugrid));
+            s_beta = s / s_rz;
+            s_rz = s;
+          }
         }
       }
       __syncthreads();
@@ -455,15 +525,15 @@ bool launch_pcg_persistent64(bool rows, const double* K, const int* ge, int nelm
     return (int)(g < 1 ? 1 : g > (size_t)NPART ? (size_t)NPART : g);
   };
   const int ggrid = red(T.ngroups, VGATHER), ugrid = red(n1, VUPDATE);
-  int grid = nelmt > ggrid ? nelmt : ggrid;
-  if (grid < ugrid) grid = ugrid;
+  long grid = ((long)nelmt * NEDOF + 31) / 32;   // a warp of rows per block, at least
+  if (grid < 8L * ugrid) grid = 8L * ugrid;
   if (grid > p64::MAX_BLOCKS) grid = p64::MAX_BLOCKS;
-  unsigned* count = reinterpret_cast<unsigned*>(part + ggrid + 3 * ugrid);
-  static_assert(4 * NPART + 1 <= NPART * 16 * 4, "partials and the count fit the buffer");
+  unsigned* count = reinterpret_cast<unsigned*>(part + RED_THREADS / 32 * (ggrid + 3 * ugrid));
+  static_assert(RED_THREADS / 32 * 4 * NPART + 1 <= NPART * 16 * 4, "partials and the count fit the buffer");
   cudaMemsetAsync(count, 0, sizeof(unsigned), s);
   const p64::Args A{K, ge, pos, d_nbr, nelmt, T.d_ptr, T.d_dof, T.ngroups, n1, ggrid, ugrid,
                     u, r, z, p, kp, Y, dp, cs, G, part, count, chunk};
-  return rows ? p64::launch<true>(A, grid, s) : p64::launch<false>(A, grid, s);
+  return rows ? p64::launch<true>(A, (int)grid, s) : p64::launch<false>(A, (int)grid, s);
 }
 
 }  // namespace sg
