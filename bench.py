@@ -278,9 +278,9 @@ def apply_kernel_name(kr: int, nelmt: int) -> str:
     v = os.environ.get("SG_APPLY_VARIANT", "5")
     if v == "2" and kr in (8, 16):
         return f"k_apply_tc<{kr}>"
-    if v == "4" or (v == "5" and nelmt < 100000):
-        return f"k_apply_mf<{kr}>"
-    if v in ("3", "5") and kr in (8, 16):
+    if v in ("4", "5"):
+        return f"k_apply_mf_planes<{kr}>" if kr >= 4 else f"k_apply_mf_lines<{kr}>"
+    if v == "3" and kr in (8, 16):
         return f"k_apply_lanes<{kr}>"
     return f"k_apply_sparse_tma<float,{kr}>"
 
@@ -675,6 +675,8 @@ def run_ours(args, rank, world, local):
     ks_nnz_unique = 2349                      # structurally non-zero unique entries of a symmetric GLL K_e
     bytes_elem = ks_nnz_unique * 4 + 27 * 4   # matrix + connectivity
     kr = 1 << (k - 1).bit_length()
+    if apply_kernel_name(kr, ne).startswith("k_apply_mf"):
+        bytes_elem = 27 * 48 + 27 * 4         # matrix-free: point records + connectivity
     bytes_apply = ne * bytes_elem + 2 * (neq + 1) * kr * 4
     apply_ms = prof["apply_ms"] / max(1, prof["apply_launches"])
     achieved = bytes_apply / (apply_ms / 1000.0) / 1e9
@@ -682,7 +684,9 @@ def run_ours(args, rank, world, local):
     tpath = os.path.join(ROOT, "profiles", "apply_traffic.json")
     if os.path.exists(tpath):
         with open(tpath) as f:
-            traffic = json.load(f).get("bytes_per_launch")
+            measured = json.load(f)
+        if measured.get("kernel") == apply_kernel_name(kr, ne):
+            traffic = measured.get("bytes_per_launch")
 
     precision = None
     if args.no_fp64:

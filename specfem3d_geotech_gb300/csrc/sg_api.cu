@@ -432,7 +432,7 @@ sg_ctx* sg_create(int device, size_t hbm_budget) {
   upload_constants();
   // SG_APPLY_VARIANT selects another element apply for cross-checking:
   // 0 register-staged, 1 TMA node lanes, 2 tensor cores, 3 lane apply,
-  // 4 matrix-free FP32 (default 5: lane apply, matrix-free FP32 on small meshes).
+  // 4 and 5 (default) matrix-free FP32.
   if (const char* v = std::getenv("SG_APPLY_VARIANT")) set_apply_variant(std::atoi(v));
   // SG_GATHER_VARIANT=0 selects the shared-memory-staged gather everywhere.
   if (const char* v = std::getenv("SG_GATHER_VARIANT")) set_gather_variant(std::atoi(v));
@@ -802,7 +802,7 @@ static sg_model* model_build(sg_ctx* c, HostMesh&& H, int nnode8, const double* 
   M->d_geo = c->alloc<double>((size_t)ne * NGLL * GEO_STRIDE);
   M->d_K64 = c->alloc<double>((size_t)ne * KS_STRIDE);
   if (precision == SG_PREC_MIXED) {
-    M->d_K32 = c->alloc<float>((size_t)ne * KS_STRIDE);
+    if (!fp32_matrix_free()) M->d_K32 = c->alloc<float>((size_t)ne * KS_STRIDE);
     M->d_rec32 = c->alloc<float>((size_t)ne * NGLL * MF_REC);
     M->d_dprecon32 = c->alloc<float>(n1);
   }
@@ -813,7 +813,7 @@ static sg_model* model_build(sg_ctx* c, HostMesh&& H, int nnode8, const double* 
   M->d_fpart = c->alloc<double>(NPART * 2);
   bool ok = M->d_coord && M->d_gnum && M->d_matid && M->d_ge && M->d_gdof && M->d_ym && M->d_nu && M->d_gam &&
             M->d_geo && M->d_K64 && M->d_diag && M->d_dprecon && M->d_extload && M->d_Yscratch && M->d_fpart &&
-            (precision == SG_PREC_FP64 || (M->d_K32 && M->d_rec32 && M->d_dprecon32)) && upload_topo(c, M->T);
+            (precision == SG_PREC_FP64 || ((M->d_K32 || fp32_matrix_free()) && M->d_rec32 && M->d_dprecon32)) && upload_topo(c, M->T);
   if (!ok) {
     set_tag(errtag, "ERROR: the model does not fit the device memory budget!");
     sg_model_free(M);
@@ -1139,7 +1139,7 @@ struct SolveStats {
 static Op fp32_op(const sg_model* M, const Op& op64) {
   Op o = op64;
   o.K = M->d_K32;
-  if (fp32_matrix_free(op64.nelmt)) {
+  if (fp32_matrix_free()) {
     o.dense = 2;
     o.K = M->d_rec32;
   }

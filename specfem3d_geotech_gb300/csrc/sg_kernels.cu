@@ -419,16 +419,13 @@ constexpr int APPLY_WARPS = 4;
 // 0 = register-staged loads, 1 = TMA bulk-copy pipeline (node lanes),
 // 2 = tensor cores (FP32, 8/16 RHS), 3 = lane per (element, RHS) for FP32
 // with 8/16 RHS and the TMA node-lane pipeline otherwise (default),
-// 4 = as 3 for FP64, matrix-free for the FP32 operator of the mixed solve,
-// 5 = as 3, except that the FP32 operator of meshes below MF_AUTO_MAX elements
-// is matrix-free (default): on small meshes the PCG iteration is latency-
-// bound and the matrix-free apply has the shorter dependency chain (33.6
-// against 50.2 us per iteration at 270 elements, 125 against 162 us at 10k);
-// at 192k elements the two applies take the same time.
-constexpr int MF_AUTO_MAX = 100000;
+// 4, 5 = as 3 for FP64, matrix-free for the FP32 operator of the mixed solve
+// (default): 1.3 KB of point records an element instead of 9.7 KB of matrix.
+// us per apply at 120k elements, stored against matrix-free: 328, 103 with one
+// trial, 439, 133 with four, 434, 243 with eight, 722, 413 with sixteen.
 int g_apply_variant = 5;
 void set_apply_variant(int v) { g_apply_variant = v; }
-bool fp32_matrix_free(int nelmt) { return g_apply_variant == 4 || (g_apply_variant == 5 && nelmt < MF_AUTO_MAX); }
+bool fp32_matrix_free() { return g_apply_variant >= 4; }
 bool persist_default_apply() { return g_apply_variant >= 2; }
 // device copy of the stored-entry table, needed by the tensor-core apply
 const int* g_entry_dev = nullptr;

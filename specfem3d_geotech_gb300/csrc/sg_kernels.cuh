@@ -44,8 +44,8 @@ struct MatF {
 long long launch_count();        // kernel launches issued so far (host counter)
 void add_launches(long long n);  // kernels launched through a replayed CUDA graph
 void set_apply_variant(int v);   // 0 register-staged, 1 TMA pipeline, 2 tensor cores for 8/16 FP32 RHS,
-                                 // 3 lane per (element, RHS) for 8/16 FP32 RHS, 4 matrix-free FP32,
-                                 // 5 (default) 3 with matrix-free FP32 on small meshes
+                                 // 3 lane per (element, RHS) for 8/16 FP32 RHS, 4 and 5 (default)
+                                 // matrix-free FP32
 bool persist_default_apply();    // the chosen variant leaves the FP64 apply at its default
 void set_entry_table(const int* d_entry);
 // The element applies that wait on mbarriers set *err to 1 when a bounded
@@ -89,7 +89,7 @@ void launch_mf_record(const double* geo, const int* mat_id, const int* elist, in
 constexpr int MF_REC = 12;        // floats per GLL point of the matrix-free record
 void launch_nodal_average(const int* ptr, const int* slot, int nnode, const double* stress, double* out,
                           cudaStream_t s);  // sg_output.cu
-bool fp32_matrix_free(int nelmt);
+bool fp32_matrix_free();
 // Persistent cooperative FP32 PCG chunk for small and medium meshes
 // (sg_pcg_persist.cu); false when it cannot run (the caller launches the
 // separate kernels).  A chunk whose bounded wait ran out sets G->err.

@@ -79,3 +79,12 @@ def test_fp64_persistent_is_bitwise_the_separate_kernels(tmp_path, dims):
     for key in ("x", "u", "v", "w", "it", "e"):
         assert np.array_equal(a[key], b[key]), key
     assert a["e"].tolist() == [0, 0, -1] and np.array_equal(a["u"], a["v"])
+
+
+@pytest.mark.parametrize("k", [3, 8, 16])
+@pytest.mark.parametrize("dims", [(2, 2, 2), (3, 1, 11), (13, 7, 9)])
+def test_plane_apply_matches_stored_matrices(tmp_path, dims, k):
+    """One element group, a ragged last group, and more groups than one pass."""
+    a = trials(dims, k, tmp_path, SG_PERSIST="0", SG_APPLY_VARIANT="5")
+    b = trials(dims, k, tmp_path, SG_PERSIST="0", SG_APPLY_VARIANT="1")
+    same(a, b)
