@@ -63,6 +63,7 @@ struct sg_ctx {
   long long launch0 = 0;
   int* d_nbr = nullptr;
   int* d_entry = nullptr;
+  int* d_border = nullptr;
   // drop-in cache: the reference calls pcg_solver with the same dof map every
   // plastic iteration, so the gather topology is rebuilt only when it changes.
   struct DropIn {
@@ -88,7 +89,7 @@ struct sg_ctx {
     int nnode = -1, nelmt = -1, neq = -1, nel = -1;
     GatherTopo T;  // groups of the listed elements' dof map
     double *d_coord = nullptr, *d_geo = nullptr, *x = nullptr, *evpt = nullptr, *stress = nullptr, *bl = nullptr,
-           *Yb = nullptr, *wp = nullptr, *vm = nullptr, *sf = nullptr, *part = nullptr, *red = nullptr;
+           *Yb = nullptr, *wp = nullptr, *vm = nullptr, *sf = nullptr, *part = nullptr;
     int *d_gnum = nullptr, *d_ge = nullptr, *d_mat = nullptr, *d_elist = nullptr;
     MatF* mf = nullptr;
     int mfcap = 0;
@@ -439,10 +440,12 @@ sg_ctx* sg_create(int device, size_t hbm_budget) {
   const KsTables& T = ks_tables();
   c->d_nbr = c->alloc<int>(NGLL * KS_NBR);
   c->d_entry = c->alloc<int>(KS_NNZ);
+  c->d_border = c->alloc<int>(KS_NNZ / 9);
   c->d_err = c->alloc<int>(1);
   cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
   cudaMemcpy(c->d_nbr, T.nbr, sizeof(T.nbr), cudaMemcpyHostToDevice);
   cudaMemcpy(c->d_entry, T.entry, sizeof(T.entry), cudaMemcpyHostToDevice);
+  cudaMemcpy(c->d_border, T.border, sizeof(T.border), cudaMemcpyHostToDevice);
   set_entry_table(c->d_entry);
   if (cudaGetLastError() != cudaSuccess) {
     g_create_status = SG_ERR_NODEVICE;
@@ -650,7 +653,6 @@ struct TrialWork {
   double *kp64 = nullptr, *r64 = nullptr;
   float *r32 = nullptr, *d32 = nullptr;
   int* colmask = nullptr;
-  double* red = nullptr;
 };
 
 struct Slot {
@@ -703,7 +705,7 @@ static void model_release_work(sg_model* M) {
                   (void*)W.stress, (void*)W.mf, (void*)W.b64.r, (void*)W.b64.z, (void*)W.b64.p, (void*)W.b64.kp,
                   (void*)W.b64.part, (void*)W.b64.cs, (void*)W.b64.G, (void*)W.b32.r, (void*)W.b32.z,
                   (void*)W.b32.p, (void*)W.b32.kp, (void*)W.b32.Y, (void*)W.kp64, (void*)W.r64, (void*)W.r32,
-                  (void*)W.d32, (void*)W.colmask, (void*)W.red})
+                  (void*)W.d32, (void*)W.colmask})
     c->release(p);
   W = TrialWork();
 }
@@ -724,10 +726,9 @@ static bool model_work(sg_model* M, int KR, int n1, int nel) {
   W.b64.part = c->alloc<double>((size_t)NPART * 16 * 4);
   W.b64.cs = c->alloc<ColState>(16);
   W.b64.G = c->alloc<PcgGlobal>(1);
-  W.red = c->alloc<double>(64);
   W.colmask = c->alloc<int>(16);
   bool ok = W.x && W.oldx && W.load && W.bodyload && W.Yb && W.evpt && W.stress && W.mf && W.b64.part && W.b64.cs &&
-            W.b64.G && W.red && W.colmask;
+            W.b64.G && W.colmask;
   if (M->precision == SG_PREC_FP64) {
     W.b64.r = c->alloc<double>(nv); W.b64.z = c->alloc<double>(nv); W.b64.p = c->alloc<double>(nv);
     W.b64.kp = c->alloc<double>(nv); W.b64.Y = W.Yb;  // the apply and body-load gathers share Y
@@ -754,7 +755,7 @@ static bool model_stiffness(sg_model* M, const int* d_elist, int nel, const doub
   double* Ygrav = M->d_Yscratch + (size_t)M->H.nelmt * NEDOF;
   int ev = c->prof_begin();
   launch_stiffness(M->d_geo, M->d_matid, d_elist, nel, M->d_ym, d_nuv, M->d_gam, M->d_K64, M->d_K32, Ydiag,
-                   gravity ? Ygrav : nullptr, c->d_entry, T.d_pos, s, pseudoeq ? M->H.iseqload : 0, M->H.eqkx,
+                   gravity ? Ygrav : nullptr, c->d_border, T.d_pos, s, pseudoeq ? M->H.iseqload : 0, M->H.eqkx,
                    M->H.eqky, M->H.eqkz);
   launch_mf_record(M->d_geo, M->d_matid, d_elist, nel, M->d_ym, d_nuv, M->d_rec32, s);
   c->prof_end(ev, 5);
@@ -810,7 +811,7 @@ static sg_model* model_build(sg_ctx* c, HostMesh&& H, int nnode8, const double* 
   M->d_dprecon = c->alloc<double>(n1);
   M->d_extload = c->alloc<double>(n1);
   M->d_Yscratch = c->alloc<double>((size_t)2 * ne * NEDOF);
-  M->d_fpart = c->alloc<double>(NPART * 2);
+  M->d_fpart = c->alloc<double>(NPART * 16);
   bool ok = M->d_coord && M->d_gnum && M->d_matid && M->d_ge && M->d_gdof && M->d_ym && M->d_nu && M->d_gam &&
             M->d_geo && M->d_K64 && M->d_diag && M->d_dprecon && M->d_extload && M->d_Yscratch && M->d_fpart &&
             (precision == SG_PREC_FP64 || ((M->d_K32 || fp32_matrix_free()) && M->d_rec32 && M->d_dprecon32)) && upload_topo(c, M->T);
@@ -1112,11 +1113,10 @@ static void make_matf(int nmat, const double* ymv, const double* nuf, const doub
   }
 }
 
-// Reads KR*nq reduced values (fixed-order device reduction) to the host.
-static void reduce_read(sg_ctx* c, const double* part, int nblk, int KR, int nq, int maxmask, double* d_out,
-                        double* h_out) {
-  launch_final_reduce(part, nblk, KR, nq, maxmask, d_out, c->stream);
-  cudaMemcpyAsync(c->pin + 256, d_out, sizeof(double) * KR * nq, cudaMemcpyDeviceToHost, c->stream);
+// Reads KR*nq reduced values (fixed-order device reduction) to the host; the
+// reduction writes them to pinned host memory itself.
+static void reduce_read(sg_ctx* c, const double* part, int nblk, int KR, int nq, int maxmask, double* h_out) {
+  launch_final_reduce(part, nblk, KR, nq, maxmask, c->pin + 256, c->stream);
   cudaStreamSynchronize(c->stream);
   std::memcpy(h_out, c->pin + 256, sizeof(double) * KR * nq);
 }
@@ -1171,7 +1171,7 @@ static int linear_solve(sg_model* M, const sg_control* ctl, const Op& op64, cons
   for (int round = 0; round < 200; ++round) {
     apply_plain<double>(c, KR, op64, W.x, W.Yb, W.kp64);
     launch_residual_norms(n1, KR, W.load, W.kp64, W.r64, W.r32, W.b64.part, c->stream);
-    reduce_read(c, W.b64.part, NPART, KR, 2, 0, W.red, red);
+    reduce_read(c, W.b64.part, vec_blocks(n1, KR), KR, 2, 0, red);
     S.refine++;
     c->prof.counts[3]++;
     bool any = false;
@@ -1199,7 +1199,7 @@ static int linear_solve(sg_model* M, const sg_control* ctl, const Op& op64, cons
     }
     cudaMemcpyAsync(W.colmask, mask, sizeof(int) * 16, cudaMemcpyHostToDevice, c->stream);
     launch_axpy_correction(n1, KR, W.colmask, W.d32, W.x, W.b64.part, c->stream);
-    reduce_read(c, W.b64.part, NPART, KR, 2, 3, W.red, red);
+    reduce_read(c, W.b64.part, vec_blocks(n1, KR), KR, 2, 3, red);
     // the reference's step test on the last CG step: |alpha|*max|p| <= cg_tol*max|x|
     for (int j = 0; j < k; ++j)
       if (live[j]) step_ok[j] = (red[2 * j + 1] > 0) && (step[j] <= ctl->cg_tol * red[2 * j + 1]);
@@ -1300,7 +1300,7 @@ static void slot_finish(sg_model* M, int j) {
   Slot& S = M->B.slot[j];
   double red[64];
   launch_disp_max(M->H.nnode, M->d_gdof, M->W.x, M->B.KR, j, M->W.b64.part, c->stream);
-  reduce_read(c, M->W.b64.part, NPART, 1, 2, 3, M->W.red, red);
+  reduce_read(c, M->W.b64.part, vec_blocks(M->H.nnode, 1), 1, 2, 3, red);
   S.res.uxmax = red[0];
   S.res.umax = red[1];
   S.res.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - S.t0).count();
@@ -1356,10 +1356,11 @@ static int batch_iteration(sg_model* M) {
   // uerr = max|x-oldx| / max|x|; oldx = x (src/slope.F90:307-309)
   double red[64];
   launch_nl_check(n1, KR, k, W.x, W.oldx, W.b64.part, s);
-  reduce_read(c, W.b64.part, NPART, KR, 2, 3, W.red, red);
+  reduce_read(c, W.b64.part, vec_blocks(n1, KR), KR, 2, 3, red);
   std::vector<int> fin(k, 0), conv(k, 0);
   int gmask[16] = {0};
   bool anyg = false;
+  StressCols cols;
   for (int t = 0; t < k; ++t) {
     if (!live[t]) continue;
     Slot& S = B.slot[t];
@@ -1367,16 +1368,16 @@ static int batch_iteration(sg_model* M) {
     S.res.uerr = uerr;
     conv[t] = uerr <= ctl->nl_tol;
     fin[t] = conv[t] || S.res.nl_iter == ctl->nl_maxiter;
-    int ev = c->prof_begin();
-    launch_stress_update(M->d_geo, nullptr, ne, M->d_ge, M->d_matid, W.x, KR, t, W.mf + (size_t)t * h.nmatblk, S.dt,
-                         conv[t], fin[t], W.evpt + nst * t, W.stress + nst * t, W.Yb, KR, t, M->d_fpart, M->T.d_pos, s,
-                         nullptr, nullptr, M->d_wp, M->d_gnum, 0);
-    c->prof_end(ev, 4);
-    reduce_read(c, M->d_fpart, NPART, 1, 1, 1, W.red, red + 32);
-    S.res.fmax = red[32];
+    cols.add(t, S.dt, conv[t], fin[t]);
     gmask[t] = !fin[t];
     anyg = anyg || gmask[t];
   }
+  int ev = c->prof_begin();
+  launch_stress_update(M->d_geo, nullptr, ne, M->d_ge, M->d_matid, W.x, KR, W.mf, h.nmatblk, cols, nst, W.evpt, W.stress,
+                       W.Yb, KR, M->d_fpart, M->T.d_pos, s, nullptr, nullptr, M->d_wp, M->d_gnum, 0);
+  c->prof_end(ev, 4);
+  reduce_read(c, M->d_fpart, stress_blocks(ne), cols.stride(), 1, 1, red);
+  for (int q = 0; q < cols.n; ++q) B.slot[cols.col[q]].res.fmax = red[q];
   // bodyload(egdof) += bload for the slots that continue
   if (anyg) {
     cudaMemcpyAsync(W.colmask, gmask, sizeof(int) * 16, cudaMemcpyHostToDevice, s);
@@ -1918,12 +1919,14 @@ extern "C" int sg_excavation(sg_model* M, const sg_control* ctl, int s0_type, do
             if (st != SG_OK) { status = st; break; }
             cg_tot += S.iters[0];
             launch_nl_check(n1, 1, 1, W.x, W.oldx, W.b64.part, s);
-            reduce_read(c, W.b64.part, NPART, 1, 2, 3, W.red, red);
+            reduce_read(c, W.b64.part, vec_blocks(n1, 1), 1, 2, 3, red);
             double uerr = red[0] / red[1];
             int conv = uerr <= ctl->nl_tol, fin = conv || nl_iter == ctl->nl_maxiter;
-            launch_stress_update(M->d_geo, d_eint, nint, d_geall, M->d_matid, W.x, 1, 0, W.mf, dt, conv, fin, evpt,
-                                 stress, W.Yb, 1, 0, M->d_fpart, Ti.d_pos, s, d_vm, d_sf, M->d_wp, M->d_gnum, 1);
-            reduce_read(c, M->d_fpart, NPART, 1, 1, 1, W.red, red);
+            StressCols one;
+            one.add(0, dt, conv, fin);
+            launch_stress_update(M->d_geo, d_eint, nint, d_geall, M->d_matid, W.x, 1, W.mf, nm, one, nst, evpt, stress,
+                                 W.Yb, 1, M->d_fpart, Ti.d_pos, s, d_vm, d_sf, M->d_wp, M->d_gnum, 1);
+            reduce_read(c, M->d_fpart, stress_blocks(nint), 1, 1, 1, red);
             fmax = red[0];
             if (!fin) launch_gather_plain<double>(Ti, 1, W.Yb, W.bodyload, 1, nullptr, s);
             if (fin) {
@@ -2004,7 +2007,7 @@ static void release_sdrop(sg_ctx* c) {
   auto& D = c->sdrop;
   free_topo(c, D.T);
   for (void* p : {(void*)D.d_coord, (void*)D.d_geo, (void*)D.x, (void*)D.evpt, (void*)D.stress, (void*)D.bl,
-                  (void*)D.Yb, (void*)D.wp, (void*)D.vm, (void*)D.sf, (void*)D.part, (void*)D.red, (void*)D.d_gnum,
+                  (void*)D.Yb, (void*)D.wp, (void*)D.vm, (void*)D.sf, (void*)D.part, (void*)D.d_gnum,
                   (void*)D.d_ge, (void*)D.d_mat, (void*)D.d_elist, (void*)D.mf})
     c->release(p);
   D = sg_ctx::StressDropIn();
@@ -2064,7 +2067,7 @@ extern "C" int sg_stress_bodyload(sg_ctx* c, int neq, int nelmt, int nnode, cons
     D.Yb = c->alloc<double>((size_t)nel * NEDOF);
     D.wp = c->alloc<double>(nnode);
     D.vm = c->alloc<double>((size_t)nel * NGLL); D.sf = c->alloc<double>((size_t)nel * NGLL);
-    D.part = c->alloc<double>(NPART); D.red = c->alloc<double>(64);
+    D.part = c->alloc<double>(NPART);
     D.d_gnum = c->alloc<int>((size_t)NGLL * nelmt); D.d_ge = c->alloc<int>((size_t)NEDOF * nelmt);
     D.d_mat = c->alloc<int>(nelmt); D.d_elist = c->alloc<int>(nel);
     // the topology of the listed elements' dof map, element slots in list order
@@ -2076,7 +2079,7 @@ extern "C" int sg_stress_bodyload(sg_ctx* c, int neq, int nelmt, int nnode, cons
     for (size_t i = 0; i < gnum0.size(); ++i) gnum0[i] = g_num[i] - 1;
     build_groups_from_gdof(ge_sub.data(), nel, neq, D.T);
     bool ok = D.d_coord && D.d_geo && D.x && D.bl && D.evpt && D.stress && D.Yb && D.wp && D.vm && D.sf && D.part &&
-              D.red && D.d_gnum && D.d_ge && D.d_mat && D.d_elist && upload_topo(c, D.T);
+              D.d_gnum && D.d_ge && D.d_mat && D.d_elist && upload_topo(c, D.T);
     if (!ok) {
       release_sdrop(c);
       set_tag(errtag, "ERROR: out of device memory!");
@@ -2111,11 +2114,13 @@ extern "C" int sg_stress_bodyload(sg_ctx* c, int neq, int nelmt, int nnode, cons
   cudaMemcpyAsync(D.stress, stress_elmt, sizeof(double) * nst, cudaMemcpyHostToDevice, s);
   if (wpressure) cudaMemcpyAsync(D.wp, wpressure, sizeof(double) * nnode, cudaMemcpyHostToDevice, s);
   const bool fields = last && form == 1 && (vmeps || scf);
-  launch_stress_update(D.d_geo, D.d_elist, nel, D.d_ge, D.d_mat, D.x, 1, 0, D.mf, dt, nl_isconv, last, D.evpt,
-                       D.stress, D.Yb, 1, 0, D.part, D.T.d_pos, s, fields ? D.vm : nullptr, fields ? D.sf : nullptr,
+  StressCols one;
+  one.add(0, dt, nl_isconv != 0, last != 0);
+  launch_stress_update(D.d_geo, D.d_elist, nel, D.d_ge, D.d_mat, D.x, 1, D.mf, nmatblk, one, nst, D.evpt, D.stress,
+                       D.Yb, 1, D.part, D.T.d_pos, s, fields ? D.vm : nullptr, fields ? D.sf : nullptr,
                        wpressure ? D.wp : nullptr, D.d_gnum, form);
   double fm = 0.0;
-  reduce_read(c, D.part, NPART, 1, 1, 1, D.red, &fm);
+  reduce_read(c, D.part, stress_blocks(nel), 1, 1, 1, &fm);
   // bodyload(egdof) += bload in element order, unless finalising; bodyload(0) = 0
   if (!last) launch_gather_plain<double>(D.T, 1, D.Yb, D.bl, 1, nullptr, s);
   cudaMemsetAsync(D.bl, 0, sizeof(double), s);

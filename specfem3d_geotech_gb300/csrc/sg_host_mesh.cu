@@ -300,6 +300,12 @@ const KsTables& ks_tables() {
         for (int d = 0; d < 3; ++d) T.entry[ne++] = (3 * n + c) | ((3 * m + d) << 8);
       o += 9;
     }
+  int nb = 0;
+  for (int ndiff = 0; ndiff <= 2; ++ndiff)   // own node: seven shared points, one lattice line: three, else two
+    for (int m = 0; m < NGLL; ++m)
+      for (int n = 0; n <= m; ++n)
+        if ((n % 3 != m % 3) + ((n / 3) % 3 != (m / 3) % 3) + (n / 9 != m / 9) == ndiff)
+          T.border[nb++] = n | (m << 5) | (off[n][m] << 10);
   for (int n = 0; n < NGLL; ++n) {
     int s = 0;
     for (int m = 0; m < NGLL; ++m) {

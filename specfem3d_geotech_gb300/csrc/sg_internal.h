@@ -98,6 +98,7 @@ void build_groups_from_gdof(const int* gdof_elmt, int nelmt, int neq, GatherTopo
 struct KsTables {
   int nbr[NGLL][KS_NBR];   // lane table: m | kind<<5 | off<<8 ; kind 0 own block, 1 stored (n,m), 2 stored (m,n)
   int entry[KS_NNZ];       // (row, col) of each stored entry: row | col<<8, node(row) <= node(col)
+  int border[KS_NNZ / 9];  // stored node blocks n | m<<5 | off<<10, those that share most points first
 };
 const KsTables& ks_tables();
 
@@ -109,7 +110,7 @@ void launch_geometry(const double* g_coord, const int* g_num, int nelmt, double*
 // per element, both gathered later into global vectors.
 void launch_stiffness(const double* geo, const int* mat_id, const int* elist, int nel, const double* ym,
                       const double* nu, const double* gam, double* Ks64, float* Ks32, double* Ydiag,
-                      double* Ygrav, const int* d_entry, const int* pos, cudaStream_t s,
+                      double* Ygrav, const int* d_border, const int* pos, cudaStream_t s,
                       int pseudoeq = 0, double eqkx = 0, double eqky = 0, double eqkz = 0);
 void launch_expand_dense(const double* Ks64, int nel, double* dense, const int* d_entry, cudaStream_t s);
 

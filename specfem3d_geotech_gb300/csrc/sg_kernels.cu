@@ -302,15 +302,28 @@ __device__ __forceinline__ void point_grad(const double* __restrict__ Ji, int i,
 // K(3n+c,3m+d) = sum_i w_i detJ_i [B_i^T C B_i](3n+c,3m+d) with the isotropic
 // C of compute_cmat: for c = d, C11 g_n[c] g_m[c] + C44 sum_{e!=c} g_n[e] g_m[e];
 // for c != d, C12 g_n[c] g_m[d] + C44 g_n[d] g_m[c]  (g = deriv columns).
-// One block per element; threads loop over the 2430 stored entries.
+// One block per element, a thread per stored node block: it forms the nine
+// entries from the two to seven points that the nodes share (a mask), so the
+// products of a gradient with a modulus serve three entries and no thread looks
+// at the other points.  The FP64 unit bounds it (1,000 warp instructions an
+// element at 16 cycles; 6,900 elements in 0.60 ms, against 1.91 ms with a thread
+// per entry looking at all 27 points); own-node blocks, which share seven
+// points, come first so that a warp's threads have equally many.  The roundings
+// are written out: every solve starts from these bits.
 // ---------------------------------------------------------------------------
-constexpr int STIFF_THREADS = 256;
+constexpr int STIFF_THREADS = 288;
+
+// points on the three lattice lines through node n
+__device__ __forceinline__ unsigned line_mask(int n) {
+  const int x = n % 3, y = (n / 3) % 3, z = n / 9;
+  return (7u << (3 * y + 9 * z)) | (0x49u << (x + 9 * z)) | (0x40201u << (x + 3 * y));
+}
 
 __global__ void __launch_bounds__(STIFF_THREADS) k_stiffness(
     const double* __restrict__ geo, const int* __restrict__ mat_id, const int* __restrict__ elist, int nel,
     const double* __restrict__ ym, const double* __restrict__ nu, const double* __restrict__ gam,
     double* __restrict__ Ks64, float* __restrict__ Ks32, double* __restrict__ Ydiag, double* __restrict__ Ygrav,
-    const int* __restrict__ entry, const int* __restrict__ pos, int pseudoeq, double eqkx, double eqky,
+    const int* __restrict__ border, const int* __restrict__ pos, int pseudoeq, double eqkx, double eqky,
     double eqkz) {
   __shared__ double sg[NGLL][NGLL][3];   // grad of node n at point i (zero off the lines)
   __shared__ double sgeo[NGLL][GEO_STRIDE];
@@ -335,32 +348,49 @@ __global__ void __launch_bounds__(STIFF_THREADS) k_stiffness(
     sg[i][n][0] = g[0]; sg[i][n][1] = g[1]; sg[i][n][2] = g[2];
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < KS_NNZ; t += blockDim.x) {
-    int pk = entry[t];
-    int row = pk & 255, col = pk >> 8;
-    int n = row / 3, c = row % 3, m = col / 3, d = col % 3;
-    if (n == m && c > d) { int tmp = c; c = d; d = tmp; }  // exact symmetry inside own-node blocks
-    double acc = 0.0;
-    for (int i = 0; i < NGLL; ++i) {
-      if (!on_line(i, n) || !on_line(i, m)) continue;
+  for (int t = threadIdx.x; t < KS_NNZ / 9; t += blockDim.x) {
+    const int pk = border[t], n = pk & 31, m = (pk >> 5) & 31, off = pk >> 10;
+    double acc[3][3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) acc[c][d] = 0.0;
+    // the points on a lattice line of n and on one of m, in increasing order
+    unsigned pts = line_mask(n) & line_mask(m);
+    while (pts) {
+      const int i = __ffs(pts) - 1;
+      pts &= pts - 1;
       const double* gn = sg[i][n];
       const double* gm = sg[i][m];
-      double b;
-      if (c == d) {
-        int e1 = (c + 1) % 3, e2 = (c + 2) % 3;
-        b = c11 * gn[c] * gm[c] + c44 * (gn[e1] * gm[e1] + gn[e2] * gm[e2]);
-      } else {
-        b = c12 * gn[c] * gm[d] + c44 * gn[d] * gm[c];
+      const double wd = swd[i];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          double b;
+          if (c == d) {
+            const int e1 = (c + 1) % 3, e2 = (c + 2) % 3;
+            const double shear = fma(gn[e1], gm[e1], __dmul_rn(gn[e2], gm[e2]));
+            b = fma(c44, shear, __dmul_rn(__dmul_rn(c11, gn[c]), gm[c]));
+          } else {
+            b = fma(__dmul_rn(c44, gn[d]), gm[c], __dmul_rn(__dmul_rn(c12, gn[c]), gm[d]));
+          }
+          acc[c][d] = fma(b, wd, acc[c][d]);
+        }
+    }
+    const size_t o = (size_t)le * KS_STRIDE + off;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const double v = n == m && c > d ? acc[d][c] : acc[c][d];   // exact symmetry inside own-node blocks
+        if (Ks64) Ks64[o + 3 * c + d] = v;
+        if (Ks32) Ks32[o + 3 * c + d] = (float)v;
+        if (n == m && c == d && Ydiag) {
+          const int ps = pos[(size_t)le * NGLL + n];
+          if (ps >= 0) Ydiag[(size_t)ps * 3 + c] = v;
+        }
       }
-      acc = acc + b * swd[i];
-    }
-    size_t o = (size_t)le * KS_STRIDE + t;
-    if (Ks64) Ks64[o] = acc;
-    if (Ks32) Ks32[o] = (float)acc;
-    if (row == col && Ydiag) {
-      int ps = pos[(size_t)le * NGLL + row / 3];
-      if (ps >= 0) Ydiag[(size_t)ps * 3 + row % 3] = acc;
-    }
   }
   if (Ks64 || Ks32)
     for (int t = KS_NNZ + threadIdx.x; t < KS_STRIDE; t += blockDim.x) {
@@ -384,11 +414,11 @@ __global__ void __launch_bounds__(STIFF_THREADS) k_stiffness(
 
 void launch_stiffness(const double* geo, const int* mat_id, const int* elist, int nel, const double* ym,
                       const double* nu, const double* gam, double* Ks64, float* Ks32, double* Ydiag,
-                      double* Ygrav, const int* d_entry, const int* pos, cudaStream_t s, int pseudoeq,
+                      double* Ygrav, const int* d_border, const int* pos, cudaStream_t s, int pseudoeq,
                       double eqkx, double eqky, double eqkz) {
   if (nel <= 0) return;
   SG_LAUNCH k_stiffness<<<nel, STIFF_THREADS, 0, s>>>(geo, mat_id, elist, nel, ym, nu, gam, Ks64, Ks32, Ydiag, Ygrav,
-                                           d_entry, pos, pseudoeq, eqkx, eqky, eqkz);
+                                           d_border, pos, pseudoeq, eqkx, eqky, eqkz);
 }
 
 // Expand the sparse symmetric layout to the reference's dense column-major
@@ -1757,7 +1787,10 @@ void pcg_update(int n1, V* u, V* r, V* z, const V* p, const V* kp, const V* f, c
 }
 
 // ---------------------------------------------------------------------------
-// K5: one stress / yield / flow / body-load pass for one trial.
+// K5: one stress / yield / flow / body-load pass, block row y for trial column y.
+// The FP64 unit bounds it at large meshes and its latency (some 400 dependent
+// operations a point) at small ones, so all trials go in one launch: at 576
+// elements 219 us for eight trials, against eight launches of 57.
 // One warp per element, lane i < 27 = GLL point i.  Mirrors src/slope.F90:311-383:
 // eps = B x_e - evpt; sigma = C eps; eff = sigma + stress; invariants
 // (stress_invariant), F (mohcouf); if F >= 0: dQ (mohcouq), M1..M3 (formm),
@@ -1769,12 +1802,29 @@ void pcg_update(int n1, V* u, V* r, V* z, const V* p, const V* kp, const V* f, c
 constexpr int STRESS_WARPS = 4;
 constexpr double DEG2RAD_D = 3.141592653589793 / 180.0;
 
+// x / b for a constant b, correctly rounded: the quotient by the rounded
+// reciprocal, its exact remainder and one correction (P. Markstein,
+// Computation of elementary functions on the IBM RISC System/6000 processor,
+// IBM J. Res. Dev. 34, 1990, theorem 7).  Three FP64 operations: 24,000 elements
+// in 1.20 ms, against 1.36 with the general divisions by 3, 6 and sqrt(3).
+__device__ __forceinline__ double div_const(double x, double b, double rb) {
+  const double q = x * rb;
+  return fma(fma(-b, q, x), rb, q);
+}
+template <int B>
+__device__ __forceinline__ double div_by(double x) { return div_const(x, (double)B, 1.0 / (double)B); }
+__device__ __forceinline__ double div3(double x) { return div_by<3>(x); }
+__device__ __forceinline__ double div_sq3(double x) {
+  constexpr double SQ3 = 1.7320508075688772;   // the double nearest sqrt(3)
+  return div_const(x, SQ3, 1.0 / SQ3);
+}
+
 __device__ __forceinline__ void stress_invariant_d(const double* s, double& sigm, double& dsbar, double& theta) {
-  const double small = 1.e-12, three = 3.0, six = 6.0;
+  const double small = 1.e-12, three = 3.0;
   const double sq3 = sqrt(three);
   double s1 = s[0], s2 = s[1], s3 = s[2], s4 = s[3], s5 = s[4], s6 = s[5];
-  sigm = (s1 + s2 + s3) / three;
-  double d2 = ((s1 - s2) * (s1 - s2) + (s2 - s3) * (s2 - s3) + (s3 - s1) * (s3 - s1)) / six + s4 * s4 + s5 * s5 +
+  sigm = div3(s1 + s2 + s3);
+  double d2 = div_by<6>((s1 - s2) * (s1 - s2) + (s2 - s3) * (s2 - s3) + (s3 - s1) * (s3 - s1)) + s4 * s4 + s5 * s5 +
               s6 * s6;
   if (d2 < small) d2 = small;
   double ds1 = s1 - sigm, ds2 = s2 - sigm, ds3 = s3 - sigm;
@@ -1787,17 +1837,22 @@ __device__ __forceinline__ void stress_invariant_d(const double* s, double& sigm
     double sine = -three * sq3 * d3 / (2.0 * (sq * sq * sq));
     if (sine >= 1.0) sine = 1.0;
     if (sine < -1.0) sine = -1.0;
-    theta = asin(sine) / three;
+    theta = div3(asin(sine));
   }
 }
 
 __global__ void __launch_bounds__(STRESS_WARPS * 32) k_stress_update(
     const double* __restrict__ geo, const int* __restrict__ elist, int nel, const int* __restrict__ ge,
-    const int* __restrict__ mat_id, const double* __restrict__ x, int xstride, int xcol, const MatF* __restrict__ mf,
-    double dt, int nl_isconv, int finalize, double* __restrict__ evpt, double* __restrict__ stress,
-    double* __restrict__ Yb, int ystride, int ycol, double* __restrict__ fmax_part, const int* __restrict__ pos,
-    double* __restrict__ vm_pt, double* __restrict__ sf_pt, const double* __restrict__ wp,
-    const int* __restrict__ gnum, int wp_first) {
+    const int* __restrict__ mat_id, const double* __restrict__ x, int xstride, const MatF* __restrict__ mf0, int nmat,
+    StressCols C, size_t nst, double* __restrict__ evpt0, double* __restrict__ stress0, double* __restrict__ Yb,
+    int ystride, double* __restrict__ fmax_part, const int* __restrict__ pos, double* __restrict__ vm_pt,
+    double* __restrict__ sf_pt, const double* __restrict__ wp, const int* __restrict__ gnum, int wp_first) {
+  const int xcol = C.col[blockIdx.y], ycol = xcol;
+  const double dt = C.dt[blockIdx.y];
+  const bool finalize = C.fin[blockIdx.y], nl_isconv = C.conv[blockIdx.y];
+  const MatF* mf = mf0 + (size_t)xcol * nmat;
+  double* evpt = evpt0 + nst * xcol;
+  double* stress = stress0 + nst * xcol;
   __shared__ double s_eld[STRESS_WARPS][NEDOF];
   __shared__ double s_q[STRESS_WARPS][NGLL][9];
   __shared__ double s_fmax[STRESS_WARPS];
@@ -1871,7 +1926,8 @@ __global__ void __launch_bounds__(STRESS_WARPS * 32) k_stress_update(
       sincos(theta, &snth, &csth);
       const double r3 = 3.0, sq3 = sqrt(3.0);
       // mohcouf (src/plastic_library.f90:95-108)
-      double f = m.snph * sigm + dsbar * (csth / sq3 - snth * m.snph / r3) - m.cohf * m.csph;
+      const double yield = div_sq3(csth) - div3(snth * m.snph);
+      double f = m.snph * sigm + dsbar * yield - m.cohf * m.csph;
       fmax_l = fmax(fmax_l, f);
       double q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
       if (f >= 0.0) {
@@ -1879,19 +1935,19 @@ __global__ void __launch_bounds__(STRESS_WARPS * 32) k_stress_update(
         double dq1 = m.snps, dq2, dq3;
         if (fabs(snth) > 0.49) {
           double c1 = snth < 0.0 ? -1.0 : 1.0;
-          dq2 = (sq3 * 0.5 - c1 * m.snps * 0.5 / sq3) * sq3 * 0.5 / dsbar;
+          dq2 = (sq3 * 0.5 - div_sq3(c1 * m.snps * 0.5)) * sq3 * 0.5 / dsbar;
           dq3 = 0.0;
         } else {
           double cs3th = cos(r3 * theta), tn3th = tan(r3 * theta), tnth = snth / csth;
-          dq2 = sq3 * csth / dsbar * ((1.0 + tnth * tn3th) + m.snps * (tn3th - tnth) / sq3) * 0.5;
+          dq2 = sq3 * csth / dsbar * ((1.0 + tnth * tn3th) + div_sq3(m.snps * (tn3th - tnth))) * 0.5;
           dq3 = 0.5 * r3 * (sq3 * snth + m.snps * csth) / (cs3th * dsbar * dsbar);
         }
         // formm (src/plastic_library.f90:150-208): M1, M2, M3 (divided by 3)
         const double sx = eff[0], sy = eff[1], sz = eff[2], txy = eff[3], tyz = eff[4], tzx = eff[5];
-        const double sgm = (sx + sy + sz) / r3;
+        const double sgm = div3(sx + sy + sz);
         const double dx = sx - sgm, dy = sy - sgm, dz = sz - sgm;
         double M[6][6];
-        const double m1v = 1.0 / (r3 * sgm) / r3;
+        const double m1v = div3(1.0 / (r3 * sgm));
 #pragma unroll
         for (int a = 0; a < 6; ++a)
 #pragma unroll
@@ -1911,7 +1967,7 @@ __global__ void __launch_bounds__(STRESS_WARPS * 32) k_stress_update(
             double m2 = 0.0;
             if (a == b) m2 = (a < 3 ? 2.0 : 6.0) / r3;
             else if (b < 3) m2 = -1.0 / r3;
-            double v = f * (m1 * dq1 + m2 * dq2 + (m3[a][b] / r3) * dq3);
+            double v = f * (m1 * dq1 + m2 * dq2 + div3(m3[a][b]) * dq3);
             M[a][b] = v;
             M[b][a] = v;
           }
@@ -1952,7 +2008,7 @@ __global__ void __launch_bounds__(STRESS_WARPS * 32) k_stress_update(
         }
         if (sf_pt)
           sf_pt[(size_t)le * NGLL + i] =
-              (sigm * m.snph - m.cohf * m.csph) / (-dsbar * (csth / sq3 - snth * m.snph / r3));
+              (sigm * m.snph - m.cohf * m.csph) / (-dsbar * yield);
       }
 #pragma unroll
       for (int t = 0; t < 9; ++t) s_q[warp][i][t] = q[t];
@@ -1996,19 +2052,20 @@ __global__ void __launch_bounds__(STRESS_WARPS * 32) k_stress_update(
   if (threadIdx.x == 0) {
     double v = 0.0;
     for (int w = 0; w < STRESS_WARPS; ++w) v = fmax(v, s_fmax[w]);
-    fmax_part[blockIdx.x] = v;
+    fmax_part[(size_t)blockIdx.x * C.stride() + blockIdx.y] = v;
   }
 }
 
+int stress_blocks(int nel) { return std::max(1, std::min((nel + STRESS_WARPS - 1) / STRESS_WARPS, NPART)); }
+
 void launch_stress_update(const double* geo, const int* elist, int nel, const int* ge_glob, const int* mat_id,
-                          const double* x, int xstride, int xcol, const MatF* mf, double dt, int nl_isconv,
-                          int finalize, double* evpt, double* stress, double* Yb, int ystride, int ycol,
-                          double* fmax_part, const int* pos, cudaStream_t s, double* vm_pt, double* sf_pt,
-                          const double* wp, const int* gnum, int wp_first) {
-  // fixed grid so that fmax_part has NPART entries
-  SG_LAUNCH k_stress_update<<<NPART, STRESS_WARPS * 32, 0, s>>>(geo, elist, nel, ge_glob, mat_id, x, xstride, xcol, mf, dt,
-                                                       nl_isconv, finalize, evpt, stress, Yb, ystride, ycol,
-                                                       fmax_part, pos, vm_pt, sf_pt, wp, gnum, wp_first);
+                          const double* x, int xstride, const MatF* mf, int nmat, const StressCols& C, size_t nst,
+                          double* evpt, double* stress, double* Yb, int ystride, double* fmax_part, const int* pos,
+                          cudaStream_t s, double* vm_pt, double* sf_pt, const double* wp, const int* gnum,
+                          int wp_first) {
+  SG_LAUNCH k_stress_update<<<dim3(stress_blocks(nel), C.n), STRESS_WARPS * 32, 0, s>>>(
+      geo, elist, nel, ge_glob, mat_id, x, xstride, mf, nmat, C, nst, evpt, stress, Yb, ystride, fmax_part, pos, vm_pt,
+      sf_pt, wp, gnum, wp_first);
 }
 
 // ---------------------------------------------------------------------------
@@ -2230,35 +2287,74 @@ void launch_release_load(const double* geo, const int* elist, int nel, const int
 }
 
 // ---------------------------------------------------------------------------
-// Small vector kernels with per-column reductions written to part[NPART][KR][q].
+// Small vector kernels with per-column reductions written to part[block][KR][2].
+// A thread's column is fixed (its index mod KR).  Sums and maxima go over the
+// lanes of a column by shuffles, maxima on the bits of the absolute values: an
+// FP64 add or compare holds the SM's FP64 unit for 16 cycles a warp and takes
+// some 70 to answer, and a serial tail over 256 threads made these kernels 33 us
+// each on a mesh whose data they read in three.
 // ---------------------------------------------------------------------------
+static inline int vec_grid(int n1, int KR) { return red_grid((size_t)n1 * KR, RED_THREADS * 4, NPART); }
+int vec_blocks(int n1, int KR) { return vec_grid(n1, KR); }
+
+__device__ __forceinline__ unsigned long long mag_bits(double x) {   // |x|; a NaN counts as 0, as fmax has it
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+  return b > 0x7ff0000000000000ull ? 0ull : b;
+}
+__device__ __forceinline__ void block_pair_max(unsigned long long a, unsigned long long b, int KR,
+                                               double* __restrict__ part) {
+  __shared__ unsigned long long s[RED_THREADS / 32][32][2];
+  for (int o = 16; o >= KR; o >>= 1) {
+    const unsigned long long x = __shfl_xor_sync(FULL, a, o), y = __shfl_xor_sync(FULL, b, o);
+    a = a > x ? a : x;
+    b = b > y ? b : y;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane < KR) { s[warp][lane][0] = a; s[warp][lane][1] = b; }
+  __syncthreads();
+  if (threadIdx.x < 2 * KR) {
+    const int j = threadIdx.x >> 1, q = threadIdx.x & 1;
+    unsigned long long v = 0;
+#pragma unroll
+    for (int w = 0; w < RED_THREADS / 32; ++w) v = v > s[w][j][q] ? v : s[w][j][q];
+    part[((size_t)blockIdx.x * KR + j) * 2 + q] = __longlong_as_double((long long)v);
+  }
+}
+__device__ __forceinline__ void block_pair_sum(double a, double b, int KR, double* __restrict__ part) {
+  __shared__ double s[RED_THREADS / 32][32][2];
+  for (int o = 16; o >= KR; o >>= 1) {
+    a += __shfl_xor_sync(FULL, a, o);
+    b += __shfl_xor_sync(FULL, b, o);
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane < KR) { s[warp][lane][0] = a; s[warp][lane][1] = b; }
+  __syncthreads();
+  if (threadIdx.x < 2 * KR) {
+    const int j = threadIdx.x >> 1, q = threadIdx.x & 1;
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < RED_THREADS / 32; ++w) v += s[w][j][q];
+    part[((size_t)blockIdx.x * KR + j) * 2 + q] = v;
+  }
+}
+
 // K8 nl check (src/slope.F90:307-309): max|x-oldx|, max|x| per column, oldx = x.
-__global__ void k_nl_check(int n1, int KR, const double* __restrict__ x, double* __restrict__ oldx,
-                           double* __restrict__ part) {
-  __shared__ double s[RED_THREADS][2];
-  double a = 0.0, b = 0.0;
-  const int j = threadIdx.x % KR;
+__global__ void __launch_bounds__(RED_THREADS) k_nl_check(int n1, int KR, const double* __restrict__ x,
+                                                          double* __restrict__ oldx, double* __restrict__ part) {
+  unsigned long long a = 0, b = 0;
   const size_t n = (size_t)n1 * KR;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double xi = x[i];
-    a = fmax(a, fabs(xi - oldx[i]));
-    b = fmax(b, fabs(xi));
+    const double xi = x[i];
+    a = max(a, mag_bits(xi - oldx[i]));
+    b = max(b, mag_bits(xi));
     oldx[i] = xi;
   }
-  s[threadIdx.x][0] = a;
-  s[threadIdx.x][1] = b;
-  __syncthreads();
-  if (threadIdx.x < KR) {
-    double A = 0.0, B = 0.0;
-    for (int t = threadIdx.x; t < RED_THREADS; t += KR) { A = fmax(A, s[t][0]); B = fmax(B, s[t][1]); }
-    part[((size_t)blockIdx.x * KR + j) * 2] = A;
-    part[((size_t)blockIdx.x * KR + j) * 2 + 1] = B;
-  }
+  block_pair_max(a, b, KR, part);
 }
 
 void launch_nl_check(int n1, int KR, int k, const double* x, double* oldx, double* part, cudaStream_t s) {
   (void)k;
-  SG_LAUNCH k_nl_check<<<NPART, RED_THREADS, 0, s>>>(n1, KR, x, oldx, part);
+  SG_LAUNCH k_nl_check<<<vec_grid(n1, KR), RED_THREADS, 0, s>>>(n1, KR, x, oldx, part);
 }
 
 // load = extload + bodyload; load(0) = 0 (src/slope.F90:288-289)
@@ -2273,71 +2369,53 @@ __global__ void k_load_combine(int n1, int KR, const double* __restrict__ ext, c
 
 void launch_load_combine(int n1, int KR, const double* extload, const double* bodyload, double* load,
                          cudaStream_t s) {
-  SG_LAUNCH k_load_combine<<<NPART, RED_THREADS, 0, s>>>(n1, KR, extload, bodyload, load);
+  SG_LAUNCH k_load_combine<<<vec_grid(n1, KR), RED_THREADS, 0, s>>>(n1, KR, extload, bodyload, load);
 }
 
 // r64 = f - kp (FP64), r32 = (float) r64; partials |r|^2, |f|^2 per column.
-__global__ void k_residual(int n1, int KR, const double* __restrict__ f, const double* __restrict__ kp,
-                           double* __restrict__ r64, float* __restrict__ r32, double* __restrict__ part) {
-  __shared__ double s[RED_THREADS][2];
+__global__ void __launch_bounds__(RED_THREADS) k_residual(int n1, int KR, const double* __restrict__ f,
+                                                          const double* __restrict__ kp, double* __restrict__ r64,
+                                                          float* __restrict__ r32, double* __restrict__ part) {
   double a = 0.0, b = 0.0;
-  const int j = threadIdx.x % KR;
   const size_t n = (size_t)n1 * KR;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double ri = (i < (size_t)KR) ? 0.0 : f[i] - kp[i];
+    const double fi = f[i], ri = (i < (size_t)KR) ? 0.0 : fi - kp[i];
     r64[i] = ri;
     r32[i] = (float)ri;
     a += ri * ri;
-    b += f[i] * f[i];
+    b += fi * fi;
   }
-  s[threadIdx.x][0] = a;
-  s[threadIdx.x][1] = b;
-  __syncthreads();
-  if (threadIdx.x < KR) {
-    double A = 0.0, B = 0.0;
-    for (int t = threadIdx.x; t < RED_THREADS; t += KR) { A += s[t][0]; B += s[t][1]; }
-    part[((size_t)blockIdx.x * KR + j) * 2] = A;
-    part[((size_t)blockIdx.x * KR + j) * 2 + 1] = B;
-  }
+  block_pair_sum(a, b, KR, part);
 }
 
 void launch_residual_norms(int n1, int KR, const double* f, const double* kp, double* r64, float* r32,
                            double* part, cudaStream_t s) {
-  SG_LAUNCH k_residual<<<NPART, RED_THREADS, 0, s>>>(n1, KR, f, kp, r64, r32, part);
+  SG_LAUNCH k_residual<<<vec_grid(n1, KR), RED_THREADS, 0, s>>>(n1, KR, f, kp, r64, r32, part);
 }
 
 // x += d for the columns in colmask; partials max|d|, max|x| per column.
-__global__ void k_axpy_corr(int n1, int KR, const int* __restrict__ colmask, const float* __restrict__ d,
-                            double* __restrict__ x, double* __restrict__ part) {
-  __shared__ double s[RED_THREADS][2];
-  double a = 0.0, b = 0.0;
-  const int j = threadIdx.x % KR;
-  const bool on = colmask[j] != 0;
+__global__ void __launch_bounds__(RED_THREADS) k_axpy_corr(int n1, int KR, const int* __restrict__ colmask,
+                                                           const float* __restrict__ d, double* __restrict__ x,
+                                                           double* __restrict__ part) {
+  unsigned long long a = 0, b = 0;
+  const bool on = colmask[threadIdx.x % KR] != 0;
   const size_t n = (size_t)n1 * KR;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     double xi = x[i];
     if (on) {
-      double di = (double)d[i];
+      const double di = (double)d[i];
       xi = xi + di;
       x[i] = xi;
-      a = fmax(a, fabs(di));
+      a = max(a, mag_bits(di));
     }
-    b = fmax(b, fabs(xi));
+    b = max(b, mag_bits(xi));
   }
-  s[threadIdx.x][0] = a;
-  s[threadIdx.x][1] = b;
-  __syncthreads();
-  if (threadIdx.x < KR) {
-    double A = 0.0, B = 0.0;
-    for (int t = threadIdx.x; t < RED_THREADS; t += KR) { A = fmax(A, s[t][0]); B = fmax(B, s[t][1]); }
-    part[((size_t)blockIdx.x * KR + j) * 2] = A;
-    part[((size_t)blockIdx.x * KR + j) * 2 + 1] = B;
-  }
+  block_pair_max(a, b, KR, part);
 }
 
 void launch_axpy_correction(int n1, int KR, const int* colmask, const float* d, double* x, double* part,
                             cudaStream_t s) {
-  SG_LAUNCH k_axpy_corr<<<NPART, RED_THREADS, 0, s>>>(n1, KR, colmask, d, x, part);
+  SG_LAUNCH k_axpy_corr<<<vec_grid(n1, KR), RED_THREADS, 0, s>>>(n1, KR, colmask, d, x, part);
 }
 
 // dprecon(1:) = 1/dprecon(1:), dprecon(0) = 0 (src/slope.F90:199), plus an FP32 copy.
@@ -2377,26 +2455,32 @@ template void launch_gather_plain<float>(const GatherTopo&, int, const float*, f
                                          cudaStream_t);
 
 // Fixed-order reduction of block partials part[nblk][KR][nq] into out[KR][nq];
-// bit q of maxmask selects max instead of sum for quantity q.
-__global__ void k_final_reduce(const double* __restrict__ part, int nblk, int KR, int nq, int maxmask,
-                               double* __restrict__ out) {
-  // thread t owns entry t % (KR*nq) of blocks t/(KR*nq), ...; 256 threads, KR*nq <= 64 divides 256
+// bit q of maxmask selects max instead of sum for quantity q.  Thread t owns
+// entry t % (KR*nq) of blocks t/(KR*nq), ... (KR*nq <= 64 divides 256), eight
+// loads in flight; the entry's threads are then added by halves.
+__global__ void __launch_bounds__(256) k_final_reduce(const double* __restrict__ part, int nblk, int KR, int nq,
+                                                      int maxmask, double* __restrict__ out) {
   __shared__ double s[256];
-  const int W = KR * nq;
-  const int e = threadIdx.x % W, q = e % nq;
-  const bool mx = (maxmask >> q) & 1;
+  const int W = KR * nq, n = nblk * W;
+  const bool mx = (maxmask >> (threadIdx.x % W % nq)) & 1;
   double v = 0.0;
-  for (int idx = threadIdx.x; idx < nblk * W; idx += blockDim.x) {
-    double x = part[idx];
-    v = mx ? fmax(v, x) : v + x;
+  for (int i0 = threadIdx.x; i0 < n; i0 += 8 * 256) {
+    double x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = i0 + 256 * k < n ? part[i0 + 256 * k] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v = mx ? fmax(v, x[k]) : v + x[k];
   }
   s[threadIdx.x] = v;
   __syncthreads();
-  if (threadIdx.x < W) {
-    double r = 0.0;
-    for (int t = threadIdx.x; t < (int)blockDim.x; t += W) r = mx ? fmax(r, s[t]) : r + s[t];
-    out[threadIdx.x] = r;
+  for (int h = 128; h >= W; h >>= 1) {
+    if ((int)threadIdx.x < h) {
+      v = mx ? fmax(v, s[threadIdx.x + h]) : v + s[threadIdx.x + h];
+      s[threadIdx.x] = v;
+    }
+    __syncthreads();
   }
+  if ((int)threadIdx.x < W) out[threadIdx.x] = v;
 }
 
 void launch_final_reduce(const double* part, int nblk, int KR, int nq, int maxmask, double* out, cudaStream_t s) {
@@ -2405,33 +2489,25 @@ void launch_final_reduce(const double* part, int nblk, int KR, int nq, int maxma
 
 // Nodal displacement maxima of one column (src/slope.F90:400-415):
 // part[b][0] = max |u_d| over nodes and dofs, part[b][1] = max |u| (node norm).
-__global__ void k_disp_max(int nnode, const int* __restrict__ gdof, const double* __restrict__ x, int KR, int col,
-                           double* __restrict__ part) {
-  __shared__ double s[RED_THREADS][2];
-  double a = 0.0, b = 0.0;
+__global__ void __launch_bounds__(RED_THREADS) k_disp_max(int nnode, const int* __restrict__ gdof,
+                                                          const double* __restrict__ x, int KR, int col,
+                                                          double* __restrict__ part) {
+  unsigned long long a = 0, b = 0;
   for (int nd = blockIdx.x * blockDim.x + threadIdx.x; nd < nnode; nd += gridDim.x * blockDim.x) {
     double u[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       int g = gdof[3 * nd + d];
       u[d] = g ? x[(size_t)g * KR + col] : 0.0;
-      a = fmax(a, fabs(u[d]));
+      a = max(a, mag_bits(u[d]));
     }
-    b = fmax(b, sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]));
+    b = max(b, mag_bits(sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2])));
   }
-  s[threadIdx.x][0] = a;
-  s[threadIdx.x][1] = b;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double A = 0.0, B = 0.0;
-    for (int t = 0; t < RED_THREADS; ++t) { A = fmax(A, s[t][0]); B = fmax(B, s[t][1]); }
-    part[2 * blockIdx.x] = A;
-    part[2 * blockIdx.x + 1] = B;
-  }
+  block_pair_max(a, b, 1, part);
 }
 
 void launch_disp_max(int nnode, const int* gdof, const double* x, int KR, int col, double* part, cudaStream_t s) {
-  SG_LAUNCH k_disp_max<<<NPART, RED_THREADS, 0, s>>>(nnode, gdof, x, KR, col, part);
+  SG_LAUNCH k_disp_max<<<vec_grid(nnode, 1), RED_THREADS, 0, s>>>(nnode, gdof, x, KR, col, part);
 }
 
 // x(:,col) /= n etc.: y[i*KR+col] = a*y[i*KR+col] (all columns when col < 0)
@@ -2447,7 +2523,7 @@ __global__ void k_col_zero(int n1, int KR, int j, double* __restrict__ a, double
   }
 }
 void launch_col_zero(int n1, int KR, int j, double* a, double* b, double* c, cudaStream_t s) {
-  SG_LAUNCH k_col_zero<<<NPART, RED_THREADS, 0, s>>>(n1, KR, j, a, b, c);
+  SG_LAUNCH k_col_zero<<<vec_grid(n1, 1), RED_THREADS, 0, s>>>(n1, KR, j, a, b, c);
 }
 
 void launch_div(size_t n, double* y, double a, cudaStream_t s) { SG_LAUNCH k_scale<<<NPART, RED_THREADS, 0, s>>>(n, y, a); }

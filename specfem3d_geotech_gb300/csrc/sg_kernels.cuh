@@ -124,13 +124,29 @@ template <typename V, int KR>
 void pcg_update(int n1, V* u, V* r, V* z, const V* p, const V* kp, const V* f, const V* dprecon, int init,
                 ColState* cs, PcgGlobal* G, double* part, cudaStream_t s);
 
-// Yb layout [nel][81][ystride] at column ycol (ystride = KR of the trial batch)
+// The trial columns of a stress pass: column, pseudo-time step, and whether it
+// has converged or is at its last pass.
+struct StressCols {
+  int n = 0;
+  int col[16];
+  unsigned char conv[16], fin[16];
+  double dt[16];
+  void add(int c, double dtc, bool cv, bool fn) {
+    col[n] = c; dt[n] = dtc; conv[n] = cv; fin[n] = fn;
+    ++n;
+  }
+  // columns of the block maxima: n rounded up to a power of two
+  __host__ __device__ int stride() const { return n <= 1 ? 1 : n <= 2 ? 2 : n <= 4 ? 4 : n <= 8 ? 8 : 16; }
+};
+// Column c uses mf + c * nmat, evpt and stress + c * nst, and column c of x and
+// Yb; fmax_part gets [stress_blocks(nel)][C.stride()] block maxima.
 void launch_stress_update(const double* geo, const int* elist, int nel, const int* ge_glob, const int* mat_id,
-                          const double* x, int xstride, int xcol, const MatF* mf, double dt, int nl_isconv,
-                          int finalize, double* evpt, double* stress, double* Yb, int ystride, int ycol,
-                          double* fmax_part, const int* pos, cudaStream_t s, double* vm_pt = nullptr,
-                          double* sf_pt = nullptr, const double* wp = nullptr, const int* gnum = nullptr,
-                          int wp_first = 0);
+                          const double* x, int xstride, const MatF* mf, int nmat, const StressCols& C, size_t nst,
+                          double* evpt, double* stress, double* Yb, int ystride, double* fmax_part, const int* pos,
+                          cudaStream_t s, double* vm_pt = nullptr, double* sf_pt = nullptr,
+                          const double* wp = nullptr, const int* gnum = nullptr, int wp_first = 0);
+int stress_blocks(int nel);
+int vec_blocks(int n1, int KR);   // blocks, and partials, of the vector kernels below
 // submerged-node flags and hydrostatic pore pressure per node; err (set to
 // INT_MAX by the caller) gets the smallest node + 1 whose free surface cannot
 // be determined
