@@ -248,9 +248,10 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
   cudaMemcpyAsync(B.cs, hcs, sizeof(ColState) * KR, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(B.G, &hg, sizeof(hg), cudaMemcpyHostToDevice, s);
   if (!keep_dir) cudaMemsetAsync(B.p, 0, sizeof(V) * (size_t)n1 * KR, s);
+  if (mode & 4) cudaMemsetAsync(u, 0, sizeof(V) * (size_t)n1 * KR, s);
   cudaMemsetAsync(B.kp, 0, sizeof(V) * (size_t)n1 * KR, s);
   int ev;
-  if (!(mode & 4)) {  // bit 2: the caller guarantees u = 0, so kp = K u = 0 without an apply
+  if (!(mode & 4)) {  // bit 2: the solve starts from u = 0, so kp = K u = 0 without an apply
     ev = C->prof_begin();
     pcg_apply<V, KR>(op.dense, op.K, op.ge, op.nelmt, u, (const V*)nullptr, 0, B.Y, B.cs, B.G, C->d_nbr, op.T->d_pos,
                      &B.G->err, s);
@@ -310,14 +311,10 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
       (uintptr_t)C->d_nbr, (uintptr_t)B.Y, (uintptr_t)B.kp, (uintptr_t)B.p, (uintptr_t)B.z, (uintptr_t)B.r,
       (uintptr_t)B.cs, (uintptr_t)B.G, (uintptr_t)B.part, (uintptr_t)u, (uintptr_t)f, (uintptr_t)dp,
       (uintptr_t)n1, (uintptr_t)KR, (uintptr_t)sizeof(V), (uintptr_t)chunk, (uintptr_t)fused};
-  // small and medium meshes with the matrix-free FP32 operator: the whole chunk
-  // as one persistent cooperative launch (sg_pcg_persist.cu).  It stops by
-  // itself at the solve's end, so the chunk only bounds the time between two
-  // looks of the host.
+  // FP64, one column: the matrices' products bound every size (sg_pcg_persist64.cu).
+  // The chunk stops by itself at the solve's end; its length only bounds the
+  // time between two looks of the host.
   bool persist = false;
-  if constexpr (std::is_same<V, float>::value)
-    persist = op.dense == 2 && (mode & 1) && op.nelmt < persist_max_elements(KR) && persist_enabled();
-  // FP64, one column: the matrices' products bound every size (sg_pcg_persist64.cu)
   if constexpr (std::is_same<V, double>::value && KR == 1)
     persist = !(mode & 1) && (op.dense == 0 ? persist_default_apply() : op.rows != nullptr) && persist_enabled();
   constexpr int persist_chunk = 512;
@@ -330,13 +327,6 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
         done_chunk = launch_pcg_persistent64(op.dense != 0, op.dense ? op.rows : (const double*)op.K, op.ge, op.nelmt,
                                              op.T->d_pos, C->d_nbr, *op.T, n1, u, B.r, B.z, B.p, B.kp, B.Y, dp, B.cs,
                                              B.G, B.part, persist_chunk, s);
-        C->prof_end(ev, 0);
-      }
-    if constexpr (std::is_same<V, float>::value)
-      if (persist) {
-        ev = C->prof_begin();
-        done_chunk = launch_pcg_persistent<KR>((const float*)op.K, op.ge, op.nelmt, op.T->d_pos, *op.T, u, B.r, B.z,
-                                               B.p, B.kp, B.Y, dp, B.cs, B.G, B.part, persist_chunk, s);
         C->prof_end(ev, 0);
       }
     cudaGraphExec_t ex = (!done_chunk && graphs && nchunks > 0) ? C->chunk_graph(key, eager_chunk) : nullptr;
@@ -1116,10 +1106,11 @@ static void make_matf(int nmat, const double* ymv, const double* nuf, const doub
 
 // Reads KR*nq reduced values (fixed-order device reduction) to the host; the
 // reduction writes them to pinned host memory itself.
-static void reduce_read(sg_ctx* c, const double* part, int nblk, int KR, int nq, int maxmask, double* h_out) {
-  launch_final_reduce(part, nblk, KR, nq, maxmask, c->pin + 256, c->stream);
+static void reduce_read(sg_ctx* c, const double* part, int nblk, int KR, int nq, int maxmask, double* h_out,
+                        const double* part2 = nullptr) {
+  launch_final_reduce(part, nblk, KR, nq, maxmask, c->pin + 256, c->stream, part2);
   cudaStreamSynchronize(c->stream);
-  std::memcpy(h_out, c->pin + 256, sizeof(double) * KR * nq);
+  std::memcpy(h_out, c->pin + 256, sizeof(double) * KR * nq * (part2 ? 2 : 1));
 }
 
 // ---------------------------------------------------------------------------
@@ -1147,6 +1138,25 @@ static Op fp32_op(const sg_model* M, const Op& op64) {
   return o;
 }
 
+// One persistent FP32 solve, or its next chunk; false when it cannot run.
+static bool persist_round(sg_ctx* c, int KR, const Op& op, TrialWork& W, const float* dp, const PersistStart& st,
+                          PersistOut* out) {
+  constexpr int chunk = 4096;   // bounds the time between two looks of the host
+  auto run = [&](auto kr) {
+    return launch_pcg_persistent<decltype(kr)::value>((const float*)op.K, op.ge, op.nelmt, op.T->d_pos, *op.T, W.r32,
+                                                      W.d32, W.b32.r, W.b32.z, W.b32.p, W.b32.kp, W.b32.Y, dp,
+                                                      W.b32.cs, W.b32.G, W.b32.part, st, out, chunk, c->stream);
+  };
+  switch (KR) {
+    case 1: return run(std::integral_constant<int, 1>{});
+    case 2: return run(std::integral_constant<int, 2>{});
+    case 4: return run(std::integral_constant<int, 4>{});
+    case 8: return run(std::integral_constant<int, 8>{});
+    case 16: return run(std::integral_constant<int, 16>{});
+  }
+  return false;
+}
+
 static int linear_solve(sg_model* M, const sg_control* ctl, const Op& op64, const Op& op32, int k,
                         const std::vector<int>& active, SolveStats& S, const double* dprecon, const float* dprecon32) {
   sg_ctx* c = M->ctx;
@@ -1169,10 +1179,51 @@ static int linear_solve(sg_model* M, const sg_control* ctl, const Op& op64, cons
   // across rounds; each round ends when its recursive residual has dropped by
   // itol, the correction is added to the FP64 solution, and the FP32 residual
   // is replaced by the true residual f - K64 x computed in FP64.
-  for (int round = 0; round < 200; ++round) {
+  //
+  // With the persistent solve a round is one chain of launches and one wait:
+  // solve, correction (which the device skips while the solve is not done), FP64
+  // residual, and the norms and maxima together.
+  bool persist = op32.dense == 2 && op32.nelmt < persist_max_elements(KR) && persist_enabled();
+  PersistOut* out = reinterpret_cast<PersistOut*>(c->pin + 384);
+  double* corr_part = W.b64.part + (size_t)NPART * 32;   // the residual's partials take the first half
+  bool pending = false;                                  // a persistent solve and its correction are under way
+  bool fresh = true;                                     // no solve of this call has finished yet
+  unsigned mask = 0;
+  auto launch = [&](bool init) -> bool {
+    const PersistStart st{init, !fresh, ctl->cg_maxiter, k, mask, itol};
+    out->state = PERSIST_NONE;
+    int ev = c->prof_begin();
+    const bool ok = persist_round(c, KR, op32, W, dprecon32, st, out);
+    c->prof_end(ev, 0);
+    if (ok) launch_axpy_correction(n1, KR, mask, W.b32.G, W.d32, W.x, corr_part, c->stream);
+    return ok;
+  };
+  auto judge_steps = [&](const double* m, const double* step) {
+    // the reference's step test on the last CG step: |alpha|*max|p| <= cg_tol*max|x|
+    for (int j = 0; j < k; ++j)
+      if (live[j]) step_ok[j] = (m[2 * j + 1] > 0) && (step[j] <= ctl->cg_tol * m[2 * j + 1]);
+  };
+  for (int round = 0; round < 200;) {
     apply_plain<double>(c, KR, op64, W.x, W.Yb, W.kp64);
     launch_residual_norms(n1, KR, W.load, W.kp64, W.r64, W.r32, W.b64.part, c->stream);
-    reduce_read(c, W.b64.part, vec_blocks(n1, KR), KR, 2, 0, red);
+    reduce_read(c, W.b64.part, vec_blocks(n1, KR), KR, 2, 0, red, pending ? corr_part : nullptr);
+    if (pending) {
+      if (!c->check(cudaGetLastError(), "pcg")) return SG_ERR_CUDA;
+      if (out->state == PERSIST_NONE) {
+        c->err = "PCG: a bounded wait timed out";
+        return SG_ERR_TIMEOUT;
+      }
+      if (out->state == PERSIST_MORE) {   // the chunk ended first: nothing was added to x
+        if (!launch(false)) { c->err = "PCG: the persistent solve could not continue"; return SG_ERR_CUDA; }
+        continue;
+      }
+      pending = fresh = false;
+      ++round;
+      c->prof.counts[2] += out->it;
+      for (int j = 0; j < k; ++j)
+        if (live[j]) S.iters[j] += out->iters[j];
+      judge_steps(red + 2 * KR, out->step);
+    }
     S.refine++;
     c->prof.counts[3]++;
     bool any = false;
@@ -1186,24 +1237,25 @@ static int linear_solve(sg_model* M, const sg_control* ctl, const Op& op64, cons
     if (!any) return SG_OK;
     // round 0 starts the FP32 PCG; later rounds continue its search direction
     // (all live columns enter a solve together, so they share the round structure)
-    cudaMemsetAsync(W.d32, 0, sizeof(float) * (size_t)n1 * KR, c->stream);
+    mask = 0;
+    for (int j = 0; j < k; ++j) mask |= (unsigned)(live[j] != 0) << j;
+    if (persist) {
+      pending = launch(true);
+      if (pending) continue;
+      persist = false;   // a cooperative launch of this size is not possible here
+    }
     int it[16] = {0}, fl[16] = {0}, used = 0;
-    (void)fl;
     double step[16] = {0};
-    int mask[16] = {0};
     int st = pcg_run<float>(c, KR, op32, W.b32, n1, W.d32, W.r32, dprecon32, k, live.data(), ctl->cg_maxiter, itol,
                             (round == 0 ? 1 : 3) | 4, it, fl, &used, step);
     if (st != SG_OK && st != SG_ERR_NOCONV) return st;
-    for (int j = 0; j < k; ++j) {
-      mask[j] = live[j];
-      if (live[j]) S.iters[j] += it[j];
-    }
-    cudaMemcpyAsync(W.colmask, mask, sizeof(int) * 16, cudaMemcpyHostToDevice, c->stream);
-    launch_axpy_correction(n1, KR, W.colmask, W.d32, W.x, W.b64.part, c->stream);
-    reduce_read(c, W.b64.part, vec_blocks(n1, KR), KR, 2, 3, red);
-    // the reference's step test on the last CG step: |alpha|*max|p| <= cg_tol*max|x|
     for (int j = 0; j < k; ++j)
-      if (live[j]) step_ok[j] = (red[2 * j + 1] > 0) && (step[j] <= ctl->cg_tol * red[2 * j + 1]);
+      if (live[j]) S.iters[j] += it[j];
+    launch_axpy_correction(n1, KR, mask, W.b32.G, W.d32, W.x, W.b64.part, c->stream);
+    reduce_read(c, W.b64.part, vec_blocks(n1, KR), KR, 2, 3, red);
+    judge_steps(red, step);
+    fresh = false;
+    ++round;
   }
   c->err = "iterative refinement did not converge";
   return SG_ERR_NOCONV;

@@ -2393,12 +2393,13 @@ void launch_residual_norms(int n1, int KR, const double* f, const double* kp, do
   SG_LAUNCH k_residual<<<vec_grid(n1, KR), RED_THREADS, 0, s>>>(n1, KR, f, kp, r64, r32, part);
 }
 
-// x += d for the columns in colmask; partials max|d|, max|x| per column.
-__global__ void __launch_bounds__(RED_THREADS) k_axpy_corr(int n1, int KR, const int* __restrict__ colmask,
+// x += d for the columns in mask once the solve is done; partials max|d|, max|x| per column.
+__global__ void __launch_bounds__(RED_THREADS) k_axpy_corr(int n1, int KR, unsigned mask,
+                                                           const PcgGlobal* __restrict__ G,
                                                            const float* __restrict__ d, double* __restrict__ x,
                                                            double* __restrict__ part) {
   unsigned long long a = 0, b = 0;
-  const bool on = colmask[threadIdx.x % KR] != 0;
+  const bool on = ((mask >> (threadIdx.x % KR)) & 1u) && G->all_done;
   const size_t n = (size_t)n1 * KR;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     double xi = x[i];
@@ -2413,9 +2414,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_axpy_corr(int n1, int KR, const
   block_pair_max(a, b, KR, part);
 }
 
-void launch_axpy_correction(int n1, int KR, const int* colmask, const float* d, double* x, double* part,
+void launch_axpy_correction(int n1, int KR, unsigned mask, const PcgGlobal* G, const float* d, double* x, double* part,
                             cudaStream_t s) {
-  SG_LAUNCH k_axpy_corr<<<vec_grid(n1, KR), RED_THREADS, 0, s>>>(n1, KR, colmask, d, x, part);
+  SG_LAUNCH k_axpy_corr<<<vec_grid(n1, KR), RED_THREADS, 0, s>>>(n1, KR, mask, G, d, x, part);
 }
 
 // dprecon(1:) = 1/dprecon(1:), dprecon(0) = 0 (src/slope.F90:199), plus an FP32 copy.
@@ -2459,8 +2460,10 @@ template void launch_gather_plain<float>(const GatherTopo&, int, const float*, f
 // entry t % (KR*nq) of blocks t/(KR*nq), ... (KR*nq <= 64 divides 256), eight
 // loads in flight; the entry's threads are then added by halves.
 __global__ void __launch_bounds__(256) k_final_reduce(const double* __restrict__ part, int nblk, int KR, int nq,
-                                                      int maxmask, double* __restrict__ out) {
+                                                      int maxmask, double* __restrict__ out,
+                                                      const double* __restrict__ part2) {
   __shared__ double s[256];
+  if (blockIdx.x) { part = part2; maxmask = ~0; out += KR * nq; }
   const int W = KR * nq, n = nblk * W;
   const bool mx = (maxmask >> (threadIdx.x % W % nq)) & 1;
   double v = 0.0;
@@ -2483,8 +2486,9 @@ __global__ void __launch_bounds__(256) k_final_reduce(const double* __restrict__
   if ((int)threadIdx.x < W) out[threadIdx.x] = v;
 }
 
-void launch_final_reduce(const double* part, int nblk, int KR, int nq, int maxmask, double* out, cudaStream_t s) {
-  SG_LAUNCH k_final_reduce<<<1, 256, 0, s>>>(part, nblk, KR, nq, maxmask, out);
+void launch_final_reduce(const double* part, int nblk, int KR, int nq, int maxmask, double* out, cudaStream_t s,
+                         const double* part2) {
+  SG_LAUNCH k_final_reduce<<<part2 ? 2 : 1, 256, 0, s>>>(part, nblk, KR, nq, maxmask, out, part2);
 }
 
 // Nodal displacement maxima of one column (src/slope.F90:400-415):

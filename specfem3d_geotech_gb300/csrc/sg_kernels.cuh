@@ -92,11 +92,26 @@ void launch_nodal_average(const int* ptr, const int* slot, int nnode, const doub
 bool fp32_matrix_free();
 // Persistent cooperative FP32 PCG chunk for small and medium meshes
 // (sg_pcg_persist.cu); false when it cannot run (the caller launches the
-// separate kernels).  A chunk whose bounded wait ran out sets G->err.
+// separate kernels).  A new solve (init) has u = 0 and r = f; keep continues the
+// last solve's direction.  The outcome goes to *out in pinned host memory, which
+// the caller sets to PERSIST_NONE before: it stays that when a bounded wait ran
+// out (G->err is set then).
+struct PersistStart {
+  int init, keep, maxiter, kcols;
+  unsigned active;   // columns that take part
+  double tol;        // residual reduction at which a column stops
+};
+enum { PERSIST_NONE = 0, PERSIST_MORE = 1, PERSIST_DONE = 2 };
+struct PersistOut {
+  int state, it;
+  int iters[16], failed[16];
+  double step[16];   // |alpha| max|p| of the last step
+};
 template <int KR>
-bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int* pos, const GatherTopo& T, float* u,
-                           float* r, float* z, float* p, float* kp, float* Y, const float* dp, ColState* cs,
-                           PcgGlobal* G, double* part, int chunk, cudaStream_t s);
+bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int* pos, const GatherTopo& T,
+                           const float* f, float* u, float* r, float* z, float* p, float* kp, float* Y,
+                           const float* dp, ColState* cs, PcgGlobal* G, double* part, const PersistStart& st,
+                           PersistOut* out, int chunk, cudaStream_t s);
 bool persist_enabled();                 // SG_PERSIST=0 turns the persistent chunk off
 int persist_max_elements(int KR);       // meshes below this use it
 // FP64 solve of one right-hand side as a persistent cooperative kernel
@@ -166,13 +181,16 @@ void launch_load_combine(int n1, int KR, const double* extload, const double* bo
 template <typename V>
 void launch_gather_plain(const GatherTopo& T, int KR, const V* Y, V* out, int accumulate, const int* colmask,
                          cudaStream_t s);
-void launch_final_reduce(const double* part, int nblk, int KR, int nq, int maxmask, double* out, cudaStream_t s);
+// part2 (or null): a second set of the same shape, all maxima, to out + KR * nq
+void launch_final_reduce(const double* part, int nblk, int KR, int nq, int maxmask, double* out, cudaStream_t s,
+                         const double* part2 = nullptr);
 void launch_disp_max(int nnode, const int* gdof, const double* x, int KR, int col, double* part, cudaStream_t s);
 void launch_div(size_t n, double* y, double a, cudaStream_t s);
 void launch_col_zero(int n1, int KR, int j, double* a, double* b, double* c, cudaStream_t s);
 void launch_residual_norms(int n1, int KR, const double* f, const double* kp, double* r64, float* r32,
                            double* part, cudaStream_t s);
-void launch_axpy_correction(int n1, int KR, const int* colmask, const float* d, double* x, double* part,
+// x += d for the columns in mask, unless G says that the solve for d is not done
+void launch_axpy_correction(int n1, int KR, unsigned mask, const PcgGlobal* G, const float* d, double* x, double* part,
                             cudaStream_t s);
 void launch_invert_diag(int n1, double* dprecon, float* dprecon32, cudaStream_t s);
 

@@ -26,7 +26,9 @@
 //
 // A dof row's u, r, p stay in the registers of the thread that owns it while
 // the mesh is small enough (R pieces of up to four columns a thread, R = 1 or
-// 2); beyond that (R = 0) they stream through L2.  The element maps and point
+// 2, for one or two columns also 4, for one 8); beyond that (R = 0) they stream
+// through L2 (5,880 elements and one column: 17.9 us an iteration streamed, 15.2
+// in registers).  The element maps and point
 // records of a block's elements stay in shared memory where they fit.
 //
 // Phase A gives a warp one element and up to four columns, lane = node: the
@@ -171,9 +173,11 @@ struct Args {
   float *u, *r, *z, *p, *kp, *Y;
   const float* dp;    // inverted diagonal
   ColState* cs;
-  PcgGlobal* G;
+  PcgGlobal* G;       // cntB counts the barrier's arrivals
   float2* part;       // block partials: phase B [KR][grid], phase C [2 KR][grid]
-  unsigned* count;    // barrier arrivals
+  const float* f;     // right-hand side of a new solve
+  PersistStart st;
+  PersistOut* out;    // pinned host memory
   int chunk;          // iterations to run
   int cached;         // elements whose maps and records a block keeps in shared memory
 };
@@ -321,15 +325,22 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
   __shared__ int c_live[KR], c_iters[KR], c_failed[KR];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   PcgGlobal* G = A.G;
-  if (G->all_done) return;
+  const int init = A.st.init, keep = A.st.keep, maxiter = A.st.maxiter, kcols = A.st.kcols;
+  if (!init && G->all_done) return;
   if (t < KR) {
     const ColState c = A.cs[t];
-    c_rz[t] = split(c.rz); c_alpha[t] = split(c.alpha); c_beta[t] = split(c.beta); c_rr[t] = split(c.rr);
-    c_goal[t] = split(c.tol * c.tol * c.rr0);   // |r|^2 at which the column stops
-    c_live[t] = c.active && !c.done; c_iters[t] = c.iters; c_failed[t] = c.failed;
+    c_rz[t] = split(c.rz);
+    c_live[t] = (A.st.active >> t) & 1u;
+    if (!init) {
+      c_alpha[t] = split(c.alpha); c_beta[t] = split(c.beta); c_rr[t] = split(c.rr);
+      c_goal[t] = split(c.tol * c.tol * c.rr0);   // |r|^2 at which the column stops
+      c_live[t] = c_live[t] && !c.done; c_iters[t] = c.iters; c_failed[t] = c.failed;
+    } else {
+      c_alpha[t] = c_beta[t] = c_rr[t] = c_goal[t] = make_float2(0.f, 0.f);
+      c_iters[t] = c_failed[t] = 0;
+    }
   }
-  int itn = G->it, alldone = 0;
-  const int maxiter = G->maxiter, kcols = G->kcols;
+  int itn = init ? 0 : G->it, alldone = 0;
   const int grid = gridDim.x, bid = blockIdx.x;
   unsigned arrivals = 0;
 
@@ -339,12 +350,12 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
     __syncthreads();
     bool good = true;
     if (t == 0) {
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(A.count) : "memory");
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&G->cntB) : "memory");
       arrivals += (unsigned)grid;
       unsigned n;
       int tries = 0;
       do {
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(A.count) : "memory");
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(&G->cntB) : "memory");
         if (++tries > POLL_TRIES) good = false;
       } while (n < arrivals && good);
       if (!good) atomicExch(&G->err, 1);
@@ -405,9 +416,16 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
       sb[m] = g < A.ngroups ? A.gptr[g + 1] : 0;
       dv[m] = A.dp[gd[m]];
       const size_t o = (size_t)gd[m] * KR + c0;
-      ru[m].load_cg(A.u + o);
-      rr[m].load_cg(A.r + o);
-      rp[m].load_cg(A.p + o);
+      rp[m].zero();
+      if (init) {
+        ru[m].zero();
+        rr[m].load_cg(A.f + o);
+        if (keep) rp[m].load_cg(A.p + o);
+      } else {
+        ru[m].load_cg(A.u + o);
+        rr[m].load_cg(A.r + o);
+        rp[m].load_cg(A.p + o);
+      }
     }
   }
   float* U = smem + (size_t)warp * (S::UF + S::FF);
@@ -455,6 +473,74 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
           for (int c = 0; c < VW; ++c) acc.v[c] = acc.v[c] + v[k].v[c];
     }
   };
+
+  // r.z and r.r of the thread's columns over the grid, then each column's step,
+  // identical in every block: the start of a solve, or stop test and beta
+  auto column_steps = [&](CompSum (&zz)[2 * VW], bool first) -> bool {
+    reduce_lanes(zz);
+    publish(std::integral_constant<int, 2 * KR>{}, std::false_type{}, partC);
+    if (!barrier()) return false;
+    for (int j = warp; j < KR; j += NWARP) {
+      const CompSum x = block_sum(partC + (size_t)j * grid), y = block_sum(partC + (size_t)(KR + j) * grid);
+      if (lane == 0 && c_live[j]) {
+        c_rr[j] = norm2(y.pair());
+        if (first) {
+          if (keep) c_beta[j] = div2(x.pair(), c_rz[j]);
+          c_rz[j] = x.pair();
+          c_goal[j] = split(A.st.tol * A.st.tol * value(y.pair()));
+        } else if ((c_rr[j].x - c_goal[j].x) + (c_rr[j].y - c_goal[j].y) <= 0.f) {
+          c_live[j] = 0; c_iters[j] = itn;
+        } else if (itn >= maxiter) {
+          c_live[j] = 0; c_failed[j] = 1; c_iters[j] = maxiter + 1;
+        } else {
+          c_beta[j] = div2(x.pair(), c_rz[j]);
+          c_rz[j] = x.pair();
+        }
+      }
+    }
+    __syncthreads();
+    return true;
+  };
+
+  // ---- a new solve: u = 0, r = f, z = D r, and p = 0 unless the last solve's
+  // direction is continued (beta = r.z / the last r.z) ----
+  if (init) {
+    CompSum zz[2 * VW];
+    if (bid == 0 && t < KR) { A.u[t] = 0.f; A.r[t] = 0.f; A.z[t] = 0.f; A.p[t] = 0.f; }   // constrained dofs
+    auto start = [&](size_t o, float D, const Vec<VW>& rv) {
+      Vec<VW> zv;
+#pragma unroll
+      for (int q = 0; q < VW; ++q) {
+        zv.v[q] = D * rv.v[q];
+        zz[q].add(rv.v[q], zv.v[q]);
+        zz[VW + q].add(rv.v[q], rv.v[q]);
+      }
+      zv.store(A.z + o);
+      if (!keep) {
+        Vec<VW> none;
+        none.zero();
+        none.store(A.p + o);
+      }
+    };
+    if constexpr (R > 0) {
+#pragma unroll
+      for (int m = 0; m < R; ++m)
+        if (gd[m]) start((size_t)gd[m] * KR + c0, dv[m], rr[m]);
+    } else {
+      for (int g = g0; g < A.ngroups; g += gstride) {
+        const int gq = __ldg(A.gdof + 3 * g + d);
+        if (!gq) continue;
+        const size_t o = (size_t)gq * KR + c0;
+        Vec<VW> rv, none;
+        none.zero();
+        rv.load_cg(A.f + o);
+        none.store(A.u + o);
+        rv.store(A.r + o);
+        start(o, __ldg(A.dp + gq), rv);
+      }
+    }
+    if (!column_steps(zz, true)) return;
+  }
 
   for (int k = 0; k < A.chunk; ++k) {
     // ---- A: element products ----
@@ -562,26 +648,8 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
         zv.store(A.z + o);
       }
     }
-    reduce_lanes(zz);
-    publish(std::integral_constant<int, 2 * KR>{}, std::false_type{}, partC);
-    if (!barrier()) return;
-    // stop test and beta, identical in every block
     ++itn;
-    for (int j = warp; j < KR; j += NWARP) {
-      const CompSum x = block_sum(partC + (size_t)j * grid), y = block_sum(partC + (size_t)(KR + j) * grid);
-      if (lane == 0 && c_live[j]) {
-        c_rr[j] = norm2(y.pair());
-        if ((c_rr[j].x - c_goal[j].x) + (c_rr[j].y - c_goal[j].y) <= 0.f) {
-          c_live[j] = 0; c_iters[j] = itn;
-        } else if (itn >= maxiter) {
-          c_live[j] = 0; c_failed[j] = 1; c_iters[j] = maxiter + 1;
-        } else {
-          c_beta[j] = div2(x.pair(), c_rz[j]);
-          c_rz[j] = x.pair();
-        }
-      }
-    }
-    __syncthreads();
+    if (!column_steps(zz, false)) return;
     alldone = !__syncthreads_or(t < kcols && c_live[t < KR ? t : 0]);
     if (alldone) break;
   }
@@ -624,14 +692,21 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
       ColState& c = A.cs[t];
       float m = 0.f;
       for (int b = 0; b < grid; ++b) m = fmaxf(m, __ldcg(partB + (size_t)t * grid + b).x);
+      c.active = (A.st.active >> t) & 1u;
       if (c.active) {
         c.rz = value(c_rz[t]); c.alpha = value(c_alpha[t]); c.beta = value(c_beta[t]); c.rr = value(c_rr[t]);
         c.maxp = m; c.done = !c_live[t]; c.iters = c_iters[t]; c.failed = c_failed[t];
+        if (init) { c.tol = 1.0; c.rr0 = value(c_goal[t]); }   // their product is the goal
+        A.out->iters[t] = c_iters[t];
+        A.out->failed[t] = c_failed[t];
+        A.out->step[t] = fabs(c.alpha) * (double)m;
       }
     }
     if (t == 0) {
       G->it = itn;
       G->all_done = alldone;
+      A.out->it = itn;
+      A.out->state = alldone ? PERSIST_DONE : PERSIST_MORE;
     }
   }
 }
@@ -675,13 +750,14 @@ static bool launch_persistent(const pp::Args& A, int grid, size_t smem, cudaStre
   return true;
 }
 
-// Runs up to `chunk` PCG iterations of the FP32 solve (residual test) as one
-// cooperative launch.  Returns false when the launch is not possible (the
-// caller then runs the separate kernels).
+// Up to `chunk` PCG iterations of the FP32 solve (residual test) as one
+// cooperative launch; st says whether a new solve begins.  Returns false when
+// the launch is not possible (the caller then runs the separate kernels).
 template <int KR>
-bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int* pos, const GatherTopo& T, float* u,
-                           float* r, float* z, float* p, float* kp, float* Y, const float* dp, ColState* cs,
-                           PcgGlobal* G, double* part, int chunk, cudaStream_t s) {
+bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int* pos, const GatherTopo& T,
+                           const float* f, float* u, float* r, float* z, float* p, float* kp, float* Y,
+                           const float* dp, ColState* cs, PcgGlobal* G, double* part, const PersistStart& st,
+                           PersistOut* out, int chunk, cudaStream_t s) {
   using S = pp::Shape<KR>;
   // one block per SM, fewer where that still gives every scheduler of the
   // SMs in use no more than one warp of phase A
@@ -691,28 +767,31 @@ bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int
   if (grid > pp::MAX_BLOCKS) grid = pp::MAX_BLOCKS;
   if (grid < 1) return false;
   const long per = (pieces + grid * pp::NT - 1) / (grid * pp::NT);   // pieces per thread
-  // the block partials (3 KR pairs per block) and, behind them, the barrier count
-  const size_t np = (size_t)grid * 3 * KR * sizeof(float2);
-  static_assert((size_t)pp::MAX_BLOCKS * 3 * KR * sizeof(float2) + 64 <= (size_t)NPART * 16 * 4 * sizeof(double),
-                "partials fit the buffer");
-  unsigned* count = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(part) + np);
-  cudaMemsetAsync(count, 0, sizeof(unsigned), s);
+  static_assert((size_t)pp::MAX_BLOCKS * 3 * KR * sizeof(float2) <= (size_t)NPART * 16 * 2 * sizeof(double),
+                "partials fit half the buffer");
+  if (st.init) cudaMemsetAsync(G, 0, sizeof(PcgGlobal), s);
+  else cudaMemsetAsync(&G->cntB, 0, sizeof(unsigned), s);
   // elements a block works on: its run of pairs touches at most this many
   const long runs = (warps + grid - 1) / grid;
   long cached = (runs + S::QPD - 1) / S::QPD + (S::QPD > 1 ? 1 : 0);
   if (cached > S::CACHE) cached = S::CACHE;
   const size_t smem = S::SMEM + (size_t)cached * S::EF * sizeof(float);
   const pp::Args A{rec, ge, nelmt, pos, T.d_ptr, T.d_dof, T.ngroups, u, r, z, p, kp, Y, dp, cs, G,
-                   reinterpret_cast<float2*>(part), count, chunk, (int)cached};
+                   reinterpret_cast<float2*>(part), f, st, out, chunk, (int)cached};
   if (per <= 1) return launch_persistent<KR, 1>(A, (int)grid, smem, s);
   if (per <= 2) return launch_persistent<KR, 2>(A, (int)grid, smem, s);
+  if constexpr (KR <= 2)
+    if (per <= 4) return launch_persistent<KR, 4>(A, (int)grid, smem, s);
+  if constexpr (KR == 1)
+    if (per <= 8) return launch_persistent<KR, 8>(A, (int)grid, smem, s);
   return launch_persistent<KR, 0>(A, (int)grid, smem, s);
 }
 
 #define SG_PP_INST(KR)                                                                                             \
-  template bool launch_pcg_persistent<KR>(const float*, const int*, int, const int*, const GatherTopo&, float*,    \
-                                          float*, float*, float*, float*, float*, const float*, ColState*,         \
-                                          PcgGlobal*, double*, int, cudaStream_t);
+  template bool launch_pcg_persistent<KR>(const float*, const int*, int, const int*, const GatherTopo&,            \
+                                          const float*, float*, float*, float*, float*, float*, float*,            \
+                                          const float*, ColState*, PcgGlobal*, double*, const PersistStart&,       \
+                                          PersistOut*, int, cudaStream_t);
 SG_PP_INST(1)
 SG_PP_INST(2)
 SG_PP_INST(4)
