@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(Shape<KR>::NT, 1) k_apply_mf_planes(
     const PcgGlobal* __restrict__ G, const int* __restrict__ pos) {
   using S = Shape<KR>;
   constexpr int PV = S::PV, QPD = KR / PV;
+  chain_wait();
   if (G && G->all_done) return;
   extern __shared__ __align__(16) float smem[];
   const int grp = threadIdx.x / 96, t = threadIdx.x - 96 * grp, kz = t >> 5, lane = t & 31;
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(Shape<KR>::NT, 1) k_apply_mf_planes(
   float* Fz = U + S::UF;
   float* R = Fz + S::UF;                       // two buffers of records
   int* X = reinterpret_cast<int*>(R + 2 * S::RF);   // two buffers of maps
-  const int ngroups = (nelmt + S::EPG - 1) / S::EPG, gstride = gridDim.x * S::NG;
+  const int ngroups = (nelmt + S::EPG - 1) / S::EPG;
   float beta[PV];
 #pragma unroll
   for (int k = 0; k < PV; ++k) beta[k] = COMBINE ? (float)cs[PV * (t % QPD) + k].beta : 0.f;   // 96 % QPD == 0
@@ -186,14 +187,16 @@ __global__ void __launch_bounds__(Shape<KR>::NT, 1) k_apply_mf_planes(
 
   int g = blockIdx.x * S::NG + grp;
   if (g >= ngroups) return;   // whole groups leave: their barriers are their own
+  int gstep = gridDim.x * S::NG;
+  if (pass_down(G, 0)) { g = ngroups - 1 - g; gstep = -gstep; }
   fetch(g, 0);
   cp_async_wait();
   group_sync(grp);
   ask(0);
   stage();
   for (int b = 0;; b ^= 1) {
-    const int gn = g + gstride;
-    const bool more = gn < ngroups;
+    const int gn = g + gstep;
+    const bool more = (unsigned)gn < (unsigned)ngroups;
     group_sync(grp);   // p of this group is staged; the other buffer's last readers are done
     if (more) fetch(gn, b ^ 1);
     const float* ue = U + (size_t)el * NEDOF * KR + j;
@@ -448,8 +451,8 @@ void launch_apply_mf(const float* rec, const int* ge, int nelmt, const float* po
     const int ng = (nelmt + S::EPG - 1) / S::EPG, nb = (ng + S::NG - 1) / S::NG;
     const int grid = nb < 152 ? nb : 152;
     if (grid < 1) return;
-    if (combine) mf::k_apply_mf_planes<KR, true><<<grid, S::NT, S::SMEM, s>>>(rec, ge, nelmt, pold, z, Y, cs, G, pos);
-    else mf::k_apply_mf_planes<KR, false><<<grid, S::NT, S::SMEM, s>>>(rec, ge, nelmt, pold, z, Y, cs, G, pos);
+    launch_chained(combine ? mf::k_apply_mf_planes<KR, true> : mf::k_apply_mf_planes<KR, false>, grid, S::NT, S::SMEM, s,
+                   rec, ge, nelmt, pold, z, Y, cs, G, pos);
   }
 }
 

@@ -1057,6 +1057,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_pcg_gather_flat(
     const int* __restrict__ ptr, const int* __restrict__ dof, int ng, const float* __restrict__ Y,
     float* __restrict__ kp, float* __restrict__ p, const float* __restrict__ z, int mode, ColState* __restrict__ cs,
     PcgGlobal* __restrict__ G, double* __restrict__ part) {
+  chain_wait();
   if (G->all_done) return;
   constexpr int VW = KR < 4 ? KR : 4;   // columns per piece
   constexpr int QPD = KR / VW;          // pieces per dof row
@@ -1073,11 +1074,12 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_pcg_gather_flat(
     beta[k] = (float)cs[c0 + k].beta;
   }
   const float* yq = Y + VW * q;
-  const int gstride = gridDim.x * (FG_THREADS / LPN);
+  int gstride = gridDim.x * (FG_THREADS / LPN);
   int g = blockIdx.x * (FG_THREADS / LPN) + threadIdx.x / LPN;
+  if (pass_down(G, 1)) { g = ng - 1 - g; gstride = -gstride; }
   int a = 0, b = 0, gd = 0;
-  if (g < ng) { a = ptr[g]; b = ptr[g + 1]; gd = dof[3 * g + d]; }
-  for (; g < ng; g += gstride) {
+  if ((unsigned)g < (unsigned)ng) { a = ptr[g]; b = ptr[g + 1]; gd = dof[3 * g + d]; }
+  for (; (unsigned)g < (unsigned)ng; g += gstride) {
     // the p and z rows do not depend on the sums: their loads go out with the
     // first slot loads
     Piece<VW> pv, zv, acc, v[4];
@@ -1093,7 +1095,7 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_pcg_gather_flat(
       if (a + k < b) v[k].load_once(yq + (size_t)(a + k) * 3 * KR);
     const int gn = g + gstride;
     int an = 0, bn = 0, gdn = 0;
-    if (gn < ng) { an = ptr[gn]; bn = ptr[gn + 1]; gdn = dof[3 * gn + d]; }
+    if ((unsigned)gn < (unsigned)ng) { an = ptr[gn]; bn = ptr[gn + 1]; gdn = dof[3 * gn + d]; }
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       if (a + k < b)
@@ -1401,8 +1403,8 @@ void pcg_gather(const GatherTopo& T, const V* Y, V* kp, V* p, const V* z, int mo
     if (g_gather_variant == 1) {
       // at most one block per SM; the grid depends only on the problem size
       constexpr int NPB = FG_THREADS / (3 * KR / (KR < 4 ? KR : 4));   // nodes per block and pass
-      SG_LAUNCH k_pcg_gather_flat<KR><<<red_grid(T.ngroups, NPB, F_BLOCKS), FG_THREADS, 0, s>>>(
-          T.d_ptr, T.d_dof, T.ngroups, Y, kp, p, z, mode, cs, G, part);
+      SG_LAUNCH launch_chained(k_pcg_gather_flat<KR>, red_grid(T.ngroups, NPB, F_BLOCKS), FG_THREADS, 0, s, T.d_ptr,
+                               T.d_dof, T.ngroups, Y, kp, p, z, mode, cs, G, part);
       return;
     }
   }
@@ -1627,6 +1629,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
     int n1, float* __restrict__ u, float* __restrict__ r, float* __restrict__ z, const float* __restrict__ p,
     const float* __restrict__ kp, const float* __restrict__ f, const float* __restrict__ dprecon, int init,
     ColState* __restrict__ cs, PcgGlobal* __restrict__ G, double* __restrict__ part) {
+  chain_wait();
   if (G->all_done) return;
   constexpr int QP = KR < 4 ? 1 : KR / 4;          // pieces per row (KR >= 4)
   constexpr int NC = KR < 4 ? KR : 4;              // columns a thread touches
@@ -1645,7 +1648,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
   float mp[4] = {0.f, 0.f, 0.f, 0.f};
   DotAcc<float> rza[4], rra[4];
   const size_t n = (size_t)n1 * KR, n4 = (n + 3) / 4;
-  const size_t stride = (size_t)gridDim.x * FU_THREADS;   // a multiple of QP
+  size_t stride = (size_t)gridDim.x * FU_THREADS;   // a multiple of QP
   size_t i = (size_t)blockIdx.x * FU_THREADS + threadIdx.x;
   // diagonal entries of piece o (KR < 4 spans several rows; the last piece may be cut)
   auto diag = [&](size_t o, float (&dv)[4]) {
@@ -1694,6 +1697,10 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
     }
   } else if (any) {
     constexpr int U = 4;
+    if (pass_down(G, 0)) {   // rows from the last one up, columns as they are; past the first the index wraps
+      i = n4 - QP + 2 * (threadIdx.x % QP) - i;
+      stride = 0 - stride;
+    }
     for (; i < n4; i += U * stride) {
       float pv[U][4], uv[U][4], rv[U][4], kv[U][4], dv[U][4];
 #pragma unroll
@@ -1778,12 +1785,12 @@ template <typename V, int KR>
 void pcg_update(int n1, V* u, V* r, V* z, const V* p, const V* kp, const V* f, const V* dprecon, int init,
                 ColState* cs, PcgGlobal* G, double* part, cudaStream_t s) {
   if constexpr (std::is_same<V, float>::value) {
-    SG_LAUNCH k_pcg_update_flat<KR><<<red_grid((size_t)n1 * KR, FU_THREADS * 4, F_BLOCKS), FU_THREADS, 0, s>>>(
+    SG_LAUNCH launch_chained(k_pcg_update_flat<KR>, red_grid((size_t)n1 * KR, FU_THREADS * 4, F_BLOCKS), FU_THREADS, 0,
+                             s, n1, u, r, z, p, kp, f, dprecon, init, cs, G, part);
+  } else {
+    SG_LAUNCH k_pcg_update<V, KR><<<red_grid((size_t)n1 * KR, VUPDATE, NPART), RED_THREADS, 0, s>>>(
         n1, u, r, z, p, kp, f, dprecon, init, cs, G, part);
-    return;
   }
-  SG_LAUNCH k_pcg_update<V, KR><<<red_grid((size_t)n1 * KR, VUPDATE, NPART), RED_THREADS, 0, s>>>(
-      n1, u, r, z, p, kp, f, dprecon, init, cs, G, part);
 }
 
 // ---------------------------------------------------------------------------

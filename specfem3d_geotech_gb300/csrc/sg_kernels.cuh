@@ -31,6 +31,38 @@ struct PcgGlobal {
   int err;        // set to 1 by a bounded wait of this solve's kernels that ran out
 };
 
+#ifdef __CUDACC__
+// The kernels of an FP32 iteration are launched with programmatic stream
+// serialization: a kernel's blocks take the SMs as the blocks of the one before
+// leave them and wait in chain_wait() until it is complete, instead of being
+// launched after that.  Every kernel of the chain waits before it touches
+// memory, so it also stands behind all earlier ones.  (62,000 elements, 8
+// trials: 301 -> 293 us per iteration.)
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Direction of a pass over the mesh in iteration G->it: each of an iteration's
+// three passes starts where the one before it ended, whose data L2 still holds.
+// (62,000 elements, 8 trials: 310 -> 301 us per iteration; 16,000 and 16: 188 -> 185.)
+__device__ __forceinline__ bool pass_down(const PcgGlobal* G, int phase) { return G && ((G->it + phase) & 1); }
+#endif
+
 // Factored material block for the stress update, per trial.
 struct MatF {
   double c11, c12, c44;  // compute_cmat(ym, nuf) entries (src/elastic.f90:13-42)
