@@ -13,8 +13,8 @@
 //   stress    K5, strain, Mohr-Coulomb yield, viscoplastic flow and body load
 //             (src/slope.F90:311-383, src/excavation.F90:546-616)
 //
-// All reductions use a fixed grid (NPART blocks) and fixed-order trees, so a
-// run is bitwise reproducible on the same device type.
+// Every reduction's grid depends only on the problem size and its tree is
+// fixed, so a run is bitwise reproducible on the same device type.
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
@@ -965,20 +965,23 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_gather(
 
 // Flat gather for FP32: thread = one piece (VW columns, up to 16 bytes) of one
 // dof row of one node.  Consecutive threads take the LPN pieces of a node's
-// slot row, so a warp's loads are coalesced runs of Y and no lane idles; 960
+// slot row, so a warp's loads are coalesced runs of Y and no lane idles; 384
 // threads per block keep the stride a multiple of LPN (3, 6 or 12), so a
 // thread's columns are fixed.  A node's pieces sum its slots in element order,
 // as the staged gather does: kp and p are bitwise equal to it.
-// What bounds it: HBM at large meshes, and below that the chain ptr -> slots
-// -> reduction tail.  So the next piece's slot range and dof number are
-// fetched one step ahead, and one block per SM (not four) leaves a quarter of
-// the partials for the last block, which reads them in one batch.  Gather and
-// update together at 16k elements and 16 columns: 145 us before, 94 now; at
-// 62k and 8 columns 189, 158 (event-timed).
+// What bounds it: the latency of HBM at large meshes (the bytes that 64,000
+// registers can have in flight), and below that the chain ptr -> slots ->
+// reduction tail.  So a node's slots and its p and z rows are asked for while
+// the node before is summed, and the slot ranges and dof numbers one node
+// earlier still; two blocks of 384 per SM drain independently and leave few
+// partials for the last block, which reads them in one batch.  us at 62,000
+// elements and 8 columns (16,000 and 16): staged 89 (66); 960 threads without
+// the read-ahead 80 (45); with it, one block of 768 76 (42), two of 384 73 (41).
+// Bulk copies of the slots into shared memory took 93, 32-byte pieces 101.
 int g_gather_variant = 1;   // 0 = staged gather for every case
 void set_gather_variant(int v) { g_gather_variant = v; }
-constexpr int FG_THREADS = 960;   // 30 warps at 64 registers: one block per SM
-constexpr int FU_THREADS = 512;   // update: 16 warps, four pieces a thread in flight
+constexpr int FG_THREADS = 384, FG_PER_SM = 2;   // gather: 24 warps at 80 registers
+constexpr int FU_THREADS = 512;                  // update: 16 warps, four pieces a thread in flight
 constexpr int F_BLOCKS = 152;
 
 // Last-block sum of part[nblk][NQ] for the FP32 kernels: thread t adds entry
@@ -1053,7 +1056,7 @@ struct Piece {
 };
 
 template <int KR>
-__global__ void __launch_bounds__(FG_THREADS, 1) k_pcg_gather_flat(
+__global__ void __launch_bounds__(FG_THREADS, FG_PER_SM) k_pcg_gather_flat(
     const int* __restrict__ ptr, const int* __restrict__ dof, int ng, const float* __restrict__ Y,
     float* __restrict__ kp, float* __restrict__ p, const float* __restrict__ z, int mode, ColState* __restrict__ cs,
     PcgGlobal* __restrict__ G, double* __restrict__ part) {
@@ -1077,50 +1080,62 @@ __global__ void __launch_bounds__(FG_THREADS, 1) k_pcg_gather_flat(
   int gstride = gridDim.x * (FG_THREADS / LPN);
   int g = blockIdx.x * (FG_THREADS / LPN) + threadIdx.x / LPN;
   if (pass_down(G, 1)) { g = ng - 1 - g; gstride = -gstride; }
-  int a = 0, b = 0, gd = 0;
-  if ((unsigned)g < (unsigned)ng) { a = ptr[g]; b = ptr[g + 1]; gd = dof[3 * g + d]; }
-  for (; (unsigned)g < (unsigned)ng; g += gstride) {
-    // the p and z rows do not depend on the sums: their loads go out with the
-    // first slot loads
-    Piece<VW> pv, zv, acc, v[4];
-    pv.zero(); zv.zero(); acc.zero();
-    float* pp = p + (size_t)gd * KR + c0;
-    if (mode != 0 && gd) {
-      pv.load(pp);
-      zv.load(z + (size_t)gd * KR + c0);
+  // a node's first four slots and its p and z rows, which do not depend on the
+  // sums, are asked for while the node before is summed
+  struct Node { int a, b, gd; Piece<VW> pv, zv, v[4]; };
+  auto maps = [&](int i, Node& n) {
+    n.a = n.b = n.gd = 0;
+    if ((unsigned)i < (unsigned)ng) { n.a = ptr[i]; n.b = ptr[i + 1]; n.gd = dof[3 * i + d]; }
+  };
+  auto ask = [&](Node& n) {
+    n.pv.zero(); n.zv.zero();
+    if (mode != 0 && n.gd) {
+      n.pv.load(p + (size_t)n.gd * KR + c0);
+      n.zv.load(z + (size_t)n.gd * KR + c0);
     }
-    // up to four slots in flight at once, summed in slot order
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      if (a + k < b) v[k].load_once(yq + (size_t)(a + k) * 3 * KR);
-    const int gn = g + gstride;
-    int an = 0, bn = 0, gdn = 0;
-    if ((unsigned)gn < (unsigned)ng) { an = ptr[gn]; bn = ptr[gn + 1]; gdn = dof[3 * gn + d]; }
+      if (n.a + k < n.b) n.v[k].load_once(yq + (size_t)(n.a + k) * 3 * KR);
+  };
+  auto sum = [&](Node& n) {   // in slot order
+    Piece<VW> acc;
+    acc.zero();
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      if (a + k < b)
+      if (n.a + k < n.b)
 #pragma unroll
-        for (int c = 0; c < VW; ++c) acc.v[c] = acc.v[c] + v[k].v[c];
-    for (int s0 = a + 4; s0 < b; s0 += 4) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (s0 + k < b) v[k].load_once(yq + (size_t)(s0 + k) * 3 * KR);
+        for (int c = 0; c < VW; ++c) acc.v[c] = acc.v[c] + n.v[k].v[c];
+    for (int s0 = n.a + 4; s0 < n.b; s0 += 4) {
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        if (s0 + k < b)
+        if (s0 + k < n.b) n.v[k].load_once(yq + (size_t)(s0 + k) * 3 * KR);
 #pragma unroll
-          for (int c = 0; c < VW; ++c) acc.v[c] = acc.v[c] + v[k].v[c];
+      for (int k = 0; k < 4; ++k)
+        if (s0 + k < n.b)
+#pragma unroll
+          for (int c = 0; c < VW; ++c) acc.v[c] = acc.v[c] + n.v[k].v[c];
     }
-    if (gd) {
+    if (n.gd) {
       if (mode != 0) {
 #pragma unroll
         for (int c = 0; c < VW; ++c)
-          if (live[c]) { pv.v[c] = pdir(beta[c], pv.v[c], zv.v[c]); dacc[c].add(pv.v[c], acc.v[c]); }
-        pv.store(pp);
+          if (live[c]) { n.pv.v[c] = pdir(beta[c], n.pv.v[c], n.zv.v[c]); dacc[c].add(n.pv.v[c], acc.v[c]); }
+        n.pv.store(p + (size_t)n.gd * KR + c0);
       }
-      acc.store(kp + (size_t)gd * KR + c0);
+      acc.store(kp + (size_t)n.gd * KR + c0);
     }
-    a = an; b = bn; gd = gdn;
+  };
+  Node A, B;
+  maps(g, A);
+  ask(A);
+  maps(g + gstride, B);
+  for (; (unsigned)g < (unsigned)ng; g += 2 * gstride) {
+    ask(B);
+    sum(A);
+    maps(g + 2 * gstride, A);
+    ask(A);
+    sum(B);
+    maps(g + 3 * gstride, B);
   }
   if (mode == 0) return;
   __shared__ double sred[FG_THREADS / 32][KR];
@@ -1401,9 +1416,9 @@ void pcg_gather(const GatherTopo& T, const V* Y, V* kp, V* p, const V* z, int mo
                 double* part, cudaStream_t s) {
   if constexpr (std::is_same<V, float>::value) {
     if (g_gather_variant == 1) {
-      // at most one block per SM; the grid depends only on the problem size
+      // the grid depends only on the problem size
       constexpr int NPB = FG_THREADS / (3 * KR / (KR < 4 ? KR : 4));   // nodes per block and pass
-      SG_LAUNCH launch_chained(k_pcg_gather_flat<KR>, red_grid(T.ngroups, NPB, F_BLOCKS), FG_THREADS, 0, s, T.d_ptr,
+      SG_LAUNCH launch_chained(k_pcg_gather_flat<KR>, red_grid(T.ngroups, NPB, FG_PER_SM * F_BLOCKS), FG_THREADS, 0, s, T.d_ptr,
                                T.d_dof, T.ngroups, Y, kp, p, z, mode, cs, G, part);
       return;
     }
