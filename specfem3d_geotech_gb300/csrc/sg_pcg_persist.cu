@@ -716,12 +716,16 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
 // Largest mesh that takes the persistent chunk: where a phase has more work
 // than 15 warps per SM hide, separate launches with their own register budgets
 // win.  us per iteration of a whole trial, persistent against separate kernels:
-//   elements x columns   576 x 1   576 x 8   3289 x 8   5880 x 16   16000 x 8   12000 x 16   16000 x 1
-//   persistent              11.0      18.8         39         108         133          212          32
-//   separate                36.0      48.8         69         118         134          187          61
-// (with flags polled by every block and FP64 sums it was 21, 31 and 50 us for
-// the first three).
-int persist_max_elements(int KR) { return 130000 / KR; }
+//   elements   1 column       2 columns      4 columns      8 columns      16 columns
+//    1,071    9.8 /  34.8   11.3 /  36.1   14.3 /  43.1   20.0 /  45.1    34.8 /  56.0
+//    3,289   12.9 /  42.0   15.4 /  48.0   21.8 /  48.9   39.2 /  58.5    70.2 /  79.2
+//    5,488   15.0 /  50.1   18.8 /  53.1   28.7 /  55.8   53.6 /  68.8   105.2 / 101.3
+//    9,600   19.8 /  60.0   26.4 /  59.8   44.3 /  61.4   82.9 /  85.4
+//   12,000   22.6 /  63.9   33.1 /  64.0   52.7 /  68.0   99.6 /  93.1
+//   25,000   44.2 /  80.1   57.9 /  87.7   99.6 /  96.4
+//   40,000   66.7 / 100.7   96.6 / 114.5
+//   64,800  126.3 / 132.3  183.3 / 158.0
+int persist_max_elements(int KR) { return KR == 1 ? 65000 : 85000 / KR; }
 
 bool persist_enabled() {
   static const bool on = !(getenv("SG_PERSIST") && atoi(getenv("SG_PERSIST")) == 0);
