@@ -206,7 +206,6 @@ struct Op {
   int nelmt = 0;
   const GatherTopo* T = nullptr;
   const double* rows = nullptr;   // dense: the matrices packed by rows, where their pattern allows it
-  const double* rec = nullptr;    // sparse FP64: the point records, where there is room for them
 };
 
 template <typename V>
@@ -325,8 +324,8 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
     if constexpr (std::is_same<V, double>::value && KR == 1)
       if (persist) {
         ev = C->prof_begin();
-        done_chunk = launch_pcg_persistent64(op.dense != 0, op.dense ? op.rows : (const double*)op.K, op.rec, op.ge,
-                                             op.nelmt,                                             op.T->d_pos, C->d_nbr, *op.T, n1, u, B.r, B.z, B.p, B.kp, B.Y, dp, B.cs,
+        done_chunk = launch_pcg_persistent64(op.dense != 0, op.dense ? op.rows : (const double*)op.K, op.ge, op.nelmt,
+                                             op.T->d_pos, C->d_nbr, *op.T, n1, u, B.r, B.z, B.p, B.kp, B.Y, dp, B.cs,
                                              B.G, B.part, persist_chunk, s);
         C->prof_end(ev, 0);
       }
@@ -676,7 +675,6 @@ struct sg_model {
   GatherTopo T;
   double* d_K64 = nullptr;
   float* d_K32 = nullptr;
-  double* d_rec64 = nullptr; // the same in FP64 (FP64 models above fp64_stored_max, where there is room)
   float* d_rec32 = nullptr;  // matrix-free FP32 operator: per GLL point J^-1 and w detJ C (MF_REC floats)
   double *d_diag = nullptr, *d_dprecon = nullptr, *d_extload = nullptr;
   float* d_dprecon32 = nullptr;
@@ -750,8 +748,7 @@ static bool model_stiffness(sg_model* M, const int* d_elist, int nel, const doub
   launch_stiffness(M->d_geo, M->d_matid, d_elist, nel, M->d_ym, d_nuv, M->d_gam, M->d_K64, M->d_K32, Ydiag,
                    gravity ? Ygrav : nullptr, c->d_border, T.d_pos, s, pseudoeq ? M->H.iseqload : 0, M->H.eqkx,
                    M->H.eqky, M->H.eqkz);
-  launch_mf_record<float>(M->d_geo, M->d_matid, d_elist, nel, M->d_ym, d_nuv, M->d_rec32, s);
-  launch_mf_record<double>(M->d_geo, M->d_matid, d_elist, nel, M->d_ym, d_nuv, M->d_rec64, s);
+  launch_mf_record(M->d_geo, M->d_matid, d_elist, nel, M->d_ym, d_nuv, M->d_rec32, s);
   c->prof_end(ev, 5);
   cudaMemsetAsync(M->d_diag, 0, sizeof(double) * n1, s);
   launch_gather_plain<double>(T, 1, Ydiag, M->d_diag, 0, nullptr, s);
@@ -800,18 +797,6 @@ static sg_model* model_build(sg_ctx* c, HostMesh&& H, int nnode8, const double* 
     if (!fp32_matrix_free()) M->d_K32 = c->alloc<float>((size_t)ne * KS_STRIDE);
     M->d_rec32 = c->alloc<float>((size_t)ne * NGLL * MF_REC);
     M->d_dprecon32 = c->alloc<float>(n1);
-  }
-  if (precision == SG_PREC_FP64 && ne > fp64_stored_max()) {
-    // no more than a quarter of what the budget has left after the rest of the
-    // model and the widest batch's workspace: the solve also runs without
-    const size_t room = sizeof(double) * (size_t)ne * NGLL * MF_REC;
-    const size_t column = sizeof(double) * ((size_t)n1 * 8 + (size_t)ne * (NEDOF + 2 * NGLL * NST));
-    const size_t later = 16 * column + sizeof(double) * ((size_t)n1 * 6 + (size_t)ne * 2 * NEDOF);
-    if (c->used + later <= c->budget && room <= (c->budget - c->used - later) / 4) {
-      const std::string before = c->err;
-      M->d_rec64 = c->alloc<double>((size_t)ne * NGLL * MF_REC);
-      if (!M->d_rec64) c->err = before;
-    }
   }
   M->d_diag = c->alloc<double>(n1);
   M->d_dprecon = c->alloc<double>(n1);
@@ -1001,7 +986,7 @@ void sg_model_free(sg_model* M) {
   free_topo(c, M->T);
   for (void* p : {(void*)M->d_coord, (void*)M->d_gnum, (void*)M->d_matid, (void*)M->d_ge, (void*)M->d_gdof,
                   (void*)M->d_ym, (void*)M->d_nu, (void*)M->d_gam, (void*)M->d_geo, (void*)M->d_K64, (void*)M->d_K32,
-                  (void*)M->d_rec32, (void*)M->d_rec64, (void*)M->d_diag, (void*)M->d_dprecon, (void*)M->d_extload, (void*)M->d_dprecon32,
+                  (void*)M->d_rec32, (void*)M->d_diag, (void*)M->d_dprecon, (void*)M->d_extload, (void*)M->d_dprecon32,
                   (void*)M->d_Yscratch, (void*)M->d_fpart, (void*)M->d_wp})
     c->release(p);
   delete M;
@@ -1391,7 +1376,7 @@ static int batch_iteration(sg_model* M) {
   for (int t = 0; t < k; ++t) { live[t] = B.slot[t].live; any = any || live[t]; }
   if (!any) return SG_OK;
   Op op64, op32;
-  op64.K = M->d_K64; op64.rec = M->d_rec64; op64.ge = M->d_ge; op64.nelmt = ne; op64.T = &M->T;
+  op64.K = M->d_K64; op64.ge = M->d_ge; op64.nelmt = ne; op64.T = &M->T;
   op32 = fp32_op(M, op64);
   launch_load_combine(n1, KR, M->d_extload, W.bodyload, W.load, s);
   SolveStats St;
@@ -1874,7 +1859,7 @@ extern "C" int sg_excavation(sg_model* M, const sg_control* ctl, int s0_type, do
       cudaMemsetAsync(M->W.x, 0, sizeof(double) * n1, s);
       cudaMemcpyAsync(M->W.load, M->d_extload, sizeof(double) * n1, cudaMemcpyDeviceToDevice, s);
       Op op64, op32;
-      op64.K = M->d_K64; op64.rec = M->d_rec64; op64.ge = M->d_ge; op64.nelmt = ne; op64.T = &M->T;
+      op64.K = M->d_K64; op64.ge = M->d_ge; op64.nelmt = ne; op64.T = &M->T;
       op32 = fp32_op(M, op64);
       SolveStats S;
       std::vector<int> act(1, 1);
@@ -1970,7 +1955,7 @@ extern "C" int sg_excavation(sg_model* M, const sg_control* ctl, int s0_type, do
         model_stiffness(M, d_eint, nint, d_nuf, Ti, d_geint, n1, false);
         c->release(d_nuf);
         Op op64, op32;
-        op64.K = M->d_K64; op64.rec = M->d_rec64; op64.ge = d_geint; op64.nelmt = nint; op64.T = &Ti;
+        op64.K = M->d_K64; op64.ge = d_geint; op64.nelmt = nint; op64.T = &Ti;
         op32 = fp32_op(M, op64);
         int cg_tot = 0, nl_tot = 0, nl_iter = 0;
         double fmax = 0.0, red[64];

@@ -405,11 +405,10 @@ __global__ void __launch_bounds__(LShape<KR>::NT, 2) k_apply_mf_lines(
 
 // Record of GLL point q of operator element le (element elist[le]):
 // J^-1 (row-major, as cached by the geometry kernel) and the compute_cmat
-// constants times w_q detJ_q, rounded to V.
-template <typename V>
+// constants times w_q detJ_q, rounded to FP32.
 __global__ void k_mf_record(const double* __restrict__ geo, const int* __restrict__ mat_id,
                             const int* __restrict__ elist, int nel, const double* __restrict__ ym,
-                            const double* __restrict__ nu, V* __restrict__ rec) {
+                            const double* __restrict__ nu, float* __restrict__ rec) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= nel * NGLL) return;
   const int le = tid / NGLL, q = tid - le * NGLL;
@@ -421,12 +420,12 @@ __global__ void k_mf_record(const double* __restrict__ geo, const int* __restric
   const double w1[3] = {1.0 / 3.0, 4.0 / 3.0, 1.0 / 3.0};
   const double* g = geo + ((size_t)e * NGLL + q) * GEO_STRIDE;
   const double wd = w1[q % 3] * w1[(q / 3) % 3] * w1[q / 9] * g[9];
-  V* r = rec + ((size_t)le * NGLL + q) * MF_REC;
+  float* r = rec + ((size_t)le * NGLL + q) * MF_REC;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) r[i] = (V)g[i];
-  r[9] = (V)(wd * onemv * Ef);
-  r[10] = (V)(wd * v * Ef);
-  r[11] = (V)(wd * 0.5 * onem2v * Ef);
+  for (int i = 0; i < 9; ++i) r[i] = (float)g[i];
+  r[9] = (float)(wd * onemv * Ef);
+  r[10] = (float)(wd * v * Ef);
+  r[11] = (float)(wd * 0.5 * onem2v * Ef);
 }
 
 }  // namespace mf
@@ -456,17 +455,12 @@ void launch_apply_mf(const float* rec, const int* ge, int nelmt, const float* po
   }
 }
 
-template <typename V>
 void launch_mf_record(const double* geo, const int* mat_id, const int* elist, int nel, const double* ym,
-                      const double* nu, V* rec, cudaStream_t s) {
+                      const double* nu, float* rec, cudaStream_t s) {
   if (nel <= 0 || !rec) return;
   const int n = nel * NGLL;
-  mf::k_mf_record<V><<<(n + 255) / 256, 256, 0, s>>>(geo, mat_id, elist, nel, ym, nu, rec);
+  mf::k_mf_record<<<(n + 255) / 256, 256, 0, s>>>(geo, mat_id, elist, nel, ym, nu, rec);
 }
-template void launch_mf_record<float>(const double*, const int*, const int*, int, const double*, const double*, float*,
-                                      cudaStream_t);
-template void launch_mf_record<double>(const double*, const int*, const int*, int, const double*, const double*,
-                                       double*, cudaStream_t);
 
 template void launch_apply_mf<1>(const float*, const int*, int, const float*, const float*, int, float*,
                                  const ColState*, const PcgGlobal*, const int*, cudaStream_t);

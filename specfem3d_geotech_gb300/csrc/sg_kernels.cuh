@@ -116,10 +116,9 @@ bool apply_uses_lanes(int dense, int KR);  // the FP32 apply of this operator is
 template <int KR>
 void launch_apply_mf(const float* rec, const int* ge, int nelmt, const float* pold, const float* z, int combine,
                      float* Y, const ColState* cs, const PcgGlobal* G, const int* pos, cudaStream_t s);
-template <typename V>
 void launch_mf_record(const double* geo, const int* mat_id, const int* elist, int nel, const double* ym,
-                      const double* nu, V* rec, cudaStream_t s);
-constexpr int MF_REC = 12;        // values per GLL point of the matrix-free record
+                      const double* nu, float* rec, cudaStream_t s);
+constexpr int MF_REC = 12;        // floats per GLL point of the matrix-free record
 void launch_nodal_average(const int* ptr, const int* slot, int nnode, const double* stress, double* out,
                           cudaStream_t s);  // sg_output.cu
 bool fp32_matrix_free();
@@ -154,8 +153,7 @@ int persist_max_elements(int KR);       // meshes below this use it
 constexpr int ROW_STRIDE = 4618;   // doubles per packed element: 57 x 81, padded to 16 bytes
 constexpr int VGATHER = RED_THREADS * 2, VUPDATE = RED_THREADS * 4;   // items per block of the FP64 gather and update
 void launch_pack_rows(const double* K, int nelmt, const int* d_nbr, double* out, int* other, cudaStream_t s);
-int fp64_stored_max();   // meshes above this use the point records rec (may be null)
-bool launch_pcg_persistent64(bool rows, const double* K, const double* rec, const int* ge, int nelmt, const int* pos, const int* d_nbr,
+bool launch_pcg_persistent64(bool rows, const double* K, const int* ge, int nelmt, const int* pos, const int* d_nbr,
                              const GatherTopo& T, int n1, double* u, double* r, double* z, double* p, double* kp,
                              double* Y, const double* dp, ColState* cs, PcgGlobal* G, double* part, int chunk,
                              cudaStream_t s);

@@ -1,6 +1,6 @@
 // sg_pcg_persist64.cu -- the FP64 PCG iterations (one right-hand side) as one
-// persistent cooperative kernel, for the model's operator (stored sparse
-// matrices, or point records) and for the drop-in's dense matrices.
+// persistent cooperative kernel, for the model's stored sparse matrices and
+// for the drop-in's dense ones.
 //
 // What bounds it: the FP64 unit takes a warp instruction in some 19 cycles, so
 // the element products (171 fused multiply-adds a lane with lane = node and 27
@@ -16,10 +16,8 @@
 //     per call (k_pack_rows) and packed; matrices that do not have it take the
 //     dense kernel;
 //   * a block's matrices stay in shared memory for the whole launch while they
-//     fit.  Beyond that the model's elements are applied from point records
-//     (point_products), and the drop-in's matrices, like the model's where the
-//     records found no room, stream through two buffers filled by bulk copies,
-//     the next iteration's first group on its way during the vector phases;
+//     fit, else they stream through two buffers filled by bulk copies, the
+//     next iteration's first group on its way during the vector phases;
 //   * the vector phases hand out warps, not blocks: the reference order of the
 //     dots groups 32 threads first, so each such warp may run on any SM, and
 //     a small mesh's few blocks of them do not queue on few FP64 units;
@@ -32,11 +30,11 @@
 // k_pcg_gather and k_pcg_update: products in column order (an exact zero adds
 // nothing), slots in element order, and dots over the same virtual grid of
 // 256-thread blocks with the same trees, so a solve is bitwise the one of the
-// separate kernels.  Only the point records round differently.
+// separate kernels.
 //
 // us per iteration, separate kernels (with short tails) -> this: 300 elements
-// dense 43 -> 16, sparse 37 -> 16; 12,000 elements sparse 256 -> 158 from stored
-// matrices, 106 from point records, of which the products take 119 and 76.  Code that one
+// dense 43 -> 16, sparse 37 -> 16; 12,000 elements sparse 256 -> 158, of which the
+// products take 119 (19 cycles for each FP64 warp instruction).  Code that one
 // warp runs once per iteration is kept short: unrolled twofold over nodes, the
 // gather took 10 us instead of 4.
 //
@@ -58,18 +56,13 @@ constexpr int POLL_TRIES = 1 << 20;
 constexpr int VT = RED_THREADS;          // threads of a virtual block
 constexpr unsigned FULL = 0xffffffffu;
 
-enum { SPARSE = 0, ROWS57 = 1, POINTS = 2 };   // stored sparse, packed rows, matrix-free point records
-
-template <int FORM>
+template <bool ROWS>
 struct Lay {
-  static constexpr bool ROWS = FORM == ROWS57;
   static constexpr int STRIDE = ROWS ? ROW_STRIDE : KS_STRIDE;        // doubles per element
   static constexpr int GE = ROWS ? 2 : 5;                             // elements per streamed group
   static constexpr int RES = ROWS ? 5 : 10;                           // elements that stay in shared memory
   static constexpr int NP = RES > 2 * GE ? RES : 2 * GE;              // direction slots
-  static constexpr int PGE = 9;                                       // matrix-free: elements per half block and pass
-  static constexpr size_t SMEM = FORM == POINTS ? (size_t)2 * PGE * NGLL * 12 * sizeof(double)
-                                                : (size_t)NP * (STRIDE + NEDOF) * sizeof(double);
+  static constexpr size_t SMEM = (size_t)NP * (STRIDE + NEDOF) * sizeof(double);
   static_assert(RES <= NP && 2 * GE <= NP && GE * NEDOF <= NT, "buffers");
   static_assert((STRIDE * sizeof(double)) % 16 == 0, "bulk copies");
 };
@@ -131,26 +124,6 @@ __device__ __forceinline__ double chain(const double* x, int n) {
   for (; i < n; ++i) s += x[i];
   return s;
 }
-// part[0..n) by a tree; the sum is thread 0's
-__device__ __forceinline__ double tree_sum(const double* part, int n, double* sm, int t, int lane, int warp) {
-  double v = 0.0;
-  for (int i0 = t; i0 < n; i0 += 8 * NT) {
-    double x[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = i0 + k * NT < n ? __ldcg(part + i0 + k * NT) : 0.0;
-    v += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
-  }
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-  if (lane == 0) sm[warp] = v;
-  __syncthreads();
-  if (warp == 0) {
-    v = lane < NWARP ? sm[lane] : 0.0;
-#pragma unroll
-    for (int o = 8; o >= 1; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-  }
-  return v;
-}
 // a block's sum from its eight warps' partials
 __device__ __forceinline__ double block_partial(const double* part, int vb) {
   const double2* w = reinterpret_cast<const double2*>(part + (size_t)vb * (VT / 32));
@@ -165,10 +138,10 @@ __device__ __forceinline__ double block_partial(const double* part, int vb) {
 
 // Rows [r0, r1) of the elements from efirst on, whose matrices start at kb and
 // directions at ps.
-template <int FORM>
+template <bool ROWS>
 __device__ __forceinline__ void row_products(const Args& A, const double* kb, const double* ps, int efirst, int r0,
                                              int r1, const int* nbr, int warp, int lane) {
-  using L = Lay<FORM>;
+  using L = Lay<ROWS>;
   for (int row = r0 + warp * 32 + lane; row < r1; row += NT) {
     const int el = row / NEDOF, rr = row - el * NEDOF, n = rr / 3, cc = rr - 3 * n;
     const double* k = kb + (size_t)el * L::STRIDE;
@@ -178,7 +151,7 @@ __device__ __forceinline__ void row_products(const Args& A, const double* kb, co
 #pragma unroll
     for (int s = 0; s < KS_NBR; ++s) {
       const int pk = tb[s], m = pk & 31;
-      if constexpr (L::ROWS) {
+      if constexpr (ROWS) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) y = fma(k[(3 * s + d) * NEDOF + rr], pe[3 * m + d], y);
       } else {
@@ -195,107 +168,9 @@ __device__ __forceinline__ void row_products(const Args& A, const double* kb, co
   }
 }
 
-__device__ __forceinline__ double dcoef(int i, int t) {   // D[i][t] of the GLL points -1, 0, 1
-  return i == 0 ? (t == 0 ? -1.5 : t == 1 ? 2.0 : -0.5)
-                : i == 1 ? (t == 0 ? -0.5 : t == 1 ? 0.0 : 0.5) : (t == 0 ? 0.5 : t == 1 ? -2.0 : 1.5);
-}
-
-// Matrix-free products of `nel` elements from e0 on (A.K: 12 values per point,
-// J^-1 and w detJ C): a half block takes nine elements at a time, a thread per
-// point, 243 of 256 at work.  The FP64 unit bounds this as it does the stored
-// product, with 123 operations a point, 1,750 cycles of an SM an element,
-// instead of 2,742: 12,000 elements take 156,000 cycles (79 elements a block,
-// the last pass of 18 partly filled), stored 238,000.  The operator's error is
-// smaller as well: against extended precision on distorted elements 1.3e-15 in
-// the median and 9e-15 at most, from stored FP64 matrices 7.7e-15 and 5.6e-14.
-__device__ __forceinline__ void point_products(const Args& A, double* sm, int e0, int nel, double beta) {
-  using L = Lay<POINTS>;
-  const int h = threadIdx.x / 256, t = threadIdx.x % 256, el = t / NGLL, a = t - el * NGLL;
-  const bool act = el < L::PGE;
-  double* U = sm + (size_t)h * L::PGE * NGLL * 12 + (size_t)(act ? el : 0) * NEDOF;
-  double* F = sm + (size_t)h * L::PGE * NGLL * 12 + (size_t)L::PGE * NEDOF + (size_t)(act ? el : 0) * NGLL * 9;
-  const int ic[3] = {a % 3, (a / 3) % 3, a / 9};
-  constexpr int st[3] = {1, 3, 9};
-  int gd[3];
-  double pv[3], zv[3];
-  auto maps = [&](int i) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) gd[c] = act && i < nel ? __ldg(A.ge + (size_t)(e0 + i) * NEDOF + 3 * a + c) : 0;
-  };
-  auto ask = [&]() {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) { pv[c] = __ldcg(A.p + gd[c]); zv[c] = __ldcg(A.z + gd[c]); }
-  };
-  maps(h * L::PGE + el);
-  ask();
-#pragma unroll 1
-  for (int b = h * L::PGE; b < nel; b += 2 * L::PGE) {
-    const int i = b + el;
-    const bool valid = act && i < nel;
-    double rec[12];
-    if (valid) {
-      const double2* R = reinterpret_cast<const double2*>(A.K + ((size_t)(e0 + i) * NGLL + a) * 12);
-#pragma unroll
-      for (int q = 0; q < 6; ++q) { const double2 x = __ldg(R + q); rec[2 * q] = x.x; rec[2 * q + 1] = x.y; }
-    }
-    if (act) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) U[3 * a + c] = fma(beta, pv[c], zv[c]);
-    }
-    maps(i + 2 * L::PGE);
-    asm volatile("bar.sync %0, 256;" ::"r"(1 + h) : "memory");
-    if (valid) {
-      double gr[3][3];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        const double* u = U + 3 * (a - ic[r] * st[r]);
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          gr[c][r] = fma(dcoef(ic[r], 2), u[6 * st[r] + c], fma(dcoef(ic[r], 1), u[3 * st[r] + c], dcoef(ic[r], 0) * u[c]));
-      }
-      double gp[3][3], T[3][3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-          gp[c][d] = fma(rec[3 * d], gr[c][0], fma(rec[3 * d + 1], gr[c][1], rec[3 * d + 2] * gr[c][2]));
-      T[0][0] = fma(rec[9], gp[0][0], rec[10] * (gp[1][1] + gp[2][2]));
-      T[1][1] = fma(rec[9], gp[1][1], rec[10] * (gp[0][0] + gp[2][2]));
-      T[2][2] = fma(rec[9], gp[2][2], rec[10] * (gp[0][0] + gp[1][1]));
-      T[0][1] = T[1][0] = rec[11] * (gp[0][1] + gp[1][0]);
-      T[1][2] = T[2][1] = rec[11] * (gp[1][2] + gp[2][1]);
-      T[0][2] = T[2][0] = rec[11] * (gp[0][2] + gp[2][0]);
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-          F[9 * a + 3 * r + c] = fma(rec[r], T[c][0], fma(rec[3 + r], T[c][1], rec[6 + r] * T[c][2]));
-    }
-    ask();
-    asm volatile("bar.sync %0, 256;" ::"r"(1 + h) : "memory");
-    if (valid) {
-      double y[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        const double* f = F + 9 * (a - ic[r] * st[r]) + 3 * r;
-#pragma unroll
-        for (int tt = 0; tt < 3; ++tt)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) y[c] = fma(dcoef(tt, ic[r]), f[9 * tt * st[r] + c], y[c]);
-      }
-      const int q = __ldg(A.pos + (size_t)(e0 + i) * NGLL + a);
-      if (q >= 0) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) A.Y[(size_t)q * 3 + c] = y[c];
-      }
-    }
-  }
-}
-
-template <int FORM>
+template <bool ROWS>
 __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
-  using L = Lay<FORM>;
-  constexpr bool MF = FORM == POINTS;
+  using L = Lay<ROWS>;
   extern __shared__ __align__(128) double dsm[];
   double* kb = dsm;                                   // matrices: resident, or two groups
   double* ps = dsm + (size_t)L::NP * L::STRIDE;       // directions of the same elements
@@ -326,7 +201,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
   // the block's rows: whole warps of 32 while the matrices they touch stay in
   // shared memory, else whole elements
   const int rows = A.nelmt * NEDOF, nchunk = (rows + 31) / 32, rper = (nchunk + grid - 1) / grid * 32;
-  const bool resident = !MF && (rper + NEDOF - 2) / NEDOF + 1 <= L::RES;   // rper rows meet no more elements
+  const bool resident = (rper + NEDOF - 2) / NEDOF + 1 <= L::RES;   // a run of rper rows meets no more elements
   const int per = (A.nelmt + grid - 1) / grid;
   const int r0 = resident ? min(rows, bid * rper) : min(A.nelmt, bid * per) * NEDOF;
   const int r1 = resident ? min(rows, r0 + rper) : min(A.nelmt, bid * per + per) * NEDOF;
@@ -353,7 +228,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
   if (resident) {
     const double2* src = reinterpret_cast<const double2*>(A.K + (size_t)e0 * L::STRIDE);
     for (int i = t; i < nel * (L::STRIDE / 2); i += NT) reinterpret_cast<double2*>(kb)[i] = __ldcs(src + i);
-  } else if (!MF && nel > 0) {
+  } else if (nel > 0) {
     copy_group(0);
   }
   auto barrier = [&]() -> bool {
@@ -401,12 +276,10 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
   bool ok = true;
   for (int k = 0; k < A.chunk && ok; ++k) {
     // ---- element products of p = z + beta p_old ----
-    if constexpr (MF) {
-      point_products(A, dsm, e0, nel, s_beta);
-    } else if (resident) {
+    if (resident) {
       for (int i = t; i < nel * NEDOF; i += NT) ps[i] = direction(0, i);
       __syncthreads();
-      row_products<FORM>(A, kb, ps, e0, r0 - e0 * NEDOF, r1 - e0 * NEDOF, nbr, warp, lane);
+      row_products<ROWS>(A, kb, ps, e0, r0 - e0 * NEDOF, r1 - e0 * NEDOF, nbr, warp, lane);
     } else {
       if (t < min(L::GE, nel) * NEDOF) ps[t] = direction(0, t);
       for (int g = 0; g < ngrp; ++g) {
@@ -418,7 +291,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
         ok = mbar_wait(bar + b, (waited >> 1) & 1);
         if (__syncthreads_or(!ok)) { ok = false; break; }
         ++waited;
-        row_products<FORM>(A, kb + (size_t)b * L::GE * L::STRIDE, ps + (g & 1) * L::GE * NEDOF, e0 + g * L::GE, 0,
+        row_products<ROWS>(A, kb + (size_t)b * L::GE * L::STRIDE, ps + (g & 1) * L::GE * NEDOF, e0 + g * L::GE, 0,
                            n * NEDOF, nbr, warp, lane);
         if (t < nn * NEDOF) ps[((g + 1) & 1) * L::GE * NEDOF + t] = nd;
         __syncthreads();
@@ -482,23 +355,16 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
       if (lane == 0) __stcg(partB + w, dot);
     }
     if (!barrier()) { ok = false; break; }
-    // alpha: the partials in the order of the last block's sum (a chain of up
-    // to 256 additions; the matrix-free products round differently anyway, and
-    // their dots are added by a tree: 3 us instead of 10 at 12,000 elements)
-    if constexpr (MF) {
-      const double v = tree_sum(partB, VW * A.ggrid, sfin, t, lane, warp);
-      if (t == 0) s_alpha = s_rz / v;
-    } else {
-      for (int b = t; b < A.ggrid; b += NT) spart[b] = block_partial(partB, b);
-      __syncthreads();
-      if (t < VT) {
-        double v = 0.0;
-        for (int b = t; b < A.ggrid; b += VT) v += spart[b];
-        sfin[t] = v;
-      }
-      __syncthreads();
-      if (t == 0) s_alpha = s_rz / chain(sfin, min(VT, A.ggrid));
+    // alpha: the partials in the order of the last block's sum
+    for (int b = t; b < A.ggrid; b += NT) spart[b] = block_partial(partB, b);
+    __syncthreads();
+    if (t < VT) {
+      double v = 0.0;
+      for (int b = t; b < A.ggrid; b += VT) v += spart[b];
+      sfin[t] = v;
     }
+    __syncthreads();
+    if (t == 0) s_alpha = s_rz / chain(sfin, min(VT, A.ggrid));
     __syncthreads();
     // ---- u, r, z, max-norms and r.z, by warps of the update's grid ----
     const double alpha = s_alpha;
@@ -539,10 +405,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
     ++it;
     {
       constexpr int NJ = VT / 4;
-      double rzn = 0.0;
-      if constexpr (MF) rzn = tree_sum(partZ, VW * A.ugrid, sfin, t, lane, warp);
-      else
-        for (int b = t; b < A.ugrid; b += NT) spart[b] = block_partial(partZ, b);
+      for (int b = t; b < A.ugrid; b += NT) spart[b] = block_partial(partZ, b);
       unsigned long long mp = 0, mu = 0;
       for (int w = t; w < VW * A.ugrid; w += NT) {
         mp = max(mp, __ldcg(partP + w));
@@ -552,7 +415,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
       mu = warp_max(mu);
       if (lane == 0) { smax[warp][0] = mp; smax[warp][1] = mu; }
       __syncthreads();
-      if (!MF && t < NJ) {
+      if (t < NJ) {
         double v = 0.0;
         for (int b = t; b < A.ugrid; b += NJ) v += spart[b];
         sfin[t] = v;
@@ -575,7 +438,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent64(Args A) {
           if (it >= maxiter) {
             s_done = 1; s_failed = 1;
           } else {
-            const double s = MF ? rzn : chain(sfin, min(NJ, A.ugrid));
+            const double s = chain(sfin, min(NJ, A.ugrid));
             s_beta = s / s_rz;
             s_rz = s;
           }
@@ -620,12 +483,12 @@ __global__ void __launch_bounds__(256) k_pack_rows(const double* __restrict__ K,
   if (__syncthreads_or(bad) && threadIdx.x == 0) *other = 1;
 }
 
-template <int FORM>
+template <bool ROWS>
 static bool launch(Args A, int grid, cudaStream_t s) {
-  using L = Lay<FORM>;
+  using L = Lay<ROWS>;
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(k_pcg_persistent64<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM) !=
+    if (cudaFuncSetAttribute(k_pcg_persistent64<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM) !=
         cudaSuccess) {
       cudaGetLastError();
       return false;
@@ -633,7 +496,7 @@ static bool launch(Args A, int grid, cudaStream_t s) {
     attr = true;
   }
   void* args[] = {&A};
-  if (cudaLaunchCooperativeKernel((const void*)k_pcg_persistent64<FORM>, grid, NT, args, L::SMEM, s) != cudaSuccess) {
+  if (cudaLaunchCooperativeKernel((const void*)k_pcg_persistent64<ROWS>, grid, NT, args, L::SMEM, s) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -650,18 +513,9 @@ void launch_pack_rows(const double* K, int nelmt, const int* d_nbr, double* out,
   add_launches(1);
 }
 
-// Largest mesh applied from stored matrices where the point records exist.  Up
-// to 1,300 elements the matrices stay in shared memory.  us per iteration,
-// stored / point records: 576 20.2 / 22.3, 882 23.7 / 24.3, 1,200 27.1 / 25.4,
-// 1,700 35.0 / 30.6, 3,289 51.3 / 43.0, 12,000 158 / 106.  The line lies where
-// they meet; below it the solve is also bitwise that of the separate kernels.
-int fp64_stored_max() { return 1000; }
-
 // Up to `chunk` PCG iterations (reference step test).  rows: K is packed by
-// k_pack_rows, else the sparse symmetric layout, which meshes too large for
-// shared memory apply from the point records rec instead, where they exist.
-// False when it cannot run.
-bool launch_pcg_persistent64(bool rows, const double* K, const double* rec, const int* ge, int nelmt, const int* pos, const int* d_nbr,
+// k_pack_rows, else the sparse symmetric layout.  False when it cannot run.
+bool launch_pcg_persistent64(bool rows, const double* K, const int* ge, int nelmt, const int* pos, const int* d_nbr,
                              const GatherTopo& T, int n1, double* u, double* r, double* z, double* p, double* kp,
                              double* Y, const double* dp, ColState* cs, PcgGlobal* G, double* part, int chunk,
                              cudaStream_t s) {
@@ -679,13 +533,7 @@ bool launch_pcg_persistent64(bool rows, const double* K, const double* rec, cons
   cudaMemsetAsync(count, 0, sizeof(unsigned), s);
   const p64::Args A{K, ge, pos, d_nbr, nelmt, T.d_ptr, T.d_dof, T.ngroups, n1, ggrid, ugrid,
                     u, r, z, p, kp, Y, dp, cs, G, part, count, chunk};
-  if (rows) return p64::launch<p64::ROWS57>(A, (int)grid, s);
-  if (rec && nelmt > fp64_stored_max()) {
-    p64::Args R = A;
-    R.K = rec;
-    return p64::launch<p64::POINTS>(R, (int)grid, s);
-  }
-  return p64::launch<p64::SPARSE>(A, (int)grid, s);
+  return rows ? p64::launch<true>(A, (int)grid, s) : p64::launch<false>(A, (int)grid, s);
 }
 
 }  // namespace sg
