@@ -126,7 +126,11 @@ struct DotAcc<float> {
     }
   }
   __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+  __device__ __forceinline__ float2 pair() const { return make_float2(hi, lo); }
 };
+// The FP64 unit takes a warp's conversion or addition in some 19 cycles, so the
+// warps of a block leave pairs and a few threads widen and add them.
+__device__ __forceinline__ double widen(float2 x) { return (double)x.x + (double)x.y; }
 
 // Per-column block reduction of `val` (threads whose index = j mod KR hold
 // column j).  Result for column j lands in out[j] on thread 0..KR-1 of warp 0.
@@ -984,26 +988,25 @@ constexpr int FG_THREADS = 384, FG_PER_SM = 2;   // gather: 24 warps at 80 regis
 constexpr int FU_THREADS = 512;                  // update: 16 warps, four pieces a thread in flight
 constexpr int F_BLOCKS = 152;
 
-// Last-block sum of part[nblk][NQ] for the FP32 kernels: thread t adds entry
-// t % NQ of blocks t / NQ, t / NQ + NT / NQ, ... (eight loads in flight), then
-// the threads of one entry are added by a fixed tree.  maxq < NQ marks the
-// entries q with q % QS == maxq as maxima.  The result is in out[0..NQ).
-template <int NQ, int QS, int NT>
-__device__ __forceinline__ void last_block_sum(const double* __restrict__ part, int nblk, int maxq, double* sfin,
-                                               double* out) {
+// Last-block sum of part[nblk][NQ] for the FP32 kernels: thread t < NT adds
+// entry t % NQ of blocks t / NQ, t / NQ + NT / NQ, ... (eight loads in flight),
+// then the threads of one entry are added by a fixed tree.  The result is in
+// out[0..NQ).
+template <int NQ, int NT>
+__device__ __forceinline__ void last_block_sum(const double* __restrict__ part, int nblk, double* sfin, double* out) {
   constexpr int R = NT / NQ;
   const int t = threadIdx.x, q = t % NQ, r = t / NQ;
-  const bool mx = q % QS == maxq;
-  double v = 0.0;
-  if (r < R)
+  if (r < R) {
+    double v = 0.0;
     for (int b0 = r; b0 < nblk; b0 += 8 * R) {
       double x[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) x[k] = b0 + k * R < nblk ? __ldcg(part + (size_t)(b0 + k * R) * NQ + q) : 0.0;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v = mx ? fmax(v, x[k]) : v + x[k];
+      for (int k = 0; k < 8; ++k) v += x[k];
     }
-  sfin[t] = v;
+    sfin[t] = v;
+  }
   __syncthreads();
   if (t < NQ) {
     // entries beyond the last block's row are zero
@@ -1012,8 +1015,8 @@ __device__ __forceinline__ void last_block_sum(const double* __restrict__ part, 
     for (int k = 0; k < rn; k += 4)
 #pragma unroll
       for (int m = 0; m < 4; ++m)
-        if (k + m < rn) a[m] = mx ? fmax(a[m], sfin[(k + m) * NQ + t]) : a[m] + sfin[(k + m) * NQ + t];
-    out[t] = mx ? fmax(fmax(a[0], a[1]), fmax(a[2], a[3])) : (a[0] + a[1]) + (a[2] + a[3]);
+        if (k + m < rn) a[m] += sfin[(k + m) * NQ + t];
+    out[t] = (a[0] + a[1]) + (a[2] + a[3]);
   }
   __syncthreads();
 }
@@ -1138,24 +1141,24 @@ __global__ void __launch_bounds__(FG_THREADS, FG_PER_SM) k_pcg_gather_flat(
     maps(g + 3 * gstride, B);
   }
   if (mode == 0) return;
-  __shared__ double sred[FG_THREADS / 32][KR];
+  __shared__ float2 sred[FG_THREADS / 32][KR];
   __shared__ double sfin[FG_THREADS];
   __shared__ double sout[KR];
 #pragma unroll
   for (int k = 0; k < VW; ++k) {
     dacc[k].warp_sum(QPD);
-    if (lane < QPD) sred[warp][VW * lane + k] = dacc[k].value();   // lane r holds pieces q % QPD of its lane class
+    if (lane < QPD) sred[warp][VW * lane + k] = dacc[k].pair();   // lane r holds pieces q % QPD of its lane class
   }
   __syncthreads();
   // lane class r = lane % QPD of warp w holds columns VW * ((32 w + r) % QPD) ..: 32 is a multiple of QPD
   if (threadIdx.x < KR) {
     double v = 0.0;
 #pragma unroll
-    for (int w = 0; w < FG_THREADS / 32; ++w) v += sred[w][threadIdx.x];
+    for (int w = 0; w < FG_THREADS / 32; ++w) v += widen(sred[w][threadIdx.x]);
     part[(size_t)blockIdx.x * KR + threadIdx.x] = v;
   }
   if (last_block(&G->cntB)) {
-    last_block_sum<KR, 1, FG_THREADS>(part, gridDim.x, 1, sfin, sout);
+    last_block_sum<KR, FG_THREADS>(part, gridDim.x, sfin, sout);
     if (threadIdx.x < KR) {
       const int j = threadIdx.x;
       if (cs[j].active && !cs[j].done) cs[j].alpha = cs[j].rz / sout[j];
@@ -1639,6 +1642,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_update(
 // and is not formed.  HBM bounds it at large meshes (7 vector passes); one
 // block of 512 threads per SM with four pieces of four vectors a thread in
 // flight (128 KB) leaves 152 partials for the last block.
+// The dots stay pairs and the maxima FP32 until a few threads add the warps' and
+// the blocks': widened by every warp, and maxima in FP64, the tail took 5 to 7
+// us more.  us at 62,000 elements and 8 columns 72 -> 67, 16,000 and 16 49 -> 42.
 template <int KR>
 __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
     int n1, float* __restrict__ u, float* __restrict__ r, float* __restrict__ z, const float* __restrict__ p,
@@ -1745,11 +1751,15 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
       }
     }
   }
-  // partials [block][column][4] = max|p|, -, r.z, |r|^2
-  constexpr int NQ = 4 * KR;
-  __shared__ double sred[FU_THREADS / 32][NQ];
-  __shared__ double sfin[FU_THREADS];
+  // block partials: r.z and |r|^2 of each column, and the maxima behind them
+  constexpr int NQ = 2 * KR, NW = FU_THREADS / 32, NS = FU_THREADS / 2, QC = 4 * QP;
+  double* psum = part;
+  float* pmax = reinterpret_cast<float*>(part + (size_t)gridDim.x * NQ);
+  __shared__ float2 sred[NW][2][QC];   // per warp: r.z and |r|^2 of its components
+  __shared__ float smp[NW][QC];
+  __shared__ double sfin[NS];
   __shared__ double sout[NQ];
+  __shared__ float smax[FU_THREADS - NS];
   __shared__ int s_alldone;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
@@ -1758,34 +1768,48 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
     rra[k].warp_sum(QP);
 #pragma unroll
     for (int o = 16; o >= QP; o >>= 1) mp[k] = fmaxf(mp[k], __shfl_xor_sync(FULL, mp[k], o));
-  }
-  if (lane < QP) {
-#pragma unroll
-    for (int k = 0; k < NC; ++k) {
-      double* o = sred[warp] + 4 * (4 * lane * (KR >= 4) + k);
-      double m = 0.0, a = 0.0, b = 0.0;
-#pragma unroll
-      for (int c = k; c < 4; c += NC) { m = fmax(m, (double)mp[c]); a += rza[c].value(); b += rra[c].value(); }
-      o[0] = m; o[1] = 0.0; o[2] = a; o[3] = b;
+    if (lane < QP) {
+      sred[warp][0][4 * lane + k] = rza[k].pair();
+      sred[warp][1][4 * lane + k] = rra[k].pair();
+      smp[warp][4 * lane + k] = mp[k];
     }
   }
   __syncthreads();
-  if (threadIdx.x < NQ) {
-    const int q = threadIdx.x & 3;
+  if (threadIdx.x < NQ) {   // quantity and column: a column's components are j, j + KR, ...
+    const int h = threadIdx.x / KR, j = threadIdx.x % KR;
     double v = 0.0;
 #pragma unroll
-    for (int w = 0; w < FU_THREADS / 32; ++w) v = q == 0 ? fmax(v, sred[w][threadIdx.x]) : v + sred[w][threadIdx.x];
-    part[(size_t)blockIdx.x * NQ + threadIdx.x] = v;
+    for (int w = 0; w < NW; ++w) {
+      double x = 0.0;
+#pragma unroll
+      for (int c = 0; c < QC; c += KR) x += widen(sred[w][h][j + c]);
+      v += x;
+    }
+    psum[(size_t)blockIdx.x * NQ + threadIdx.x] = v;
+  } else if (threadIdx.x >= 32 * ((NQ + 31) / 32) && threadIdx.x < 32 * ((NQ + 31) / 32) + KR) {
+    const int j = threadIdx.x - 32 * ((NQ + 31) / 32);
+    float m = 0.f;
+    for (int w = 0; w < NW; ++w)
+      for (int c = 0; c < QC; c += KR) m = fmaxf(m, smp[w][j + c]);
+    pmax[(size_t)blockIdx.x * KR + j] = m;
   }
   if (!last_block(&G->cntC)) return;
-  last_block_sum<NQ, 4, FU_THREADS>(part, gridDim.x, 0, sfin, sout);
+  if (threadIdx.x >= NS) {
+    const int i = threadIdx.x - NS;
+    float m = 0.f;
+    for (int b = i / KR; b < (int)gridDim.x; b += (FU_THREADS - NS) / KR)
+      m = fmaxf(m, __ldcg(pmax + (size_t)b * KR + i % KR));
+    smax[i] = m;
+  }
+  last_block_sum<NQ, NS>(psum, gridDim.x, sfin, sout);
   if (threadIdx.x == 0) s_alldone = 1;
   __syncthreads();
   const int it = init ? 0 : G->it + 1;
   if (threadIdx.x < KR) {
-    const double* o = sout + 4 * threadIdx.x;
     ColState& c = cs[threadIdx.x];
-    col_step(init, it, c, G, o[0], 0.0, o[2], o[3]);
+    float m = 0.f;
+    for (int i = threadIdx.x; i < FU_THREADS - NS; i += KR) m = fmaxf(m, smax[i]);
+    col_step(init, it, c, G, (double)m, 0.0, sout[threadIdx.x], sout[KR + threadIdx.x]);
     if ((int)threadIdx.x < G->kcols && c.active && !c.done) atomicAnd(&s_alldone, 0);
   }
   __syncthreads();

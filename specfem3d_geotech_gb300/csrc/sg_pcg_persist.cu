@@ -71,14 +71,6 @@ struct CompSum {
     hi = t;
     lo = (lo + x.y) + err;
   }
-  // sum over the lanes whose index differs in bits >= o0
-  __device__ __forceinline__ void warp_sum(int o0) {
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-      if (o < o0) break;
-      add(make_float2(__shfl_xor_sync(0xffffffffu, hi, o), __shfl_xor_sync(0xffffffffu, lo, o)));
-    }
-  }
   __device__ __forceinline__ float2 pair() const { return make_float2(hi, lo); }
 };
 __device__ __forceinline__ double value(const float2 x) { return (double)x.x + (double)x.y; }
