@@ -5,7 +5,7 @@ Workload (the 3D slope the headline metric is quoted on): 120x40x40 mapped
 hex mesh, NGLL=3, 4.63M dofs, three lognormally perturbed layers, seeded
 synthetic data; a factor-of-safety solve searches SRF on [1, 3] to 0.01 with
 nl_maxiter = 2000.  Form measured: the mixed-precision batched serving form --
-FP32 element matrices and FP32 PCG with FP64 iterative refinement, k = 8
+FP32 operator and FP32 PCG with FP64 iterative refinement, k = 8
 concurrent SRF trials sharing every element apply as 8 right-hand sides, the
 search is the bisection with its next probes run ahead in the batch (sg_fos with
 k = 8).
@@ -79,7 +79,7 @@ def workload_config(world: int, ne: int = 192000, neq: int = 4633520, nx: int = 
             "nelmt": ne, "neq": neq,
             "fos_model": "FOS solves/s = 1 / (plastic iterations per FOS solve x s per plastic iteration); "
                          "iterations counted by a complete search of the 576-element cut of the same slope",
-            "l2": "inputs larger than L2 (FP32 element matrices 1.87 GB)", "parallelism": f"replicas{world}"}
+            "l2": "inputs larger than L2 (point records, element products and vectors 1.3 GB)", "parallelism": f"replicas{world}"}
 
 
 def golden_fos():
