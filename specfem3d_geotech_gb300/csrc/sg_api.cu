@@ -541,6 +541,7 @@ int sg_pcg_solve(sg_ctx* c, int neq, int nelmt, int nedof, const double* k, doub
         set_tag(errtag, "ERROR: gdof_elmt entry out of [0,neq]!");
         return SG_ERR_BADARG;
       }
+    D.neq = -1;   // until its topology is on the device, the kept map counts as no map
     D.ge.assign(gdof_elmt, gdof_elmt + (size_t)nelmt * NEDOF);
     build_groups_from_gdof(gdof_elmt, nelmt, neq, D.T);
     if (!upload_topo(c, D.T)) { set_tag(errtag, "ERROR: out of device memory!"); return SG_ERR_OOM; }
