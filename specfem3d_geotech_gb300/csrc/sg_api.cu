@@ -142,12 +142,24 @@ struct sg_ctx {
     err = std::string(what) + ": " + cudaGetErrorString(e);
     return false;
   }
-  template <typename T>
-  T* alloc(size_t n) {
-    size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+  void* reserve(size_t bytes) {
     if (budget && used + bytes > budget) { err = "HBM budget exceeded"; return nullptr; }
     void* p = nullptr;
     if (cudaMalloc(&p, bytes) != cudaSuccess) { cudaGetLastError(); err = "cudaMalloc failed"; return nullptr; }
+    return p;
+  }
+  template <typename T>
+  T* alloc(size_t n) {
+    size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
+    void* p = reserve(bytes);
+    // the drop-in's packed rows only save time: whatever else needs the room gets it
+    if (!p && dropin.rows) {
+      release(dropin.rows);
+      dropin.rows = nullptr;
+      dropin.rowcap = 0;
+      p = reserve(bytes);
+    }
+    if (!p) return nullptr;
     used += bytes;
     live[p] = bytes;
     return (T*)p;

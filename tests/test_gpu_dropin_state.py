@@ -57,3 +57,41 @@ def test_map_of_a_refused_call_is_checked_again():
         assert sg.pcg_solver(*few, one, 500, 1e-10, ctx=ctx)[1] == 0
     """ % ROOT
     subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT, timeout=300, env=dict(os.environ, SG_PERSIST="0"))
+
+
+def rows_bytes(n):
+    return 4618 * 8 * n   # the packed matrices a solve of n elements may keep
+
+
+def needs(n):
+    """Device bytes of a context after one solve, without the packed rows."""
+    ctx = sg.Context(0)
+    solve(ctx, n)
+    return ctx.hbm_used - rows_bytes(n)
+
+
+def test_a_larger_solve_fits_after_a_smaller_one():
+    ctx = sg.Context(0, needs(400) + 65536)
+    solve(ctx, 100)
+    kept = ctx.hbm_used
+    assert kept > rows_bytes(100) + needs(100) - 65536   # the first solve's rows were kept
+    solve(ctx, 400)
+    solve(ctx, 100)
+
+
+def test_a_model_fits_after_a_solve():
+    from specfem3d_geotech_gb300 import meshgen
+
+    mesh = meshgen.slope3d(6, 5, 5)
+    ctx = sg.Context(0)
+    before = ctx.hbm_used
+    model = sg.Model(mesh, ctx=ctx)
+    room = ctx.hbm_used - before
+    model.close()
+    n = 20
+    assert rows_bytes(n) < room / 4
+    ctx = sg.Context(0, needs(n) + room + 65536)
+    solve(ctx, n)
+    assert ctx.hbm_used >= needs(n) + rows_bytes(n)
+    sg.Model(mesh, ctx=ctx).close()
+    solve(ctx, n)
