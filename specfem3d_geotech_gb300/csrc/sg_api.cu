@@ -574,12 +574,13 @@ int sg_pcg_solve(sg_ctx* c, int neq, int nelmt, int nedof, const double* k, doub
     D.r = c->alloc<double>(n1); D.z = c->alloc<double>(n1); D.p = c->alloc<double>(n1); D.kp = c->alloc<double>(n1);
     D.n1cap = n1;
   }
-  if (!D.part) {
-    D.part = c->alloc<double>((size_t)NPART * 16 * 4);
-    D.cs = c->alloc<ColState>(16);
-    D.G = c->alloc<PcgGlobal>(1);
-  }
-  if (!D.d_K || !D.d_ge || !D.Y || !D.u || !D.part || !D.cs || !D.G) {
+  if (!D.part) D.part = c->alloc<double>((size_t)NPART * 16 * 4);
+  if (!D.cs) D.cs = c->alloc<ColState>(16);
+  if (!D.G) D.G = c->alloc<PcgGlobal>(1);
+  if (!D.d_K || !D.d_ge || !D.Y || !D.u || !D.f || !D.dp || !D.r || !D.z || !D.p || !D.kp || !D.part || !D.cs ||
+      !D.G) {
+    D.kcap = 0;   // the next call asks again for what is missing
+    D.necap = D.n1cap = 0;
     set_tag(errtag, "ERROR: out of device memory!");
     return SG_ERR_OOM;
   }

@@ -95,3 +95,18 @@ def test_a_model_fits_after_a_solve():
     assert ctx.hbm_used >= needs(n) + rows_bytes(n)
     sg.Model(mesh, ctx=ctx).close()
     solve(ctx, n)
+
+
+def test_a_solve_whose_vectors_do_not_fit_is_refused():
+    """Budgets that end anywhere among the solve's buffers: refused, not run
+    with a missing one, and the context stays usable."""
+    n = 40
+    neq, k, f, dinv, ge, _ = apart(n)
+    full = needs(n)
+    for short in range(1, 40):
+        ctx = sg.Context(0, full - short * 8 * (neq + 1) // 4)
+        with pytest.raises(sg.SgError) as e:
+            sg.pcg_solver(neq, n, k, np.zeros(neq + 1), f, dinv, ge, 500, 1e-12, ctx=ctx)
+        assert e.value.code == sg.SG_ERR_OOM
+        solve(ctx, 2)
+        ctx.close()
