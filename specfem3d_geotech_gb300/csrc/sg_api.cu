@@ -1145,7 +1145,8 @@ struct SolveStats {
 static Op fp32_op(const sg_model* M, const Op& op64) {
   Op o = op64;
   o.K = M->d_K32;
-  if (fp32_matrix_free()) {
+  // also for a model built while the operator was matrix-free: it has no FP32 matrices
+  if (fp32_matrix_free() || !M->d_K32) {
     o.dense = 2;
     o.K = M->d_rec32;
   }
