@@ -350,6 +350,8 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
       eager_chunk();
     }
     ++nchunks;
+    // a refused launch leaves the others nothing new to work on
+    if (!C->check(cudaGetLastError(), "pcg")) return SG_ERR_CUDA;
     cudaMemcpyAsync((void*)hG, B.G, sizeof(PcgGlobal), cudaMemcpyDeviceToHost, s);
     if (!C->check(cudaStreamSynchronize(s), "pcg")) return SG_ERR_CUDA;
     it = hG->it;
@@ -541,6 +543,7 @@ int sg_pcg_solve(sg_ctx* c, int neq, int nelmt, int nedof, const double* k, doub
     return SG_ERR_BADARG;
   }
   cudaSetDevice(c->device);
+  cudaGetLastError();   // what other code of this thread left behind
   auto& D = c->dropin;
   const int n1 = neq + 1;
   const size_t nk = (size_t)nelmt * NEDOF * NEDOF;

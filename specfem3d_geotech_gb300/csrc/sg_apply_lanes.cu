@@ -306,13 +306,10 @@ void launch_apply_lanes(const float* Ks, const int* ge, int nelmt, const float* 
                         FusedDir fz) {
   using S = lanes::Shape<KR>;
   // one kernel per way of forming the direction (separate register budgets)
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(lanes::k_apply_lanes<KR, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-    cudaFuncSetAttribute(lanes::k_apply_lanes<KR, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-    cudaFuncSetAttribute(lanes::k_apply_lanes<KR, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-    attr = true;
-  }
+  static std::atomic<unsigned long long> a0{}, a1{}, a2{};
+  allow_smem(a0, (const void*)lanes::k_apply_lanes<KR, 0>, S::SMEM);
+  allow_smem(a1, (const void*)lanes::k_apply_lanes<KR, 1>, S::SMEM);
+  allow_smem(a2, (const void*)lanes::k_apply_lanes<KR, 2>, S::SMEM);
   const int ngroups = (nelmt + S::EPW - 1) / S::EPW;
   const int warps = (ngroups + lanes::NW - 1) / lanes::NW;
   int grid = warps < 152 ? warps : 152;

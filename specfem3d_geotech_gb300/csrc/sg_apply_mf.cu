@@ -441,12 +441,9 @@ void launch_apply_mf(const float* rec, const int* ge, int nelmt, const float* po
     mf::k_apply_mf_lines<KR><<<grid, S::NT, 0, s>>>(rec, ge, nelmt, pold, z, combine, Y, cs, G, pos);
   } else {
     using S = mf::Shape<KR>;
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(mf::k_apply_mf_planes<KR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-      cudaFuncSetAttribute(mf::k_apply_mf_planes<KR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-      attr = true;
-    }
+    static std::atomic<unsigned long long> plain{}, combined{};
+    if (combine) allow_smem(combined, (const void*)mf::k_apply_mf_planes<KR, true>, S::SMEM);
+    else allow_smem(plain, (const void*)mf::k_apply_mf_planes<KR, false>, S::SMEM);
     const int ng = (nelmt + S::EPG - 1) / S::EPG, nb = (ng + S::NG - 1) / S::NG;
     const int grid = nb < 152 ? nb : 152;
     if (grid < 1) return;

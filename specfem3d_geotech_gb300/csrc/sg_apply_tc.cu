@@ -325,11 +325,8 @@ template <int KR>
 void launch_apply_tc(const float* Ks, const int* ge, int nelmt, const float* pold, const float* z, int combine,
                      float* Y, const ColState* cs, const PcgGlobal* G, const int* d_entry, const int* pos,
                      int* err, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(tc::k_apply_tc<KR>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
-    attr = true;
-  }
+  static std::atomic<unsigned long long> allowed{};
+  allow_smem(allowed, (const void*)tc::k_apply_tc<KR>, tc::SMEM_BYTES);
   int grid = nelmt < 152 ? nelmt : 152;
   if (grid < 1) return;
   tc::k_apply_tc<KR><<<grid, tc::THREADS, tc::SMEM_BYTES, s>>>(Ks, ge, nelmt, pold, z, combine, Y, cs, G, d_entry,

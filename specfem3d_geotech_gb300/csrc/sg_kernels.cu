@@ -799,11 +799,8 @@ void pcg_apply(int dense, const void* K, const int* ge, int nelmt, const V* p_ol
   }
   if (g_apply_variant >= 1) {
     size_t sm = apply_tma_smem<V, KR>();
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(k_apply_sparse_tma<V, KR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      attr = true;
-    }
+    static std::atomic<unsigned long long> allowed{};
+    allow_smem(allowed, (const void*)k_apply_sparse_tma<V, KR>, sm);
     // persistent-style grid: each warp walks a strided list of elements
     int per_sm = (int)(200 * 1024 / sm);
     if (per_sm < 1) per_sm = 1;
@@ -813,11 +810,8 @@ void pcg_apply(int dense, const void* K, const int* ge, int nelmt, const V* p_ol
     return;
   }
   size_t sm = apply_sparse_smem<V, KR>();
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_apply_sparse<V, KR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    attr = true;
-  }
+  static std::atomic<unsigned long long> allowed{};
+  allow_smem(allowed, (const void*)k_apply_sparse<V, KR>, sm);
   SG_LAUNCH k_apply_sparse<V, KR><<<blocks, APPLY_WARPS * 32, sm, s>>>((const V*)K, ge, nelmt, p_old, z, combine, Y, cs, G,
                                                                d_nbr, pos);
 }
@@ -1427,11 +1421,8 @@ void pcg_gather(const GatherTopo& T, const V* Y, V* kp, V* p, const V* z, int mo
     }
   }
   constexpr size_t sm = GatherBuf<V, KR>::SMEM;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_pcg_gather<V, KR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    attr = true;
-  }
+  static std::atomic<unsigned long long> allowed{};
+  allow_smem(allowed, (const void*)k_pcg_gather<V, KR>, sm);
   SG_LAUNCH k_pcg_gather<V, KR><<<red_grid(T.ngroups, VGATHER, NPART), RED_THREADS, sm, s>>>(T.d_ptr, T.d_ent, T.d_dof, T.ngroups, Y, kp, p, z, mode,
                                                               cs, G, part);
 }

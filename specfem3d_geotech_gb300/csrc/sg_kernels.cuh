@@ -2,6 +2,9 @@
 // translation units.
 #pragma once
 
+#include <atomic>
+#include <type_traits>
+
 #include "sg_internal.h"
 
 namespace sg {
@@ -31,19 +34,28 @@ struct PcgGlobal {
   int err;        // set to 1 by a bounded wait of this solve's kernels that ran out
 };
 
-#ifdef __CUDACC__
+// Allows `bytes` of dynamic shared memory to a kernel, once per device: a bit of
+// `done`, which belongs to the kernel, says so.
+inline bool allow_smem(std::atomic<unsigned long long>& done, const void* kernel, size_t bytes) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load(std::memory_order_acquire) & bit) return true;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+  done.fetch_or(bit, std::memory_order_release);
+  return true;
+}
+
 // The kernels of an FP32 iteration are launched with programmatic stream
 // serialization: a kernel's blocks take the SMs as the blocks of the one before
 // leave them and wait in chain_wait() until it is complete, instead of being
 // launched after that.  Every kernel of the chain waits before it touches
 // memory, so it also stands behind all earlier ones.  (62,000 elements, 8
-// trials: 301 -> 293 us per iteration.)
-__device__ __forceinline__ void chain_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-template <typename... P, typename... A>
-inline void launch_chained(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
+// trials: 301 -> 293 us per iteration.)  A refused launch stays the thread's
+// last CUDA error, as with any other launch.
+template <typename... P>
+inline void launch_chained(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t s,
+                           std::common_type_t<P>... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -54,7 +66,14 @@ inline void launch_chained(void (*kernel)(P...), int grid, int threads, size_t s
   cfg.stream = s;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  void* argv[] = {(void*)&args...};
+  cudaLaunchKernelExC(&cfg, (const void*)kernel, argv);
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // Direction of a pass over the mesh in iteration G->it: each of an iteration's

@@ -726,14 +726,10 @@ bool persist_enabled() {
 
 template <int KR, int R>
 static bool launch_persistent(const pp::Args& A, int grid, size_t smem, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(pp::k_pcg_persistent<KR, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             220 * 1024) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    attr = true;
+  static std::atomic<unsigned long long> allowed{};
+  if (!allow_smem(allowed, (const void*)pp::k_pcg_persistent<KR, R>, 220 * 1024)) {
+    cudaGetLastError();
+    return false;
   }
   pp::Args a = A;
   void* args[] = {&a};

@@ -486,14 +486,10 @@ __global__ void __launch_bounds__(256) k_pack_rows(const double* __restrict__ K,
 template <bool ROWS>
 static bool launch(Args A, int grid, cudaStream_t s) {
   using L = Lay<ROWS>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_pcg_persistent64<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    attr = true;
+  static std::atomic<unsigned long long> allowed{};
+  if (!allow_smem(allowed, (const void*)k_pcg_persistent64<ROWS>, L::SMEM)) {
+    cudaGetLastError();
+    return false;
   }
   void* args[] = {&A};
   if (cudaLaunchCooperativeKernel((const void*)k_pcg_persistent64<ROWS>, grid, NT, args, L::SMEM, s) != cudaSuccess) {
