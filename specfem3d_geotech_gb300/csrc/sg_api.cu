@@ -220,6 +220,13 @@ struct Op {
   const double* rows = nullptr;   // dense: the matrices packed by rows, where their pattern allows it
 };
 
+// A solve that is not done ends with SG_ERR_TIMEOUT after SG_WALL_LIMIT seconds
+// (an hour), looked at whenever the host looks at the solve.
+static bool past_wall_limit(std::chrono::steady_clock::time_point t0) {
+  static const double limit = std::getenv("SG_WALL_LIMIT") ? std::atof(std::getenv("SG_WALL_LIMIT")) : 3600.0;
+  return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > limit;
+}
+
 template <typename V>
 struct PcgBufs {
   V *r = nullptr, *z = nullptr, *p = nullptr, *kp = nullptr, *Y = nullptr;
@@ -329,7 +336,7 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
   bool persist = false;
   if constexpr (std::is_same<V, double>::value && KR == 1)
     persist = !(mode & 1) && (op.dense == 0 ? persist_default_apply() : op.rows != nullptr) && persist_enabled();
-  constexpr int persist_chunk = 512;
+  const int persist_chunk = persist_iterations(512);
   int nchunks = 0;
   while (true) {
     bool done_chunk = false;
@@ -363,8 +370,7 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
     }
     if (hG->all_done) break;
     if (it >= maxiter + std::max(chunk, persist_chunk)) { status = SG_ERR_TIMEOUT; break; }
-    double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-    if (el > 3600.0) { status = SG_ERR_TIMEOUT; C->err = "PCG wall-clock guard"; break; }
+    if (past_wall_limit(t0)) { status = SG_ERR_TIMEOUT; C->err = "PCG wall-clock guard"; break; }
   }
   if constexpr (std::is_same<V, float>::value && (KR == 8 || KR == 16))
     if (fused) fused_dir_restore<KR>(n1, B.p, B.r, dp, B.cs, s);
@@ -1159,7 +1165,7 @@ static Op fp32_op(const sg_model* M, const Op& op64) {
 // One persistent FP32 solve, or its next chunk; false when it cannot run.
 static bool persist_round(sg_ctx* c, int KR, const Op& op, TrialWork& W, const float* dp, const PersistStart& st,
                           PersistOut* out) {
-  constexpr int chunk = 4096;   // bounds the time between two looks of the host
+  const int chunk = persist_iterations(4096);   // bounds the time between two looks of the host
   auto run = [&](auto kr) {
     return launch_pcg_persistent<decltype(kr)::value>((const float*)op.K, op.ge, op.nelmt, op.T->d_pos, *op.T, W.r32,
                                                       W.d32, W.b32.r, W.b32.z, W.b32.p, W.b32.kp, W.b32.Y, dp,
@@ -1206,6 +1212,7 @@ static int linear_solve(sg_model* M, const sg_control* ctl, const Op& op64, cons
   double* corr_part = W.b64.part + (size_t)NPART * 32;   // the residual's partials take the first half
   bool pending = false;                                  // a persistent solve and its correction are under way
   bool fresh = true;                                     // no solve of this call has finished yet
+  std::chrono::steady_clock::time_point t0;              // start of the solve under way
   unsigned mask = 0;
   auto launch = [&](bool init) -> bool {
     const PersistStart st{init, !fresh, ctl->cg_maxiter, k, mask, itol};
@@ -1232,6 +1239,10 @@ static int linear_solve(sg_model* M, const sg_control* ctl, const Op& op64, cons
         return SG_ERR_TIMEOUT;
       }
       if (out->state == PERSIST_MORE) {   // the chunk ended first: nothing was added to x
+        if (out->it >= ctl->cg_maxiter || past_wall_limit(t0)) {   // the solve itself ends at cg_maxiter
+          c->err = "PCG wall-clock guard";
+          return SG_ERR_TIMEOUT;
+        }
         if (!launch(false)) { c->err = "PCG: the persistent solve could not continue"; return SG_ERR_CUDA; }
         continue;
       }
@@ -1258,6 +1269,7 @@ static int linear_solve(sg_model* M, const sg_control* ctl, const Op& op64, cons
     mask = 0;
     for (int j = 0; j < k; ++j) mask |= (unsigned)(live[j] != 0) << j;
     if (persist) {
+      t0 = std::chrono::steady_clock::now();
       pending = launch(true);
       if (pending) continue;
       persist = false;   // a cooperative launch of this size is not possible here

@@ -165,6 +165,7 @@ bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int
                            PersistOut* out, int chunk, cudaStream_t s);
 bool persist_enabled();                 // SG_PERSIST=0 turns the persistent chunk off
 int persist_max_elements(int KR);       // meshes below this use it
+int persist_iterations(int n);          // of one persistent launch: n, or what SG_PERSIST_CHUNK says
 // FP64 solve of one right-hand side as a persistent cooperative kernel
 // (sg_pcg_persist64.cu), bitwise the separate kernels' solve; false when it
 // cannot run.  rows: K packed by launch_pack_rows, whose *other says that a

@@ -724,6 +724,11 @@ bool persist_enabled() {
   return on;
 }
 
+int persist_iterations(int n) {
+  static const int set = getenv("SG_PERSIST_CHUNK") ? atoi(getenv("SG_PERSIST_CHUNK")) : 0;
+  return set > 0 ? set : n;
+}
+
 template <int KR, int R>
 static bool launch_persistent(const pp::Args& A, int grid, size_t smem, cudaStream_t s) {
   static std::atomic<unsigned long long> allowed{};
