@@ -285,6 +285,40 @@ def apply_kernel_name(kr: int, nelmt: int) -> str:
     return f"k_apply_sparse_tma<float,{kr}>"
 
 
+def kernel_report(prof, ne: int, neq: int, kr: int, steps: int):
+    """Roofline of the dominant kernel of the mixed PCG, and milliseconds per
+    iteration: the batched FP32 element apply, or, where an iteration runs
+    inside one kernel, that kernel (whose applies the profile does not count)."""
+    hbm, peak_kind = peaks()
+    vec = (neq + 1) * kr * 4
+    bytes_mf = ne * (27 * 48 + 27 * 4)        # matrix-free: point records + connectivity
+    stress = {"stress_per_step": prof["stress_ms"] / max(1, steps)}
+    if prof["persistent_ms"] > 0:
+        it_ms = prof["persistent_ms"] / max(1, prof["pcg_iters"])
+        nbytes = bytes_mf + 7 * vec           # p, u, r read and written, kp read
+        achieved = nbytes / (it_ms / 1000.0) / 1e9
+        return ({"bound": "latency", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
+                 "traffic": None, "kernel": f"k_pcg_persistent<{kr}>", "algorithmic_bytes_per_iteration": nbytes,
+                 "avg_iteration_ms": it_ms, "peak_source": peak_kind}, {"persistent": it_ms, **stress})
+    name = apply_kernel_name(kr, ne)
+    ks_nnz_unique = 2349                      # structurally non-zero unique entries of a symmetric GLL K_e
+    nbytes = (bytes_mf if name.startswith("k_apply_mf") else ne * (ks_nnz_unique * 4 + 27 * 4)) + 2 * vec
+    n = max(1, prof["apply_launches"])
+    apply_ms = prof["apply_ms"] / n
+    achieved = nbytes / (apply_ms / 1000.0) / 1e9
+    traffic = None
+    tpath = os.path.join(ROOT, "profiles", "apply_traffic.json")
+    if os.path.exists(tpath):
+        with open(tpath) as f:
+            measured = json.load(f)
+        if measured.get("kernel") == name:
+            traffic = measured.get("bytes_per_launch")
+    return ({"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
+             "traffic": traffic, "kernel": name, "algorithmic_bytes_per_launch": nbytes, "avg_launch_ms": apply_ms,
+             "peak_source": peak_kind},
+            {"apply": apply_ms, "gather": prof["gather_ms"] / n, "update": prof["update_ms"] / n, **stress})
+
+
 PREC_STEPS = 2               # plastic iterations compared by the 192k precision check
 
 
@@ -670,23 +704,7 @@ def run_ours(args, rank, world, local):
         count_src = "upper bounds: 3 rounds x nl_maxiter (batched), 8 trials x nl_maxiter (bisection)"
     value = world / (s_mixed * step_s)
 
-    # roofline of the dominant kernel: the batched FP32 element apply (k RHS)
-    hbm, peak_kind = peaks()
-    ks_nnz_unique = 2349                      # structurally non-zero unique entries of a symmetric GLL K_e
-    bytes_elem = ks_nnz_unique * 4 + 27 * 4   # matrix + connectivity
-    kr = 1 << (k - 1).bit_length()
-    if apply_kernel_name(kr, ne).startswith("k_apply_mf"):
-        bytes_elem = 27 * 48 + 27 * 4         # matrix-free: point records + connectivity
-    bytes_apply = ne * bytes_elem + 2 * (neq + 1) * kr * 4
-    apply_ms = prof["apply_ms"] / max(1, prof["apply_launches"])
-    achieved = bytes_apply / (apply_ms / 1000.0) / 1e9
-    traffic = None
-    tpath = os.path.join(ROOT, "profiles", "apply_traffic.json")
-    if os.path.exists(tpath):
-        with open(tpath) as f:
-            measured = json.load(f)
-        if measured.get("kernel") == apply_kernel_name(kr, ne):
-            traffic = measured.get("bytes_per_launch")
+    roofline, kernel_ms = kernel_report(prof, ne, neq, 1 << (k - 1).bit_length(), args.steps)
 
     precision = None
     if args.no_fp64:
@@ -717,14 +735,8 @@ def run_ours(args, rank, world, local):
                        "mixed_batched_over_plain_fos": value / value64 if value64 == value64 else None},
         "fos_measured": fosm,
         "precision": precision,
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                     "traffic": traffic, "kernel": apply_kernel_name(kr, ne),
-                     "algorithmic_bytes_per_launch": bytes_apply, "avg_launch_ms": apply_ms,
-                     "peak_source": peak_kind},
-        "kernel_ms_per_pcg_iter": {"apply": apply_ms,
-                                   "gather": prof["gather_ms"] / max(1, prof["apply_launches"]),
-                                   "update": prof["update_ms"] / max(1, prof["apply_launches"]),
-                                   "stress_per_step": prof["stress_ms"] / max(1, args.steps)},
+        "roofline": roofline,
+        "kernel_ms_per_pcg_iter": kernel_ms,
         "gpu_launches": prof["launches"],
         "clocks": clk,
         "e2e": e2e,

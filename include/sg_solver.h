@@ -353,8 +353,10 @@ int sg_excavation(sg_model* model, const sg_control* ctl, int s0_type, double z0
 int sg_excavation_fields(const sg_model* model, double* vmeps, double* scf);
 
 /* ---- timing of the device work of the last call ----------------------- */
-/* ms[0] PCG chunks that run as one kernel (small meshes), ms[1] element apply, ms[2] gather, ms[3] PCG vector update,
- * ms[4] stress update, ms[5] stiffness build; counts[0..3] = launches of the
+/* ms[0] total of the following, ms[1] element apply, ms[2] gather, ms[3] PCG vector update,
+ * ms[4] stress update, ms[5] stiffness build, ms[6] PCG iterations that run inside one
+ * kernel (small and medium meshes, FP64 solves of one column): their applies, gathers and
+ * updates are not in ms[1..3]; counts[0..3] = launches of the
  * apply kernel, total kernel launches, PCG iterations, FP64 refinement residuals.
  * Collected with CUDA events on the context's stream when enabled. */
 int sg_profile_enable(sg_ctx* ctx, int on);

@@ -252,7 +252,7 @@ class Context:
         cnt = np.zeros(4, np.int64)
         lib().sg_profile_read(self.h, _ptr(ms), _ptr(cnt))
         return dict(total_ms=ms[0], apply_ms=ms[1], gather_ms=ms[2], update_ms=ms[3], stress_ms=ms[4],
-                    stiffness_ms=ms[5], apply_launches=int(cnt[0]), launches=int(cnt[1]), pcg_iters=int(cnt[2]),
+                    stiffness_ms=ms[5], persistent_ms=ms[6], apply_launches=int(cnt[0]), launches=int(cnt[1]), pcg_iters=int(cnt[2]),
                     refine_residuals=int(cnt[3]))
 
 

@@ -346,7 +346,7 @@ static int pcg_run_t(sg_ctx* C, const Op& op, const PcgBufs<V>& B, int n1, V* u,
         done_chunk = launch_pcg_persistent64(op.dense != 0, op.dense ? op.rows : (const double*)op.K, op.ge, op.nelmt,
                                              op.T->d_pos, C->d_nbr, *op.T, n1, u, B.r, B.z, B.p, B.kp, B.Y, dp, B.cs,
                                              B.G, B.part, persist_chunk, s);
-        C->prof_end(ev, 0);
+        if (done_chunk) C->prof_end(ev, 6);
       }
     cudaGraphExec_t ex = (!done_chunk && graphs && nchunks > 0) ? C->chunk_graph(key, eager_chunk) : nullptr;
     if (done_chunk) {
@@ -530,7 +530,8 @@ double sg_timer_ms(sg_ctx* c, int a, int b) {
 int sg_profile_read(sg_ctx* c, double* ms, long long* counts) {
   if (!c) return SG_ERR_BADARG;
   c->prof_flush();
-  for (int i = 0; i < 8; ++i) ms[i] = c->prof.ms[i];
+  for (int i = 1; i < 8; ++i) ms[i] = c->prof.ms[i];
+  ms[0] = std::accumulate(ms + 1, ms + 8, 0.0);
   for (int i = 0; i < 4; ++i) counts[i] = c->prof.counts[i];
   counts[1] = launch_count() - c->launch0;
   return SG_OK;
@@ -1219,7 +1220,7 @@ static int linear_solve(sg_model* M, const sg_control* ctl, const Op& op64, cons
     out->state = PERSIST_NONE;
     int ev = c->prof_begin();
     const bool ok = persist_round(c, KR, op32, W, dprecon32, st, out);
-    c->prof_end(ev, 0);
+    if (ok) c->prof_end(ev, 6);
     if (ok) launch_axpy_correction(n1, KR, mask, W.b32.G, W.d32, W.x, corr_part, c->stream);
     return ok;
   };
