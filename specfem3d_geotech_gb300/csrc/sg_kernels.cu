@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "sg_kernels.cuh"
+#include "sg_sum3.cuh"
 
 #include <atomic>
 
@@ -89,10 +90,8 @@ __device__ __forceinline__ V pdir(V beta, V p, V z) { return fmav<V>(beta, p, z)
 // Dot-product accumulator.  FP64 vectors accumulate in FP64.  FP32 vectors
 // accumulate exact products (a*b = p + e with e = fma(a,b,-p)) in a
 // compensated two-float sum, which keeps FP64-level accuracy of the sum while
-// issuing only FP32 instructions.  The pair is widened to FP64 once per warp:
-// an FP64 add occupies the SM's FP64 unit for 16 cycles a warp, so a shuffle
-// tree of FP64 adds over 32 resident warps and 8 sums costs some 10 us, and
-// the two-float tree adds no error of a higher order than the lo sums carry.
+// issuing only FP32 instructions; the pair is widened to FP64 per thread.  The
+// flat kernels below, whose threads add more products, use sg_sum3.cuh instead.
 template <typename V>
 struct DotAcc;
 template <>
@@ -113,24 +112,21 @@ struct DotAcc<float> {
     hi = t;
     lo += err + e;
   }
-  // the sum over lanes that differ in lane bits >= o0, exact in the high parts
-  __device__ __forceinline__ void warp_sum(int o0) {
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-      if (o < o0) break;
-      const float h = __shfl_xor_sync(0xffffffffu, hi, o), l = __shfl_xor_sync(0xffffffffu, lo, o);
-      const float t = hi + h, bp = t - hi;
-      const float err = (hi - (t - bp)) + (h - bp);
-      hi = t;
-      lo = (lo + l) + err;
-    }
-  }
   __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
-  __device__ __forceinline__ float2 pair() const { return make_float2(hi, lo); }
 };
-// The FP64 unit takes a warp's conversion or addition in some 19 cycles, so the
-// warps of a block leave pairs and a few threads widen and add them.
-__device__ __forceinline__ double widen(float2 x) { return (double)x.x + (double)x.y; }
+// The sum over lanes that differ in lane bits o1 .. o0.  The FP64 unit takes a
+// warp's conversion or addition in some 19 cycles, so sums stay three floats up to
+// a block's.
+__device__ __forceinline__ Sum3 warp_sum3(Sum3 x, int o1, int o0) {
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    if (o > o1) continue;
+    if (o < o0) break;
+    x.add(Sum3{__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o),
+               __shfl_xor_sync(0xffffffffu, x.m, o)});
+  }
+  return x;
+}
 
 // Per-column block reduction of `val` (threads whose index = j mod KR hold
 // column j).  Result for column j lands in out[j] on thread 0..KR-1 of warp 0.
@@ -976,6 +972,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_gather(
 // elements and 8 columns (16,000 and 16): staged 89 (66); 960 threads without
 // the read-ahead 80 (45); with it, one block of 768 76 (42), two of 384 73 (41).
 // Bulk copies of the slots into shared memory took 93, 32-byte pieces 101.
+// A thread's dots are kept in two halves, the first one in shared memory, so that
+// neither adds more products than a thread of the staged gather does; a third
+// float for each took 9 us more.
 int g_gather_variant = 1;   // 0 = staged gather for every case
 void set_gather_variant(int v) { g_gather_variant = v; }
 constexpr int FG_THREADS = 384, FG_PER_SM = 2;   // gather: 24 warps at 80 registers
@@ -1063,9 +1062,12 @@ __global__ void __launch_bounds__(FG_THREADS, FG_PER_SM) k_pcg_gather_flat(
   constexpr int QPD = KR / VW;          // pieces per dof row
   constexpr int LPN = 3 * QPD;          // pieces per node
   static_assert(FG_THREADS % LPN == 0 && FG_THREADS % 32 == 0, "a thread keeps its columns");
+  constexpr int NW = FG_THREADS / 32;
+  static_assert(NW <= 16, "a lane for each warp");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = threadIdx.x % LPN, d = q / QPD, c0 = VW * (q % QPD);
-  DotAcc<float> dacc[VW];
+  CompSum dacc[VW];
+  __shared__ CompSum half[VW][FG_THREADS];   // the dots of a thread's first half
   bool live[VW];
   float beta[VW];
 #pragma unroll
@@ -1076,6 +1078,9 @@ __global__ void __launch_bounds__(FG_THREADS, FG_PER_SM) k_pcg_gather_flat(
   const float* yq = Y + VW * q;
   int gstride = gridDim.x * (FG_THREADS / LPN);
   int g = blockIdx.x * (FG_THREADS / LPN) + threadIdx.x / LPN;
+  int first = g < ng ? ((ng - 1 - g) / gstride + 4) / 4 : 0;   // pairs of nodes in that half
+#pragma unroll
+  for (int k = 0; k < VW; ++k) half[k][threadIdx.x] = CompSum();
   if (pass_down(G, 1)) { g = ng - 1 - g; gstride = -gstride; }
   // a node's first four slots and its p and z rows, which do not depend on the
   // sums, are asked for while the node before is summed
@@ -1133,23 +1138,31 @@ __global__ void __launch_bounds__(FG_THREADS, FG_PER_SM) k_pcg_gather_flat(
     ask(A);
     sum(B);
     maps(g + 3 * gstride, B);
+    if (--first == 0) {
+#pragma unroll
+      for (int k = 0; k < VW; ++k) {
+        half[k][threadIdx.x] = dacc[k];
+        dacc[k] = CompSum();
+      }
+    }
   }
   if (mode == 0) return;
-  __shared__ float2 sred[FG_THREADS / 32][KR];
+  __shared__ Sum3 sred[NW][KR];
   __shared__ double sfin[FG_THREADS];
   __shared__ double sout[KR];
 #pragma unroll
   for (int k = 0; k < VW; ++k) {
-    dacc[k].warp_sum(QPD);
-    if (lane < QPD) sred[warp][VW * lane + k] = dacc[k].pair();   // lane r holds pieces q % QPD of its lane class
+    Sum3 x = dacc[k].sum();
+    x.add(half[k][threadIdx.x].sum());
+    x = warp_sum3(x, 16, QPD);
+    if (lane < QPD) sred[warp][VW * lane + k] = x;   // lane r holds pieces q % QPD of its lane class
   }
   __syncthreads();
   // lane class r = lane % QPD of warp w holds columns VW * ((32 w + r) % QPD) ..: 32 is a multiple of QPD
-  if (threadIdx.x < KR) {
-    double v = 0.0;
-#pragma unroll
-    for (int w = 0; w < FG_THREADS / 32; ++w) v += widen(sred[w][threadIdx.x]);
-    part[(size_t)blockIdx.x * KR + threadIdx.x] = v;
+  if (threadIdx.x < (16 * KR + 31) / 32 * 32) {   // sixteen lanes a column
+    const int j = threadIdx.x / 16, w = threadIdx.x % 16;
+    const Sum3 x = warp_sum3(j < KR && w < NW ? sred[w][j] : zero3(), 8, 1);
+    if (j < KR && w == 0) part[(size_t)blockIdx.x * KR + j] = x.value();
   }
   if (last_block(&G->cntB)) {
     last_block_sum<KR, FG_THREADS>(part, gridDim.x, sfin, sout);
@@ -1633,9 +1646,10 @@ __global__ void __launch_bounds__(RED_THREADS) k_pcg_update(
 // and is not formed.  HBM bounds it at large meshes (7 vector passes); one
 // block of 512 threads per SM with four pieces of four vectors a thread in
 // flight (128 KB) leaves 152 partials for the last block.
-// The dots stay pairs and the maxima FP32 until a few threads add the warps' and
-// the blocks': widened by every warp, and maxima in FP64, the tail took 5 to 7
-// us more.  us at 62,000 elements and 8 columns 72 -> 67, 16,000 and 16 49 -> 42.
+// The dots stay FP32 (sg_sum3.cuh: a thread's in groups of the four pieces of an
+// iteration, three floats over lanes and warps) and so do the maxima, until a few
+// threads add the blocks': widened by every warp, the tail took 5 to 7 us more.
+// us at 62,000 elements and 8 columns 72 -> 66, 16,000 and 16 49 -> 42.
 template <int KR>
 __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
     int n1, float* __restrict__ u, float* __restrict__ r, float* __restrict__ z, const float* __restrict__ p,
@@ -1658,7 +1672,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
     all4 = all4 && live[k];
   }
   float mp[4] = {0.f, 0.f, 0.f, 0.f};
-  DotAcc<float> rza[4], rra[4];
+  CompSum rza[4], rra[4];
   const size_t n = (size_t)n1 * KR, n4 = (n + 3) / 4;
   size_t stride = (size_t)gridDim.x * FU_THREADS;   // a multiple of QP
   size_t i = (size_t)blockIdx.x * FU_THREADS + threadIdx.x;
@@ -1693,6 +1707,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
     }
   };
   if (any && init) {
+    CompSum3 rz3[4], rr3[4];
     for (; i < n4; i += stride) {
       float fv[4], kv[4], dv[4], rn[4], zn[4];
       load(f, i, fv);
@@ -1702,10 +1717,15 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
       for (int k = 0; k < 4; ++k) {
         rn[k] = fv[k] - kv[k];
         zn[k] = dv[k] * rn[k];
-        if (live[k]) { rza[k].add(rn[k], zn[k]); rra[k].add(rn[k], rn[k]); }
+        if (live[k]) { rz3[k].add(rn[k], zn[k]); rr3[k].add(rn[k], rn[k]); }
       }
       store(r, i, rn);
       store(z, i, zn);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      rza[k].hi = rz3[k].hi; rza[k].lo = rz3[k].lo + rz3[k].ll;
+      rra[k].hi = rr3[k].hi; rra[k].lo = rr3[k].lo + rr3[k].ll;
     }
   } else if (any) {
     constexpr int U = 4;
@@ -1720,25 +1740,31 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
         const size_t o = i + q * stride;
         if (o < n4) { load(p, o, pv[q]); load(u, o, uv[q]); load(r, o, rv[q]); load(kp, o, kv[q]); diag(o, dv[q]); }
       }
+      // a column's four products of an iteration go into two floats, then into the thread's sum
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        CompSum rz, rr;
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          uv[q][k] = fmaf(alpha[k], pv[q][k], uv[q][k]);
+          rv[q][k] = fmaf(-alpha[k], kv[q][k], rv[q][k]);
+          kv[q][k] = dv[q][k] * rv[q][k];   // z
+          if (live[k] && i + q * stride < n4) {
+            mp[k] = fmaxf(mp[k], fabsf(pv[q][k]));
+            if (q == 0) { rz.set(rv[q][k], kv[q][k]); rr.set(rv[q][k], rv[q][k]); }
+            else { rz.add(rv[q][k], kv[q][k]); rr.add(rv[q][k], rv[q][k]); }
+          }
+        }
+        rza[k].add(rz);
+        rra[k].add(rr);
+      }
 #pragma unroll
       for (int q = 0; q < U; ++q) {
         const size_t o = i + q * stride;
         if (o >= n4) continue;
-        float un[4], rn[4], zn[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          un[k] = fmaf(alpha[k], pv[q][k], uv[q][k]);
-          rn[k] = fmaf(-alpha[k], kv[q][k], rv[q][k]);
-          zn[k] = dv[q][k] * rn[k];
-          if (live[k]) {
-            mp[k] = fmaxf(mp[k], fabsf(pv[q][k]));
-            rza[k].add(rn[k], zn[k]);
-            rra[k].add(rn[k], rn[k]);
-          }
-        }
-        store(u, o, un);
-        store(r, o, rn);
-        store(z, o, zn);
+        store(u, o, uv[q]);
+        store(r, o, rv[q]);
+        store(z, o, kv[q]);
       }
     }
   }
@@ -1746,7 +1772,7 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
   constexpr int NQ = 2 * KR, NW = FU_THREADS / 32, NS = FU_THREADS / 2, QC = 4 * QP;
   double* psum = part;
   float* pmax = reinterpret_cast<float*>(part + (size_t)gridDim.x * NQ);
-  __shared__ float2 sred[NW][2][QC];   // per warp: r.z and |r|^2 of its components
+  __shared__ Sum3 sred[NW][2][QC];   // per warp: r.z and |r|^2 of its components
   __shared__ float smp[NW][QC];
   __shared__ double sfin[NS];
   __shared__ double sout[NQ];
@@ -1755,34 +1781,30 @@ __global__ void __launch_bounds__(FU_THREADS, 1) k_pcg_update_flat(
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    rza[k].warp_sum(QP);
-    rra[k].warp_sum(QP);
+    const Sum3 rz = warp_sum3(rza[k].sum(), 16, QP), rr = warp_sum3(rra[k].sum(), 16, QP);
 #pragma unroll
     for (int o = 16; o >= QP; o >>= 1) mp[k] = fmaxf(mp[k], __shfl_xor_sync(FULL, mp[k], o));
     if (lane < QP) {
-      sred[warp][0][4 * lane + k] = rza[k].pair();
-      sred[warp][1][4 * lane + k] = rra[k].pair();
+      sred[warp][0][4 * lane + k] = rz;
+      sred[warp][1][4 * lane + k] = rr;
       smp[warp][4 * lane + k] = mp[k];
     }
   }
   __syncthreads();
-  if (threadIdx.x < NQ) {   // quantity and column: a column's components are j, j + KR, ...
-    const int h = threadIdx.x / KR, j = threadIdx.x % KR;
-    double v = 0.0;
+  static_assert(NW == 16 && NQ * NW <= FU_THREADS && NQ * NW % 32 == 0, "sixteen lanes a quantity");
+  if (threadIdx.x < NQ * NW) {   // quantity and column: a column's components are j, j + KR, ...
+    const int q = threadIdx.x / NW, w = threadIdx.x % NW, h = q / KR, j = q % KR;
+    Sum3 x = sred[w][h][j];
 #pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      double x = 0.0;
-#pragma unroll
-      for (int c = 0; c < QC; c += KR) x += widen(sred[w][h][j + c]);
-      v += x;
-    }
-    psum[(size_t)blockIdx.x * NQ + threadIdx.x] = v;
-  } else if (threadIdx.x >= 32 * ((NQ + 31) / 32) && threadIdx.x < 32 * ((NQ + 31) / 32) + KR) {
-    const int j = threadIdx.x - 32 * ((NQ + 31) / 32);
+    for (int c = KR; c < QC; c += KR) x.add(sred[w][h][j + c]);
+    x = warp_sum3(x, 8, 1);
+    if (w == 0) psum[(size_t)blockIdx.x * NQ + q] = x.value();
     float m = 0.f;
-    for (int w = 0; w < NW; ++w)
-      for (int c = 0; c < QC; c += KR) m = fmaxf(m, smp[w][j + c]);
-    pmax[(size_t)blockIdx.x * KR + j] = m;
+#pragma unroll
+    for (int c = 0; c < QC; c += KR) m = fmaxf(m, smp[w][j + c]);
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
+    if (w == 0 && h == 0) pmax[(size_t)blockIdx.x * KR + j] = m;
   }
   if (!last_block(&G->cntC)) return;
   if (threadIdx.x >= NS) {

@@ -18,11 +18,12 @@
 // added by every block after it, in the same order, so all blocks take the
 // same decisions and results are deterministic.
 //
-// FP64 arithmetic is kept out of the loop: an FP64 add or conversion holds the
-// SM's FP64 unit for 16 cycles a warp, and the trees over 15 warps and up to 32
-// sums took longer than the barrier.  Sums stay two-float pairs (exact
-// products, compensated adds) up to the scalars, which are formed from pairs
-// and rounded to FP32 once, as the vector operations take them.
+// FP64 arithmetic is kept out of the loop: the trees over 15 warps and up to 32
+// sums took longer than the barrier.  Sums and the scalars formed from them are
+// three floats (sg_sum3.cuh), more bits than FP64 keeps, and rounded to FP32 once,
+// as the vector operations take them.  Against pairs that costs some 25 cycles an
+// addition, of 20 one after the other; on small meshes the nodes are spread over
+// all blocks, so that few warps of a block have sums, which gains as much.
 //
 // A dof row's u, r, p stay in the registers of the thread that owns it while
 // the mesh is small enough (R pieces of up to four columns a thread, R = 1 or
@@ -45,6 +46,7 @@
 #include <type_traits>
 
 #include "sg_kernels.cuh"
+#include "sg_sum3.cuh"
 
 namespace sg {
 
@@ -55,40 +57,9 @@ constexpr int NWARP = NT / 32;
 constexpr int MAX_BLOCKS = 152;       // one block per SM
 constexpr int POLL_TRIES = 1 << 20;   // bounded wait, below a second
 
-// compensated FP32 dot accumulator (exact products, two-float sum)
-struct CompSum {
-  float hi = 0.f, lo = 0.f;
-  __device__ __forceinline__ void add(float a, float b) {
-    const float p = a * b, e = fmaf(a, b, -p);
-    const float t = hi + p, bp = t - hi;
-    const float err = (hi - (t - bp)) + (p - bp);
-    hi = t;
-    lo += err + e;
-  }
-  __device__ __forceinline__ void add(const float2 x) {   // another such sum
-    const float t = hi + x.x, bp = t - hi;
-    const float err = (hi - (t - bp)) + (x.x - bp);
-    hi = t;
-    lo = (lo + x.y) + err;
-  }
-  __device__ __forceinline__ float2 pair() const { return make_float2(hi, lo); }
-};
-__device__ __forceinline__ double value(const float2 x) { return (double)x.x + (double)x.y; }
-__device__ __forceinline__ float2 split(double x) {
-  const float h = (float)x;
-  return make_float2(h, (float)(x - (double)h));
-}
-__device__ __forceinline__ float2 norm2(const float2 x) {   // |lo| <= ulp(hi) / 2
-  const float h = x.x + x.y;
-  return make_float2(h, x.y - (h - x.x));
-}
-// a / b of two-float numbers: the FP32 quotient and its residual's
-__device__ __forceinline__ float2 div2(float2 a, float2 b) {
-  a = norm2(a);
-  b = norm2(b);
-  const float q = a.x / b.x;
-  const float r = fmaf(-q, b.x, a.x) + fmaf(-q, b.y, a.y);
-  return norm2(make_float2(q, r / b.x));
+__device__ __forceinline__ Sum3 shfl_xor(const Sum3& x, int o) {
+  return Sum3{__shfl_xor_sync(0xffffffffu, x.h, o), __shfl_xor_sync(0xffffffffu, x.l, o),
+              __shfl_xor_sync(0xffffffffu, x.m, o)};
 }
 
 // Sums x[0..N) over the lanes that differ in bits O, O/2, ..., O0, halving the
@@ -96,21 +67,21 @@ __device__ __forceinline__ float2 div2(float2 a, float2 b) {
 // instead of N * steps): the lane ends with value index() in x[0].
 template <int N, int O, int O0>
 struct Reduce {
-  static __device__ __forceinline__ void run(CompSum (&x)[N], int lane) {
+  static __device__ __forceinline__ void run(Sum3 (&x)[N], int lane) {
     if constexpr (O >= O0) {
       if constexpr (N > 1) {
         const bool up = lane & O;
-        CompSum y[N / 2];
+        Sum3 y[N / 2];
 #pragma unroll
         for (int i = 0; i < N / 2; ++i) {
-          const CompSum keep = up ? x[i + N / 2] : x[i], send = up ? x[i] : x[i + N / 2];
+          const Sum3 keep = up ? x[i + N / 2] : x[i], send = up ? x[i] : x[i + N / 2];
           y[i] = keep;
-          y[i].add(make_float2(__shfl_xor_sync(0xffffffffu, send.hi, O), __shfl_xor_sync(0xffffffffu, send.lo, O)));
+          y[i].add(shfl_xor(send, O));
         }
         Reduce<N / 2, O / 2, O0>::run(y, lane);
         x[0] = y[0];
       } else {
-        x[0].add(make_float2(__shfl_xor_sync(0xffffffffu, x[0].hi, O), __shfl_xor_sync(0xffffffffu, x[0].lo, O)));
+        x[0].add(shfl_xor(x[0], O));
         Reduce<N, O / 2, O0>::run(x, lane);
       }
     }
@@ -166,7 +137,7 @@ struct Args {
   const float* dp;    // inverted diagonal
   ColState* cs;
   PcgGlobal* G;       // cntB counts the barrier's arrivals
-  float2* part;       // block partials: phase B [KR][grid], phase C [2 KR][grid]
+  float4* part;       // block partials (three floats): phase B [KR][grid], phase C [2 KR][grid]
   const float* f;     // right-hand side of a new solve
   PersistStart st;
   PersistOut* out;    // pinned host memory
@@ -304,37 +275,51 @@ __device__ __forceinline__ void element_product(const Args& A, int e, const floa
   }
 }
 
-// R pieces per thread in registers; R = 0: streamed.
+// R pieces per thread in registers; STREAMED_FEW: up to four, STREAMED: any number, streamed.
+constexpr int STREAMED_FEW = 0, STREAMED = -1;
 template <int KR, int R>
 __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
   using S = Shape<KR>;
   constexpr int VW = S::VW, QPD = S::QPD, LPN = S::LPN;
   constexpr int RR = R > 0 ? R : 1;
+  // A thread's products of a column: up to four in two floats; three keep the
+  // rounding errors of many.  (3,289 elements, 8 columns: 27.8 us an iteration, 28.7
+  // with three floats there too.)
+  using Dot = std::conditional_t<R != STREAMED && R <= 4, CompSum, CompSum3>;
   extern __shared__ __align__(16) float smem[];
-  __shared__ float2 sred[2 * KR][NWARP + 1];
+  __shared__ Sum3 sred[2 * KR][NWARP];
   // block-local copy of the column state (identical in every block)
-  __shared__ float2 c_rz[KR], c_alpha[KR], c_beta[KR], c_rr[KR], c_goal[KR];
-  __shared__ int c_live[KR], c_iters[KR], c_failed[KR];
+  __shared__ Sum3 c_rz[KR], c_rr[KR], c_goal[KR];
+  __shared__ Sum3 c_pkp[KR];
+  __shared__ float c_alpha[KR], c_beta[KR];
+  __shared__ int c_live[KR], c_ran[KR], c_iters[KR], c_failed[KR];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   PcgGlobal* G = A.G;
   const int init = A.st.init, keep = A.st.keep, maxiter = A.st.maxiter, kcols = A.st.kcols;
   if (!init && G->all_done) return;
   if (t < KR) {
     const ColState c = A.cs[t];
-    c_rz[t] = split(c.rz);
+    c_rz[t] = split3(c.rz);
     c_live[t] = (A.st.active >> t) & 1u;
     if (!init) {
-      c_alpha[t] = split(c.alpha); c_beta[t] = split(c.beta); c_rr[t] = split(c.rr);
-      c_goal[t] = split(c.tol * c.tol * c.rr0);   // |r|^2 at which the column stops
+      c_alpha[t] = (float)c.alpha; c_beta[t] = (float)c.beta; c_rr[t] = split3(c.rr);
+      c_goal[t] = split3(c.tol * c.tol * c.rr0);   // |r|^2 at which the column stops
       c_live[t] = c_live[t] && !c.done; c_iters[t] = c.iters; c_failed[t] = c.failed;
     } else {
-      c_alpha[t] = c_beta[t] = c_rr[t] = c_goal[t] = make_float2(0.f, 0.f);
+      c_alpha[t] = c_beta[t] = 0.f;
+      c_rr[t] = c_goal[t] = zero3();
       c_iters[t] = c_failed[t] = 0;
     }
+    c_ran[t] = c_live[t];
   }
   int itn = init ? 0 : G->it, alldone = 0;
   const int grid = gridDim.x, bid = blockIdx.x;
   unsigned arrivals = 0;
+
+  // nodes of a block and pass; with no more pieces than threads every block has its
+  // share, and the warps without a piece leave the sums to the others
+  const int npb = R == 1 ? (A.ngroups + grid - 1) / grid : NT / LPN;
+  const int nwarp = R == 1 ? (npb * LPN + 31) / 32 : NWARP;
 
   // Grid barrier: earlier writes of the block are visible to every block
   // after it.  Returns false when the wait ran out.
@@ -355,47 +340,63 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
     return !__syncthreads_or(!good);
   };
   // sred[v][warp] summed over warps into this block's column of the partials
-  // (the maximum of the high parts when MAXOP); 32 / NV lanes per value
-  auto publish = [&](auto nvc, auto maxc, float2* out) {
+  // (the maximum of the high parts when MAXOP)
+  auto publish = [&](auto nvc, auto maxc, float4* out) {
     constexpr int NV = decltype(nvc)::value;
     constexpr bool MAXOP = decltype(maxc)::value;
     __syncthreads();
-    if (warp == 0) {
-      constexpr int SUB = NV >= 32 ? 1 : (32 / NV > 8 ? 8 : 32 / NV);
-      const int v = lane / SUB, s = lane % SUB;
-      CompSum x[1];
-      if (v < NV)
-        for (int w = s; w < NWARP; w += SUB) {
-          if (MAXOP) x[0].hi = fmaxf(x[0].hi, sred[v][w].x);
+    constexpr int SUB = 8, NVW = 32 / SUB;   // lanes a value, values a warp
+    static_assert((NV + NVW - 1) / NVW <= NWARP && SUB <= NWARP, "warps and their lanes");
+    if (warp < (NV + NVW - 1) / NVW) {
+      const int v = warp * NVW + lane / SUB, s = lane % SUB;
+      Sum3 x[1] = {zero3()};
+      if (v < NV) {
+        if (s < nwarp) x[0] = sred[v][s];
+        for (int w = s + SUB; w < nwarp; w += SUB) {
+          if (MAXOP) x[0].h = fmaxf(x[0].h, sred[v][w].h);
           else x[0].add(sred[v][w]);
         }
+      }
       if (MAXOP) {
 #pragma unroll
-        for (int o = SUB / 2; o >= 1; o >>= 1) x[0].hi = fmaxf(x[0].hi, __shfl_xor_sync(0xffffffffu, x[0].hi, o));
+        for (int o = SUB / 2; o >= 1; o >>= 1) x[0].h = fmaxf(x[0].h, __shfl_xor_sync(0xffffffffu, x[0].h, o));
       } else {
         Reduce<1, SUB / 2, 1>::run(x, lane);
       }
-      if (v < NV && s == 0) __stcg(out + (size_t)v * grid + bid, x[0].pair());
+      if (v < NV && s == 0) __stcg(out + (size_t)v * grid + bid, make_float4(x[0].h, x[0].l, x[0].m, 0.f));
     }
   };
   // sum over the blocks of one value's partials, by one warp
-  auto block_sum = [&](const float2* in) -> CompSum {
+  auto block_sum = [&](const float4* in) -> Sum3 {
     constexpr int NB = (MAX_BLOCKS + 31) / 32;
-    float2 w[NB];
+    Sum3 w[NB];
 #pragma unroll
-    for (int i = 0; i < NB; ++i) w[i] = lane + 32 * i < grid ? __ldcg(in + lane + 32 * i) : make_float2(0.f, 0.f);
-    CompSum x[1];
+    for (int i = 0; i < NB; ++i) {
+      const float4 v = lane + 32 * i < grid ? __ldcg(in + lane + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      w[i] = Sum3{v.x, v.y, v.z};
+    }
 #pragma unroll
-    for (int i = 0; i < NB; ++i) x[0].add(w[i]);
+    for (int o = 1; o < NB; o *= 2)
+#pragma unroll
+      for (int i = 0; i + o < NB; i += 2 * o) w[i].add(w[i + o]);
+    Sum3 x[1] = {w[0]};
     Reduce<1, 16, 1>::run(x, lane);
-    return x[0];
+    return norm3(x[0]);
+  };
+
+  // product m of a thread
+  auto dot_add = [](auto& x, int m, float a, float b) {
+    if constexpr (R > 0 && std::is_same_v<Dot, CompSum>) {
+      if (m == 0) { x.set(a, b); return; }
+    }
+    x.add(a, b);
   };
 
   // the thread's pieces: columns c0 .. c0 + VW - 1 of dof row d of nodes g0, g0 + gstride, ...
   const int qp = t % LPN, d = qp / QPD, c0 = VW * (qp % QPD);
   const int gstride = grid * (NT / LPN);
   // consecutive nodes stay in one block
-  const int g0 = bid * (NT / LPN) + t / LPN;
+  const int g0 = t / LPN < npb ? bid * npb + t / LPN : A.ngroups;
   Vec<VW> ru[RR], rr[RR], rp[RR], rk[RR];
   int gd[RR], sa[RR], sb[RR];
   float dv[RR];
@@ -422,8 +423,8 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
   }
   float* U = smem + (size_t)warp * (S::UF + S::FF);
   float* F = U + S::UF;
-  float2* partB = A.part;
-  float2* partC = A.part + (size_t)grid * KR;
+  float4* partB = A.part;
+  float4* partC = A.part + (size_t)grid * KR;
   // the block's run of (element, column group) pairs
   const int nw = A.nelmt * QPD, per = (nw + grid - 1) / grid, w0 = bid * per, w1 = min(nw, w0 + per);
   float* cache = smem + (size_t)NWARP * (S::UF + S::FF);
@@ -441,13 +442,17 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
 
   // warp sums of the thread's values (x[i] of column VW r + i % VW, r = lane
   // class) into sred[(i / VW) KR + column][warp]
-  auto reduce_lanes = [&](auto& x) {
-    constexpr int N = sizeof(x) / sizeof(x[0]);
+  auto reduce_lanes = [&](auto& dots) {
+    constexpr int N = sizeof(dots) / sizeof(dots[0]);
+    if (warp >= nwarp) return;
+    Sum3 x[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) x[i] = dots[i].sum();
     constexpr int LOGN = N == 8 ? 3 : N == 4 ? 2 : N == 2 ? 1 : 0;
     Reduce<N, 16, QPD>::run(x, lane);
     // bit 4 of the lane chose the upper half of the values, bit 3 of that half, ...
     const int i = N == 1 ? 0 : lane >> (5 - LOGN), rest = lane & ((32 >> LOGN) - 1);
-    if (rest < QPD) sred[(i / VW) * KR + VW * rest + i % VW][warp] = x[0].pair();
+    if (rest < QPD) sred[(i / VW) * KR + VW * rest + i % VW][warp] = x[0];
   };
   // kp of one piece: the node's slots in element order, four loads in flight
   auto slot_sum = [&](int a, int b, Vec<VW>& acc) {
@@ -468,25 +473,25 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
 
   // r.z and r.r of the thread's columns over the grid, then each column's step,
   // identical in every block: the start of a solve, or stop test and beta
-  auto column_steps = [&](CompSum (&zz)[2 * VW], bool first) -> bool {
+  auto column_steps = [&](Dot (&zz)[2 * VW], bool first) -> bool {
     reduce_lanes(zz);
     publish(std::integral_constant<int, 2 * KR>{}, std::false_type{}, partC);
     if (!barrier()) return false;
     for (int j = warp; j < KR; j += NWARP) {
-      const CompSum x = block_sum(partC + (size_t)j * grid), y = block_sum(partC + (size_t)(KR + j) * grid);
+      const Sum3 x = block_sum(partC + (size_t)j * grid), y = block_sum(partC + (size_t)(KR + j) * grid);
       if (lane == 0 && c_live[j]) {
-        c_rr[j] = norm2(y.pair());
+        c_rr[j] = y;
         if (first) {
-          if (keep) c_beta[j] = div2(x.pair(), c_rz[j]);
-          c_rz[j] = x.pair();
-          c_goal[j] = split(A.st.tol * A.st.tol * value(y.pair()));
-        } else if ((c_rr[j].x - c_goal[j].x) + (c_rr[j].y - c_goal[j].y) <= 0.f) {
+          if (keep) c_beta[j] = div3(x, c_rz[j]);
+          c_rz[j] = x;
+          c_goal[j] = split3(A.st.tol * A.st.tol * y.value());
+        } else if (at_most(y, c_goal[j])) {
           c_live[j] = 0; c_iters[j] = itn;
         } else if (itn >= maxiter) {
           c_live[j] = 0; c_failed[j] = 1; c_iters[j] = maxiter + 1;
         } else {
-          c_beta[j] = div2(x.pair(), c_rz[j]);
-          c_rz[j] = x.pair();
+          c_beta[j] = div3(x, c_rz[j]);
+          c_rz[j] = x;
         }
       }
     }
@@ -497,15 +502,15 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
   // ---- a new solve: u = 0, r = f, z = D r, and p = 0 unless the last solve's
   // direction is continued (beta = r.z / the last r.z) ----
   if (init) {
-    CompSum zz[2 * VW];
+    Dot zz[2 * VW];
     if (bid == 0 && t < KR) { A.u[t] = 0.f; A.r[t] = 0.f; A.z[t] = 0.f; A.p[t] = 0.f; }   // constrained dofs
-    auto start = [&](size_t o, float D, const Vec<VW>& rv) {
+    auto start = [&](size_t o, float D, const Vec<VW>& rv, int m) {
       Vec<VW> zv;
 #pragma unroll
       for (int q = 0; q < VW; ++q) {
         zv.v[q] = D * rv.v[q];
-        zz[q].add(rv.v[q], zv.v[q]);
-        zz[VW + q].add(rv.v[q], rv.v[q]);
+        dot_add(zz[q], m, rv.v[q], zv.v[q]);
+        dot_add(zz[VW + q], m, rv.v[q], rv.v[q]);
       }
       zv.store(A.z + o);
       if (!keep) {
@@ -517,7 +522,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
     if constexpr (R > 0) {
 #pragma unroll
       for (int m = 0; m < R; ++m)
-        if (gd[m]) start((size_t)gd[m] * KR + c0, dv[m], rr[m]);
+        if (gd[m]) start((size_t)gd[m] * KR + c0, dv[m], rr[m], m);
     } else {
       for (int g = g0; g < A.ngroups; g += gstride) {
         const int gq = __ldg(A.gdof + 3 * g + d);
@@ -528,7 +533,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
         rv.load_cg(A.f + o);
         none.store(A.u + o);
         rv.store(A.r + o);
-        start(o, __ldg(A.dp + gq), rv);
+        start(o, __ldg(A.dp + gq), rv, 1);
       }
     }
     if (!column_steps(zz, true)) return;
@@ -540,7 +545,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
       const int e = w / QPD, cc = VW * (w - e * QPD);
       float beta[VW];
 #pragma unroll
-      for (int q = 0; q < VW; ++q) beta[q] = c_beta[cc + q].x;
+      for (int q = 0; q < VW; ++q) beta[q] = c_beta[cc + q];
       element_product<KR>(A, e, e - e0 < A.cached ? cache + (size_t)(e - e0) * S::EF : nullptr, cc, lane, beta, U, F);
       __syncwarp();
     }
@@ -548,9 +553,9 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
     // ---- B: kp, p and p.kp ----
     bool live[VW];
     float beta[VW];
-    CompSum dot[VW];
+    Dot dot[VW];
 #pragma unroll
-    for (int q = 0; q < VW; ++q) { live[q] = c_live[c0 + q] != 0; beta[q] = c_beta[c0 + q].x; }
+    for (int q = 0; q < VW; ++q) { live[q] = c_live[c0 + q] != 0; beta[q] = c_beta[c0 + q]; }
     if constexpr (R > 0) {
 #pragma unroll
       for (int m = 0; m < R; ++m) {
@@ -561,7 +566,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
           if (live[q]) {
             // z = D r as phase C formed it
             rp[m].v[q] = fmaf(beta[q], rp[m].v[q], dv[m] * rr[m].v[q]);
-            dot[q].add(rp[m].v[q], rk[m].v[q]);
+            dot_add(dot[q], m, rp[m].v[q], rk[m].v[q]);
           }
         rp[m].store(A.p + (size_t)gd[m] * KR + c0);
       }
@@ -588,15 +593,15 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
     publish(std::integral_constant<int, KR>{}, std::false_type{}, partB);
     if (!barrier()) return;
     for (int j = warp; j < KR; j += NWARP) {
-      const CompSum x = block_sum(partB + (size_t)j * grid);
-      if (lane == 0 && c_live[j]) c_alpha[j] = div2(c_rz[j], x.pair());
+      const Sum3 x = block_sum(partB + (size_t)j * grid);
+      if (lane == 0 && c_live[j]) { c_alpha[j] = div3(c_rz[j], x); c_pkp[j] = x; }
     }
     __syncthreads();
     // ---- C: u, r, z and r.z, r.r ----
     float alpha[VW];
-    CompSum zz[2 * VW];   // r.z of the thread's columns, then r.r
+    Dot zz[2 * VW];   // r.z of the thread's columns, then r.r
 #pragma unroll
-    for (int q = 0; q < VW; ++q) alpha[q] = live[q] ? c_alpha[c0 + q].x : 0.f;
+    for (int q = 0; q < VW; ++q) alpha[q] = live[q] ? c_alpha[c0 + q] : 0.f;
     if constexpr (R > 0) {
 #pragma unroll
       for (int m = 0; m < R; ++m) {
@@ -609,8 +614,8 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
             rr[m].v[q] = fmaf(-alpha[q], rk[m].v[q], rr[m].v[q]);
           }
           zv.v[q] = dv[m] * rr[m].v[q];
-          zz[q].add(rr[m].v[q], zv.v[q]);
-          zz[VW + q].add(rr[m].v[q], rr[m].v[q]);
+          dot_add(zz[q], m, rr[m].v[q], zv.v[q]);
+          dot_add(zz[VW + q], m, rr[m].v[q], rr[m].v[q]);
         }
         zv.store(A.z + (size_t)gd[m] * KR + c0);
       }
@@ -674,7 +679,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
   for (int q = 0; q < VW; ++q) {
 #pragma unroll
     for (int o = 16; o >= QPD; o >>= 1) mp[q] = fmaxf(mp[q], __shfl_xor_sync(0xffffffffu, mp[q], o));
-    if (lane < QPD) sred[VW * lane + q][warp] = make_float2(mp[q], 0.f);
+    if (lane < QPD) sred[VW * lane + q][warp].h = mp[q];
   }
   publish(std::integral_constant<int, KR>{}, std::true_type{}, partB);
   if (!barrier()) return;
@@ -686,9 +691,12 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
       for (int b = 0; b < grid; ++b) m = fmaxf(m, __ldcg(partB + (size_t)t * grid + b).x);
       c.active = (A.st.active >> t) & 1u;
       if (c.active) {
-        c.rz = value(c_rz[t]); c.alpha = value(c_alpha[t]); c.beta = value(c_beta[t]); c.rr = value(c_rr[t]);
+        // a column that has stopped keeps the r.z that its last step took
+        if (c_live[t]) c.alpha = c_alpha[t];
+        else if (c_ran[t]) c.alpha = c_rz[t].value() / c_pkp[t].value();
+        c.rz = c_rz[t].value(); c.beta = c_beta[t]; c.rr = c_rr[t].value();
         c.maxp = m; c.done = !c_live[t]; c.iters = c_iters[t]; c.failed = c_failed[t];
-        if (init) { c.tol = 1.0; c.rr0 = value(c_goal[t]); }   // their product is the goal
+        if (init) { c.tol = 1.0; c.rr0 = c_goal[t].value(); }   // their product is the goal
         A.out->iters[t] = c_iters[t];
         A.out->failed[t] = c_failed[t];
         A.out->step[t] = fabs(c.alpha) * (double)m;
@@ -764,7 +772,7 @@ bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int
   if (grid > pp::MAX_BLOCKS) grid = pp::MAX_BLOCKS;
   if (grid < 1) return false;
   const long per = (pieces + grid * pp::NT - 1) / (grid * pp::NT);   // pieces per thread
-  static_assert((size_t)pp::MAX_BLOCKS * 3 * KR * sizeof(float2) <= (size_t)NPART * 16 * 2 * sizeof(double),
+  static_assert((size_t)pp::MAX_BLOCKS * 3 * KR * sizeof(float4) <= (size_t)NPART * 16 * 2 * sizeof(double),
                 "partials fit half the buffer");
   if (st.init) cudaMemsetAsync(G, 0, sizeof(PcgGlobal), s);
   else cudaMemsetAsync(&G->cntB, 0, sizeof(unsigned), s);
@@ -774,14 +782,16 @@ bool launch_pcg_persistent(const float* rec, const int* ge, int nelmt, const int
   if (cached > S::CACHE) cached = S::CACHE;
   const size_t smem = S::SMEM + (size_t)cached * S::EF * sizeof(float);
   const pp::Args A{rec, ge, nelmt, pos, T.d_ptr, T.d_dof, T.ngroups, u, r, z, p, kp, Y, dp, cs, G,
-                   reinterpret_cast<float2*>(part), f, st, out, chunk, (int)cached};
+                   reinterpret_cast<float4*>(part), f, st, out, chunk, (int)cached};
   if (per <= 1) return launch_persistent<KR, 1>(A, (int)grid, smem, s);
   if (per <= 2) return launch_persistent<KR, 2>(A, (int)grid, smem, s);
   if constexpr (KR <= 2)
     if (per <= 4) return launch_persistent<KR, 4>(A, (int)grid, smem, s);
   if constexpr (KR == 1)
     if (per <= 8) return launch_persistent<KR, 8>(A, (int)grid, smem, s);
-  return launch_persistent<KR, 0>(A, (int)grid, smem, s);
+  if constexpr (KR > 2)
+    if (per <= 4) return launch_persistent<KR, pp::STREAMED_FEW>(A, (int)grid, smem, s);
+  return launch_persistent<KR, pp::STREAMED>(A, (int)grid, smem, s);
 }
 
 #define SG_PP_INST(KR)                                                                                             \
