@@ -306,7 +306,7 @@ __device__ __forceinline__ void point_grad(const double* __restrict__ Ji, int i,
 // entries from the two to seven points that the nodes share (a mask), so the
 // products of a gradient with a modulus serve three entries and no thread looks
 // at the other points.  The FP64 unit bounds it (1,000 warp instructions an
-// element at 16 cycles; 6,900 elements in 0.60 ms, against 1.91 ms with a thread
+// element at some 19 cycles; 6,900 elements in 0.60 ms, against 1.91 ms with a thread
 // per entry looking at all 27 points); own-node blocks, which share seven
 // points, come first so that a warp's threads have equally many.  The roundings
 // are written out: every solve starts from these bits.
@@ -448,9 +448,9 @@ void launch_expand_dense(const double* Ks64, int nel, double* dense, const int* 
 constexpr int APPLY_WARPS = 4;
 // 0 = register-staged loads, 1 = TMA bulk-copy pipeline (node lanes),
 // 2 = tensor cores (FP32, 8/16 RHS), 3 = lane per (element, RHS) for FP32
-// with 8/16 RHS and the TMA node-lane pipeline otherwise (default),
-// 4, 5 = as 3 for FP64, matrix-free for the FP32 operator of the mixed solve
-// (default): 1.3 KB of point records an element instead of 9.7 KB of matrix.
+// with 8/16 RHS and the TMA node-lane pipeline otherwise, 4, 5 (default) = as 3
+// for FP64, matrix-free for the FP32 operator of the mixed solve: 1.3 KB of point
+// records an element instead of 9.7 KB of matrix.
 // us per apply at 120k elements, stored against matrix-free: 328, 103 with one
 // trial, 439, 133 with four, 434, 243 with eight, 722, 413 with sixteen.
 int g_apply_variant = 5;
@@ -1861,10 +1861,13 @@ void pcg_update(int n1, V* u, V* r, V* z, const V* p, const V* kp, const V* f, c
 constexpr int STRESS_WARPS = 4;
 constexpr double DEG2RAD_D = 3.141592653589793 / 180.0;
 
-// x / b for a constant b, correctly rounded: the quotient by the rounded
-// reciprocal, its exact remainder and one correction (P. Markstein,
-// Computation of elementary functions on the IBM RISC System/6000 processor,
-// IBM J. Res. Dev. 34, 1990, theorem 7).  Three FP64 operations: 24,000 elements
+// x / b for a constant b, correctly rounded where x and the quotient are normal
+// numbers: the quotient by the rounded reciprocal, its exact remainder and one
+// correction (P. Markstein, Computation of elementary functions on the IBM RISC
+// System/6000 processor, IBM J. Res. Dev. 34, 1990, theorem 7).  An infinite x
+// gives a NaN and -0 gives 0, which changes no result here: the one quotient that
+// can be infinite, 1 / (3 sigm) / 3 of a state without mean stress, is multiplied
+// by normal stresses that add up to 0.  Three FP64 operations: 24,000 elements
 // in 1.20 ms, against 1.36 with the general divisions by 3, 6 and sqrt(3).
 __device__ __forceinline__ double div_const(double x, double b, double rb) {
   const double q = x * rb;
@@ -2349,7 +2352,7 @@ void launch_release_load(const double* geo, const int* elist, int nel, const int
 // Small vector kernels with per-column reductions written to part[block][KR][2].
 // A thread's column is fixed (its index mod KR).  Sums and maxima go over the
 // lanes of a column by shuffles, maxima on the bits of the absolute values: an
-// FP64 add or compare holds the SM's FP64 unit for 16 cycles a warp and takes
+// FP64 add or compare holds the SM's FP64 unit for some 19 cycles a warp and takes
 // some 70 to answer, and a serial tail over 256 threads made these kernels 33 us
 // each on a mesh whose data they read in three.
 // ---------------------------------------------------------------------------

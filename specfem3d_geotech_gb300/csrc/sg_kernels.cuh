@@ -155,7 +155,7 @@ struct PersistStart {
 enum { PERSIST_NONE = 0, PERSIST_MORE = 1, PERSIST_DONE = 2 };
 struct PersistOut {
   int state, it;
-  int iters[16], failed[16];
+  int iters[16];
   double step[16];   // |alpha| max|p| of the last step
 };
 template <int KR>

@@ -698,7 +698,6 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
         c.maxp = m; c.done = !c_live[t]; c.iters = c_iters[t]; c.failed = c_failed[t];
         if (init) { c.tol = 1.0; c.rr0 = c_goal[t].value(); }   // their product is the goal
         A.out->iters[t] = c_iters[t];
-        A.out->failed[t] = c_failed[t];
         A.out->step[t] = fabs(c.alpha) * (double)m;
       }
     }

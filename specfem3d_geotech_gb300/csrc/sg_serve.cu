@@ -3,10 +3,12 @@
 //
 // Requests (each its own hex8 mesh and control, with an SRF search or a list
 // of excavation stages) are queued on submission and admitted in arrival
-// order when their HBM footprint fits the server's budget.  Each worker thread owns a context (its own CUDA stream),
-// so admitted requests run concurrently and their kernels overlap on the
-// device; inside a request the SRF trials run as a continuously refilled
-// batch (sg_fos: the bisection's next k probes share every element apply).
+// order when their HBM footprint fits the server's budget.  Each worker thread
+// owns a context (its own CUDA stream), so admitted requests run concurrently:
+// their host work, copies and separate kernels overlap, while the persistent PCG
+// kernels, one block on every SM, take turns; inside a request the SRF trials run
+// as a continuously refilled batch (sg_fos: the bisection's next k probes share
+// every element apply).
 // A finished request releases its memory, which admits the next ones.
 #include <algorithm>
 #include <chrono>
@@ -45,8 +47,8 @@ struct Request {
 };
 
 // Device bytes of a request's model and an SRF batch of KR slots, per element
-// (about 25 dofs per element on 27-node meshes): FP64 and FP32 element matrices,
-// the matrix-free point records, geometry, per-slot plastic state, element
+// (about 25 dofs per element on 27-node meshes): FP64 element matrices, FP32 ones
+// (which a model has only if SG_APPLY_VARIANT asks for them), the matrix-free point records, geometry, per-slot plastic state, element
 // products and vectors.
 size_t estimate_footprint(int nelmt, int k, int precision) {
   const size_t kr = (size_t)(1 << (int)std::ceil(std::log2(std::max(1, k))));
