@@ -97,6 +97,7 @@ void add_launches(long long n);  // kernels launched through a replayed CUDA gra
 void set_apply_variant(int v);   // 0 register-staged, 1 TMA pipeline, 2 tensor cores for 8/16 FP32 RHS,
                                  // 3 lane per (element, RHS) for 8/16 FP32 RHS, 4 and 5 (default)
                                  // matrix-free FP32
+void read_switches();            // the choices of SG_APPLY_VARIANT and SG_GATHER_VARIANT
 bool persist_default_apply();    // the chosen variant leaves the FP64 apply at its default
 void set_entry_table(const int* d_entry);
 // The element applies that wait on mbarriers set *err to 1 when a bounded
