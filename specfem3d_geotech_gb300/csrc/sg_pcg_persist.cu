@@ -716,15 +716,21 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_persistent(Args A) {
 // than 15 warps per SM hide, separate launches with their own register budgets
 // win.  us per iteration of a whole trial, persistent against separate kernels:
 //   elements   1 column       2 columns      4 columns      8 columns      16 columns
-//    1,071    9.8 /  34.8   11.3 /  36.1   14.3 /  43.1   20.0 /  45.1    34.8 /  56.0
-//    3,289   12.9 /  42.0   15.4 /  48.0   21.8 /  48.9   39.2 /  58.5    70.2 /  79.2
-//    5,488   15.0 /  50.1   18.8 /  53.1   28.7 /  55.8   53.6 /  68.8   105.2 / 101.3
-//    9,600   19.8 /  60.0   26.4 /  59.8   44.3 /  61.4   82.9 /  85.4
-//   12,000   22.6 /  63.9   33.1 /  64.0   52.7 /  68.0   99.6 /  93.1
-//   25,000   44.2 /  80.1   57.9 /  87.7   99.6 /  96.4
-//   40,000   66.7 / 100.7   96.6 / 114.5
-//   64,800  126.3 / 132.3  183.3 / 158.0
-int persist_max_elements(int KR) { return KR == 1 ? 65000 : 85000 / KR; }
+//    1,071    9.5 /  28.0   10.9 /  29.9   13.0 /  33.5   17.5 /  35.9    29.8 /  41.8
+//    2,662                                                                53.8 /  58.1
+//    3,289   12.3 /  34.5   14.9 /  38.6   20.2 /  37.9   34.5 /  45.4    61.5 /  61.1
+//    5,488   14.9 /  40.5   18.2 /  43.2   26.4 /  45.4   47.8 /  55.0    84.2 /  75.5 (5,040)
+//    7,056                                                58.2 /  58.1
+//    9,600   19.7 /  47.2   25.3 /  49.3   40.6 /  49.5   72.9 /  65.8
+//   12,000   22.8 /  50.0   32.7 /  53.9   50.0 /  56.8
+//   18,000                                 68.3 /  67.1
+//   25,000   43.3 /  67.1   57.6 /  79.0
+//   43,200                 111.2 / 111.1
+//   53,760  100.7 / 105.9
+//   58,032  113.7 / 111.9
+int persist_max_elements(int KR) {
+  return KR == 1 ? 57000 : KR == 2 ? 42500 : KR == 4 ? 17000 : KR == 8 ? 7000 : 3000;
+}
 
 bool persist_enabled() {
   static const bool on = !(getenv("SG_PERSIST") && atoi(getenv("SG_PERSIST")) == 0);

@@ -56,9 +56,9 @@ def same(a, b):
     ((30, 18, 17), 1), ((30, 18, 17), 2), ((30, 18, 17), 4),   # 9,180: 4, 4, streamed
     ((40, 22, 21), 1), ((40, 22, 21), 2),                   # 18,480: 8, streamed
     ((50, 30, 27), 1),                                      # 40,500: streamed
-    ((29, 11, 13), 2), ((13, 7, 9), 4), ((40, 22, 21), 4),  # 2, 1, streamed, more than four
+    ((29, 11, 13), 2), ((13, 7, 9), 4), ((34, 20, 20), 4),  # 2, 1, streamed, more than four
     ((19, 9, 11), 8), ((19, 9, 13), 16),                    # 1,881: 2; 2,223: streamed
-    ((23, 15, 15), 11), ((27, 19, 19), 7)])                 # 5,175, 9,747: streamed, more than four
+    ((20, 11, 13), 11), ((26, 16, 16), 7)])                 # 2,860, 6,656: streamed, more than four
 def test_persistent_forms_iterate_like_the_separate_kernels(tmp_path, dims, k):
     a = trials(dims, k, tmp_path, SG_PERSIST="1")
     b = trials(dims, k, tmp_path, SG_PERSIST="0")
